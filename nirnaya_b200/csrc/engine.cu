@@ -16,6 +16,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <deque>
 #include <limits>
@@ -35,6 +36,8 @@
 #include "k_cta.cuh"
 #include "k_iter.cuh"
 #include "k_batch.cuh"
+#include "k_cluster.cuh"
+#include "cluster_plan.hpp"
 #include "nir_pdhg.h"
 
 namespace {
@@ -172,6 +175,8 @@ struct ChunkGraph {
     bool valid = false;
 };
 
+struct ClusterPlan;  // engine_cluster.cuh
+
 struct nir_pdhg {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -194,6 +199,7 @@ struct nir_pdhg {
         bool norm_valid = false;
         int power_iters = -1;
         double norm = 0.0;
+        long long version = 0;  // counts the preconditionings that changed the scaled values
     } scaled;
     double *c64 = nullptr, *l64 = nullptr, *u64 = nullptr, *rl64 = nullptr, *ru64 = nullptr;
     float *c32 = nullptr, *l32 = nullptr, *u32 = nullptr, *rl32 = nullptr, *ru32 = nullptr;
@@ -232,6 +238,8 @@ struct nir_pdhg {
     unsigned* gs_gen = nullptr;
     int* gs_err = nullptr;
     int launches = 0;
+    std::shared_ptr<ClusterPlan> cluster;  // one LP's plan (engine_cluster.cuh), built by its first solve in clusters
+    int cluster_size = -1;                 // its cluster size: 0 = not in clusters, -1 = not decided yet
     const double* last_x = nullptr;  // the point the last solve returned, still on the device (null before one)
     // the engine's row order: internal row k is the caller's row
     // row_orig[k] (empty: the caller's order; see row_order below)
@@ -270,6 +278,16 @@ struct nir_pdhg {
         bufs.push_back({p, bytes});
         device_bytes += (long long)bytes;
         return static_cast<T*>(p);
+    }
+
+    void release(void* p) {
+        for (auto it = bufs.begin(); it != bufs.end(); ++it)
+            if (it->p == p) {
+                device_bytes -= (long long)it->bytes;
+                cudaFree(it->p);
+                bufs.erase(it);
+                return;
+            }
     }
 
     ~nir_pdhg() {
@@ -598,15 +616,7 @@ void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
         NIR_CUDA(cudaMemcpyAsync(R.h_rp.data(), R.rp, (m + 1) * sizeof(int), cudaMemcpyDeviceToHost, s));
         NIR_CUDA(cudaStreamSynchronize(s));
         // scratch of the transpose is released right away
-        for (void* p : {(void*)col_of, (void*)ids, (void*)perm, (void*)keys_out, tmp, (void*)d_start}) {
-            for (auto it = h->bufs.begin(); it != h->bufs.end(); ++it)
-                if (it->p == p) {
-                    h->device_bytes -= (long long)it->bytes;
-                    cudaFree(it->p);
-                    h->bufs.erase(it);
-                    break;
-                }
-        }
+        for (void* p : {(void*)col_of, (void*)ids, (void*)perm, (void*)keys_out, tmp, (void*)d_start}) h->release(p);
     }
 
     // vectors
@@ -906,6 +916,27 @@ struct ChunkTimer {
     int prec = 0;  // 0: the timed chunk streams FP32 values, 1: FP64
 };
 
+// The controller's arguments that do not depend on the kernels before it.
+nir::CtlArgs control_args(const SolveCfg& cfg, int phase, double* hist) {
+    nir::CtlArgs ca{};
+    ca.tol = cfg.p.tol;
+    ca.feas_tol = cfg.p.feas_tol;
+    ca.K = cfg.K;
+    ca.restarts_on = cfg.restarts;
+    ca.mixed = (cfg.mixed && phase == 0) ? 1 : 0;
+    ca.phase = phase;
+    ca.suff = cfg.p.restart_sufficient;
+    ca.nec = cfg.p.restart_necessary;
+    ca.art = cfg.p.restart_artificial;
+    ca.theta = cfg.p.primal_weight_smoothing;
+    ca.polish_stall = cfg.p.polish_stall_checks;
+    ca.polish_switch = cfg.p.polish_switch_kkt;
+    ca.anchor_at_restart = cfg.p.restart_anchor ? 1 : 0;
+    ca.weight_decades = cfg.p.primal_weight_decades;
+    ca.hist = hist;
+    return ca;
+}
+
 // One launch chunk: K iterations (the last one a check), the KKT passes,
 // the controller, the restart copy and the status snapshot.  TV = type of
 // the matrix values, TX = type of the iterates, LP / LD = layouts of A' / A.
@@ -977,7 +1008,7 @@ void launch_fast_chunk_l(nir_pdhg* h, const SolveCfg& cfg, int phase, ChunkTimer
     int gkr = 0, gkc = 0;
     launch_kkt<TX>(h, phase, L.KR, L.KC, Vec<TX>::xp(h), Vec<TX>::yp(h), &gkr, &gkc);
     h->launches -= 2;  // counted with the chunk below
-    nir::CtlArgs ca;
+    nir::CtlArgs ca = control_args(cfg, phase, h->hist);
     ca.partP = L.P;
     ca.partD = L.D;
     ca.partKR = L.KR;
@@ -987,21 +1018,6 @@ void launch_fast_chunk_l(nir_pdhg* h, const SolveCfg& cfg, int phase, ChunkTimer
     ca.nKR = gkr;
     ca.nKC = gkc;
     ca.offset = h->offset;
-    ca.tol = cfg.p.tol;
-    ca.feas_tol = cfg.p.feas_tol;
-    ca.K = K;
-    ca.restarts_on = cfg.restarts;
-    ca.mixed = (cfg.mixed && phase == 0) ? 1 : 0;
-    ca.phase = phase;
-    ca.suff = cfg.p.restart_sufficient;
-    ca.nec = cfg.p.restart_necessary;
-    ca.art = cfg.p.restart_artificial;
-    ca.theta = cfg.p.primal_weight_smoothing;
-    ca.polish_stall = cfg.p.polish_stall_checks;
-    ca.polish_switch = cfg.p.polish_switch_kkt;
-    ca.anchor_at_restart = cfg.p.restart_anchor ? 1 : 0;
-    ca.weight_decades = cfg.p.primal_weight_decades;
-    ca.hist = h->hist;
     nir::k_control<<<1, nir::kBlock, 0, s>>>(ca, h->st);
     NIR_LAUNCHED();
     const int nm = std::max(h->n, h->m);
@@ -1055,8 +1071,10 @@ struct KeyHash {
 
 // prec: 0 = FP32 values and iterates, 1 = FP32 values with FP64 iterates,
 // 2 = FP64 values and iterates.
-unsigned long long chunk_key(const nir_pdhg* h, const SolveCfg& c, int phase, int prec) {
+// cl: the plan the chunk runs on, or null.
+unsigned long long chunk_key(const nir_pdhg* h, const SolveCfg& c, int phase, int prec, const ClusterPlan* cl) {
     KeyHash k;
+    k.add(cl);
     k.add(phase).add(prec).add(c.K).add(c.halpern).add(c.restarts).add(c.mixed);
     k.add(c.p.reflection).add(c.p.restart_sufficient).add(c.p.restart_necessary).add(c.p.restart_artificial);
     k.add(c.p.primal_weight_smoothing).add(c.p.polish_stall_checks).add(c.p.polish_switch_kkt).add(c.p.tol);
@@ -1337,7 +1355,9 @@ void precondition(nir_pdhg* h, const nir_pdhg_params& p, bool enable) {
         h->launches += 1;
         return;
     }
+    const long long version = sc.version + 1;
     sc = nir_pdhg::ScaleState{};
+    sc.version = version;
     nir::k_fill<<<grid_for(m), nir::kBlock, 0, s>>>(m, 1.0, h->dr);
     nir::k_fill<<<grid_for(n), nir::kBlock, 0, s>>>(n, 1.0, h->dc);
     NIR_LAUNCHED();
@@ -1557,19 +1577,28 @@ LayChoice pick_layouts(nir_pdhg* h, const nir_pdhg_params& p) {
     return c;
 }
 
+}  // namespace
+
+#include "engine_cluster.cuh"
+
+namespace {
+
 int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* ctx, double* x_out, double* y_out,
                nir_pdhg_info* info) {
     cudaStream_t s = h->stream;
     const double t0 = now_sec();
     const int n = h->n, m = h->m;
     const bool pdlp = p.algorithm == NIR_ALGO_PDLP;
-    use_layouts(h, pick_layouts(h, p));
+    ClusterPlan* const cl = cl_single(h, p);
+    if (!cl) use_layouts(h, pick_layouts(h, p));
     ensure_partials(h);
     // value / iterate precision of each phase: FP64 (double, double); MIXED
     // (float, double) then the FP64 polish; FP32 (float, float)
-    if (p.precision == NIR_PREC_FP32) warm_cfgs<float, float>(h);
-    if (p.precision == NIR_PREC_MIXED) warm_cfgs<float, double>(h);
-    if (p.precision != NIR_PREC_FP32) warm_cfgs<double, double>(h);
+    if (!cl) {
+        if (p.precision == NIR_PREC_FP32) warm_cfgs<float, float>(h);
+        if (p.precision == NIR_PREC_MIXED) warm_cfgs<float, double>(h);
+        if (p.precision != NIR_PREC_FP32) warm_cfgs<double, double>(h);
+    }
     SolveCfg cfg;
     cfg.p = p;
     cfg.K = std::max(1, p.check_every);
@@ -1597,7 +1626,7 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
 
     NIR_CUDA(cudaMemsetAsync(h->hist, 0, sizeof(double) * 8 * nir::kHist, s));
     precondition(h, p, pdlp && (p.ruiz_iters > 0 || p.pock_chambolle));
-    pad_scaled(h);
+    if (!cl) pad_scaled(h);
     nir::DevState st0{};
     st0.max_iters = p.max_iters;
     st0.best_kkt = INFINITY;
@@ -1673,6 +1702,7 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
         n, m, d_xin, d_yin, h->dc, h->dr, h->l64, h->u64, h->x64, h->x064, h->y64, h->y064, h->x32, h->x032, h->y32,
         h->y032, h->l32, h->u32);
     NIR_LAUNCHED();
+    if (cl) cl_load(h, *cl);
     // plain PDHG never reads the anchors in the update, but CHECK reads x0
     NIR_CUDA(cudaStreamSynchronize(s));
     const double t_setup = now_sec();
@@ -1691,13 +1721,14 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
         auto run_phase = [&](int phase, int prec) {
             auto launch = [&, phase, prec]() {
                 ChunkTimer* t = h->profiling ? &tm : nullptr;
-                if (prec == 2) launch_fast_chunk<double, double>(h, cfg, phase, t);
+                if (cl) launch_cluster_chunk(h, *cl, cfg, phase, prec == 2);
+                else if (prec == 2) launch_fast_chunk<double, double>(h, cfg, phase, t);
                 else if (prec == 1) launch_fast_chunk<float, double>(h, cfg, phase, t);
                 else launch_fast_chunk<float, float>(h, cfg, phase, t);
             };
-            const int per = launches_per_chunk(cfg.K, false);
+            const int per = cl ? 2 : launches_per_chunk(cfg.K, false);
             if (p.use_graphs && !h->profiling && !cfg.persistent) {
-                cudaGraphExec_t ge = chunk_graph(h, 1 + phase, chunk_key(h, cfg, phase, prec), launch);
+                cudaGraphExec_t ge = chunk_graph(h, 1 + phase, chunk_key(h, cfg, phase, prec, cl), launch);
                 return run_chunks(h, p, poll, ctx, t0, phase, per, [&]() { NIR_CUDA(cudaGraphLaunch(ge, s)); }, nullptr);
             }
             return run_chunks(h, p, poll, ctx, t0, phase, 0, launch, h->profiling ? &tm : nullptr);
@@ -1750,6 +1781,7 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
         for (auto& e : tm.e) cudaEventDestroy(e);
     nir::DevState st;
     d2h(h, &st, h->st, sizeof(st));
+    if (cl && p.max_iters > 0) cl_store_out(h, *cl, nullptr, nullptr);
     const bool out64 = p.precision != NIR_PREC_FP32;
     const unsigned g = std::max(grid_for(std::max(n, m)), 1u);
     if (out64) nir::k_unscale_out<double><<<g, nir::kBlock, 0, s>>>(n, m, h->xp64, h->yp64, h->dc, h->dr, h->out_x, h->out_y);
@@ -1777,7 +1809,7 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
     info->solve_seconds = now_sec() - t_setup;
     info->time_to_fp64_seconds = t_switch;
     info->iterations_to_tol = (status == NIR_STATUS_OPTIMAL) ? st.iter : -1;
-    if (status == NIR_STATUS_INTERNAL_ERROR) g_err = "a grid barrier of the persistent chunk kernel exceeded its wait bound";
+    if (status == NIR_STATUS_INTERNAL_ERROR) g_err = "a wait inside a chunk kernel exceeded its bound";
     return status;
 }
 
@@ -2323,6 +2355,14 @@ int nir_pdhg_kernel_times(nir_pdhg* h, nir_pdhg_kernel_time* out) {
 
 namespace {
 
+// The per-launch kernels' layouts on a handle whose solves ran in clusters:
+// the default warp row blocks and the scaled values in them.
+void ensure_kernel_layouts(nir_pdhg* h) {
+    if (!h->cluster || (h->A.lay >= 0 && h->At.lay >= 0)) return;
+    use_layouts(h, default_layouts(h));
+    pad_scaled(h);
+}
+
 // Steady-state timing of the fused iteration kernels of one precision on
 // the handle's current state: `reps` back-to-back launches of k_primal
 // alone, of k_dual alone, and of reps (k_primal, k_dual) pairs, each batch
@@ -2415,6 +2455,7 @@ int nir_pdhg_time_iteration(nir_pdhg* h, int precision, int reps, double* primal
     if (h->inner) h = h->inner.get();  // PDHG / PDLP solves ran on the equivalent LP
     try {
         NIR_CUDA(cudaSetDevice(h->device));
+        ensure_kernel_layouts(h);
         if (h->A.lay < 0 || h->At.lay < 0)
             throw std::invalid_argument("no PDHG / PDLP solve has set up the iteration kernels yet");
         if (h->last_x == h->x64) h->last_x = nullptr;  // a reference-loop result the kernels would overwrite
@@ -2464,7 +2505,14 @@ int nir_pdhg_get_layout(nir_pdhg* h, nir_pdhg_layout* out) {
     out->nrow = h->m;
     out->ncol = h->n;
     out->nnz = h->nnz;
-    const nir_pdhg* src = h->inner ? h->inner.get() : h;  // PDHG / PDLP solves ran on the equivalent LP
+    nir_pdhg* src = h->inner ? h->inner.get() : h;  // PDHG / PDLP solves ran on the equivalent LP
+    try {
+        NIR_CUDA(cudaSetDevice(src->device));
+        ensure_kernel_layouts(src);
+    } catch (const std::exception& e) {
+        g_err = e.what();
+        return NIR_STATUS_INTERNAL_ERROR;
+    }
     out->blocks_a = src->A.lay >= 0 ? lay_nblk(src->A) : 0;
     out->blocks_at = src->At.lay >= 0 ? lay_nblk(src->At) : 0;
     out->block_nnz = src->A.lay == nir::kLayCta ? kCtaCap : src->A.cap;

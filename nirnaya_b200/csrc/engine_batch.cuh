@@ -38,6 +38,9 @@ struct nir_pdhg_batch {
     int *d_act_inst = nullptr, *d_act_off_a = nullptr, *d_act_off_at = nullptr, *d_act_n = nullptr;
     double *d_bnorm = nullptr, *d_cnorm = nullptr, *d_offset = nullptr, *d_norm = nullptr;
     ChunkGraph graphs[2];
+    std::unique_ptr<ClusterPlan> cluster;  // engine_cluster.cuh, built by the first solve that can use it
+    bool cluster_tried = false;
+    const unsigned char* in_cluster = nullptr;  // [instance], device: solved by the plan in use (null: none)
     bool solved = false;  // h->out_x holds the points the last batch solve returned
     ~nir_pdhg_batch() {
         if (h && h->device >= 0) cudaSetDevice(h->device);
@@ -141,8 +144,8 @@ nir::BatchArgs bargs(nir_pdhg_batch* B, bool transpose, double* part, int i, int
 // use (after the states are set, and after every check).
 void launch_bcompact(nir_pdhg_batch* B) {
     nir_pdhg* h = B->h;
-    nir::k_bcompact<<<1, nir::kBlock, 0, h->stream>>>(B->count, B->insts, B->cur->a.lo, B->cur->at.lo, B->d_act_inst,
-                                                      B->d_act_off_a, B->d_act_off_at, B->d_act_n);
+    nir::k_bcompact<<<1, nir::kBlock, 0, h->stream>>>(B->count, B->insts, B->in_cluster, B->cur->a.lo, B->cur->at.lo,
+                                                      B->d_act_inst, B->d_act_off_a, B->d_act_off_at, B->d_act_n);
     NIR_LAUNCHED();
     h->launches += 1;
 }
@@ -230,38 +233,32 @@ void launch_batch_chunk_l(nir_pdhg_batch* B, const SolveCfg& cfg, int phase) {
     nir::k_bkkt_cols<LP, TX><<<gkc, nir::kBlock, lay_smem<LP, double>(), s>>>(kc, LT.v64, Vec<TX>::xp(h),
                                                                              Vec<TX>::yp(h), h->dc, h->c, h->l, h->u);
     NIR_LAUNCHED();
-    nir::CtlArgs ca{};
-    ca.K = K;
-    ca.tol = cfg.p.tol;
-    ca.feas_tol = cfg.p.feas_tol;
-    ca.restarts_on = cfg.restarts;
-    ca.mixed = (cfg.mixed && phase == 0) ? 1 : 0;
-    ca.phase = phase;
-    ca.suff = cfg.p.restart_sufficient;
-    ca.nec = cfg.p.restart_necessary;
-    ca.art = cfg.p.restart_artificial;
-    ca.theta = cfg.p.primal_weight_smoothing;
-    ca.polish_stall = cfg.p.polish_stall_checks;
-    ca.polish_switch = cfg.p.polish_switch_kkt;
-    ca.anchor_at_restart = cfg.p.restart_anchor ? 1 : 0;
-    ca.weight_decades = cfg.p.primal_weight_decades;
-    ca.hist = nullptr;
-    nir::BatchCtlArgs cb{P, D, KR, KC, LT.nblk, LA.nblk, LT.lo, LA.lo, B->d_bnorm, B->d_cnorm, B->d_offset};
+    const nir::CtlArgs ca = control_args(cfg, phase, nullptr);
+    nir::BatchCtlArgs cb{P, D, KR, KC, LT.nblk, LA.nblk, LT.lo, LA.lo, B->d_bnorm, B->d_cnorm, B->d_offset, B->in_cluster};
     nir::k_bcontrol<<<B->count, nir::kBlock, 0, s>>>(ca, cb, B->insts);
     nir::k_bapply_restart<TX><<<grid_for(std::max(h->n, h->m)), nir::kBlock, 0, s>>>(
-        h->n, h->m, B->d_col_inst, B->d_row_inst, B->insts, phase, Vec<TX>::x(h), Vec<TX>::x0(h), Vec<TX>::xp(h),
+        h->n, h->m, B->d_col_inst, B->d_row_inst, B->insts, B->in_cluster, phase, Vec<TX>::x(h), Vec<TX>::x0(h), Vec<TX>::xp(h),
         Vec<TX>::y(h), Vec<TX>::y0(h), Vec<TX>::yp(h));
     launch_bcompact(B);  // the next chunk visits the blocks of the instances still running
-    nir::k_bsnap<<<1, nir::kBlock, 0, s>>>(B->count, B->insts, h->snap.ring, h->snap.d_seq);
-    NIR_LAUNCHED();
-    h->launches += 7;
+    h->launches += 6;
 }
 
+// The instances of the cluster plan in use, if any, then the others.
 template <typename TV, typename TX>
 void launch_batch_chunk(nir_pdhg_batch* B, const SolveCfg& cfg, int phase) {
-    with_batch_lays(B, [&](auto lp, auto ld) {
-        launch_batch_chunk_l<TV, TX, decltype(lp)::value, decltype(ld)::value>(B, cfg, phase);
-    });
+    nir_pdhg* h = B->h;
+    if constexpr (sizeof(TX) == 8) {
+        if (B->in_cluster)
+            cl_launch<TV>(h, *B->cluster, control_args(cfg, phase, nullptr), cfg.K, 1, phase, cfg.p.reflection, B->insts,
+                          B->d_bnorm, B->d_cnorm, B->d_offset);
+    }
+    if (B->cur)
+        with_batch_lays(B, [&](auto lp, auto ld) {
+            launch_batch_chunk_l<TV, TX, decltype(lp)::value, decltype(ld)::value>(B, cfg, phase);
+        });
+    nir::k_bsnap<<<1, nir::kBlock, 0, h->stream>>>(B->count, B->insts, h->snap.ring, h->snap.d_seq);
+    NIR_LAUNCHED();
+    h->launches += 1;
 }
 
 template <typename TV, typename TX>
@@ -370,12 +367,23 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
     if (p.algorithm != NIR_ALGO_PDLP) throw std::invalid_argument("the batch runs NIR_ALGO_PDLP only");
     if (p.check_every < 1 || p.reflection < 0.0 || p.reflection > 1.0 || !(p.tol >= 0.0))
         throw std::invalid_argument("invalid parameters");
+    // clusters for the instances that fit one, where the solve takes them
+    const bool may = cl_takes(h, p);
+    if (may && !B->cluster_tried) {
+        B->cluster_tried = true;
+        B->cluster = cl_batch(h, B->row_off, B->col_off, B->d_row_off, B->d_col_off, B->d_row_inst, B->d_col_inst);
+    }
+    ClusterPlan* const cl = may ? B->cluster.get() : nullptr;
+    B->in_cluster = cl ? cl->d_member : nullptr;
+    const bool all = cl && cl->members == I;
     // layouts timed on the block-diagonal matrix, then built per instance
-    const LayChoice lc = pick_layouts(h, p);
+    const LayChoice lc = all ? LayChoice{} : pick_layouts(h, p);
     auto same = [](const LayChoice& a, const LayChoice& b) {
         return a.lay_a == b.lay_a && a.cap_a == b.cap_a && a.lay_at == b.lay_at && a.cap_at == b.cap_at;
     };
-    if (!B->cur || !same(B->cur->choice, lc)) {
+    if (all) {
+        B->cur = nullptr;
+    } else if (!B->cur || !same(B->cur->choice, lc)) {
         B->cur = nullptr;
         for (auto& l : B->layouts)
             if (same(l.choice, lc)) B->cur = &l;
@@ -410,7 +418,7 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
         }
     }
     precondition(h, p, p.ruiz_iters > 0 || p.pock_chambolle);
-    batch_pad_values(B);
+    if (B->cur) batch_pad_values(B);
     // per-instance ||A_i||_2 by power iteration on the block-diagonal matrix
     const unsigned gwm = grid_for((long long)m * 32), gwn = grid_for((long long)n * 32);
     nir::k_power_start_batch<<<grid_for(n), nir::kBlock, 0, s>>>(n, B->d_col_inst, B->d_col_off, h->tmp_n);
@@ -457,7 +465,7 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
         bn[i] = std::sqrt(bo.hi + bo.lo);
     }
     h2d(h, B->insts, st0.data(), I * sizeof(nir::DevState));
-    launch_bcompact(B);
+    if (B->cur) launch_bcompact(B);
     h2d(h, B->d_bnorm, bn.data(), I * sizeof(double));
     h2d(h, B->d_cnorm, cn.data(), I * sizeof(double));
     h2d(h, B->d_offset, B->offsets.data(), I * sizeof(double));
@@ -465,10 +473,11 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
         n, m, nullptr, nullptr, h->dc, h->dr, h->l64, h->u64, h->x64, h->x064, h->y64, h->y064, h->x32, h->x032,
         h->y32, h->y032, h->l32, h->u32);
     NIR_LAUNCHED();
+    if (cl) cl_load(h, *cl);
     // occupancy queries before any capture
-    if (p.precision == NIR_PREC_FP32) warm_batch_cfgs<float, float>(B);
-    if (p.precision == NIR_PREC_MIXED) warm_batch_cfgs<float, double>(B);
-    if (p.precision != NIR_PREC_FP32) warm_batch_cfgs<double, double>(B);
+    if (B->cur && p.precision == NIR_PREC_FP32) warm_batch_cfgs<float, float>(B);
+    if (B->cur && p.precision == NIR_PREC_MIXED) warm_batch_cfgs<float, double>(B);
+    if (B->cur && p.precision != NIR_PREC_FP32) warm_batch_cfgs<double, double>(B);
     NIR_CUDA(cudaStreamSynchronize(s));
     const double t_setup = now_sec();
     const bool fp64_first = (p.precision == NIR_PREC_FP64);
@@ -479,11 +488,14 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
             else if (prec == 1) launch_batch_chunk<float, double>(B, cfg, phase);
             else launch_batch_chunk<float, float>(B, cfg, phase);
         };
-        const int per = 2 * cfg.K + 7;
+        const int per = (cl ? 1 : 0) + (B->cur ? 2 * cfg.K + 6 : 0) + 1;
         if (p.use_graphs && !cfg.persistent) {
             KeyHash k;
-            k.add(chunk_key(h, cfg, phase, prec)).add(B->cur->a.blk).add(B->cur->at.blk).add(B->cur->a.lay);
-            k.add(B->cur->at.lay).add(B->cur->a.cap).add(B->cur->at.cap).add(B->cur->part).add(B->insts);
+            k.add(chunk_key(h, cfg, phase, prec, cl)).add(B->insts);
+            if (B->cur) {
+                k.add(B->cur->a.blk).add(B->cur->at.blk).add(B->cur->a.lay).add(B->cur->at.lay);
+                k.add(B->cur->a.cap).add(B->cur->at.cap).add(B->cur->part);
+            }
             ChunkGraph& g = B->graphs[phase];
             if (!(g.ge && g.valid && g.key == k.h)) {
                 // capture into the handle's slot, then keep it with the batch
@@ -512,6 +524,7 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
     }
     std::vector<nir::DevState> st(I);
     d2h(h, st.data(), B->insts, I * sizeof(nir::DevState));
+    if (cl && p.max_iters > 0) cl_store_out(h, *cl, B->d_col_inst, B->d_row_inst);
     nir::k_bunscale_out<<<grid_for(std::max(n, m)), nir::kBlock, 0, s>>>(
         n, m, B->d_col_inst, B->d_row_inst, B->insts, h->xp32, h->yp32, h->xp64, h->yp64,
         p.precision != NIR_PREC_FP32 ? 1 : 0, h->dc,

@@ -51,9 +51,11 @@ __device__ __forceinline__ int visited_block(const BatchArgs& a, int v, int nact
     return __ldg(a.blk_lo + inst) + (v - __ldg(a.act_off + lo));
 }
 
-// Lists the running instances (not done, in either phase) and the prefix of
-// their block counts in both orientations.  One CTA; a fixed scan order.
+// Lists the running instances (not done, in either phase; not those that
+// `skip` marks, which clusters run) and the prefix of their block counts in
+// both orientations.  One CTA; a fixed scan order.
 __global__ void __launch_bounds__(kBlock) k_bcompact(int count, const DevState* __restrict__ insts,
+                                                     const unsigned char* __restrict__ skip,
                                                      const int* __restrict__ a_lo, const int* __restrict__ at_lo,
                                                      int* __restrict__ act_inst, int* __restrict__ act_off_a,
                                                      int* __restrict__ act_off_at, int* __restrict__ act_n) {
@@ -64,7 +66,7 @@ __global__ void __launch_bounds__(kBlock) k_bcompact(int count, const DevState* 
     __syncthreads();
     for (int base = 0; base < count; base += kBlock) {
         const int i = base + threadIdx.x;
-        const bool run = i < count && !insts[i].done;
+        const bool run = i < count && !insts[i].done && !(skip && skip[i]);
         int v[3] = {run ? 1 : 0, run ? a_lo[i + 1] - a_lo[i] : 0, run ? at_lo[i + 1] - at_lo[i] : 0};
         int incl[3];
 #pragma unroll
@@ -284,6 +286,7 @@ struct BatchCtlArgs {
     const double* bnorm;   // per instance, original space
     const double* cnorm;
     const double* offset;
+    const unsigned char* skip;  // instances that clusters run, or null
 };
 
 __device__ inline double range_sum(const double* __restrict__ p, int lo, int hi, double* sh) {
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(kBlock) k_bcontrol(CtlArgs a, BatchCtlArgs b, 
     __shared__ double sh[kWarps];
     const int i = blockIdx.x;
     DevState* st = insts + i;
-    if (st->done || st->phase != a.phase) return;
+    if (st->done || st->phase != a.phase || (b.skip && b.skip[i])) return;
     const int p0 = b.at_lo[i], p1 = b.at_lo[i + 1], d0 = b.a_lo[i], d1 = b.a_lo[i + 1];
     CtlSums s;
     s.dx2 = range_sum(b.partP, p0, p1, sh);
@@ -324,13 +327,13 @@ __global__ void __launch_bounds__(kBlock) k_bcontrol(CtlArgs a, BatchCtlArgs b, 
 
 template <typename T>
 __global__ void k_bapply_restart(int n, int m, const int* __restrict__ col_inst, const int* __restrict__ row_inst,
-                                 const DevState* __restrict__ insts, int phase, T* __restrict__ x, T* __restrict__ x0,
-                                 const T* __restrict__ xplus, T* __restrict__ y, T* __restrict__ y0,
-                                 const T* __restrict__ yplus) {
+                                 const DevState* __restrict__ insts, const unsigned char* __restrict__ skip, int phase,
+                                 T* __restrict__ x, T* __restrict__ x0, const T* __restrict__ xplus, T* __restrict__ y,
+                                 T* __restrict__ y0, const T* __restrict__ yplus) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) {
         const DevState& s = insts[col_inst[t]];
-        if (s.apply_restart && !s.done && s.phase == phase) {
+        if (s.apply_restart && !s.done && s.phase == phase && !(skip && skip[col_inst[t]])) {
             const T v = xplus[t];
             x[t] = v;
             x0[t] = v;
@@ -338,7 +341,7 @@ __global__ void k_bapply_restart(int n, int m, const int* __restrict__ col_inst,
     }
     if (t < m) {
         const DevState& s = insts[row_inst[t]];
-        if (s.apply_restart && !s.done && s.phase == phase) {
+        if (s.apply_restart && !s.done && s.phase == phase && !(skip && skip[row_inst[t]])) {
             const T v = yplus[t];
             y[t] = v;
             y0[t] = v;
