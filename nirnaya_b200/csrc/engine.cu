@@ -133,6 +133,7 @@ struct Orient {
     float* v32 = nullptr;
     float* v32_orig = nullptr;  // for the FP32 SpMV test entry point
     std::vector<int> h_rp;
+    int max_len = -1;  // longest row, counted on first use
     int cap = 0;
     int nblk = 0;
     int2* blk = nullptr;  // (first row, first nonzero) of each row block, plus an end entry
@@ -239,6 +240,13 @@ struct nir_pdhg {
     int* gs_err = nullptr;
     int launches = 0;
     std::shared_ptr<ClusterPlan> cluster;  // one LP's plan (engine_cluster.cuh), built by its first solve in clusters
+    // one LP as the instance-wise kernels see it ({0, m}, {0, n}), and their
+    // partial sums and results (dd_sums)
+    int *one_row = nullptr, *one_col = nullptr;
+    nir::vfy::DD* dd_part = nullptr;
+    size_t dd_len = 0;
+    double* dd_out = nullptr;
+    size_t dd_out_len = 0;
     int cluster_size = -1;                 // its cluster size: 0 = not in clusters, -1 = not decided yet
     const double* last_x = nullptr;  // the point the last solve returned, still on the device (null before one)
     // the engine's row order: internal row k is the caller's row
@@ -1342,6 +1350,96 @@ int solve_reference(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), v
 
 // ---------------------------------------------------------------- PDHG / PDLP
 
+// Lanes per row of the set-up kernels: a power of two near a quarter of the
+// mean row length, a warp where a row is so long that fewer lanes would
+// finish on it.
+int row_lanes(Orient& o) {
+    if (o.max_len < 0) {
+        o.max_len = 0;
+        for (int r = 0; r < o.rows; ++r) o.max_len = std::max(o.max_len, o.h_rp[size_t(r) + 1] - o.h_rp[size_t(r)]);
+    }
+    const double mean = o.rows > 0 ? double(o.nnz) / double(o.rows) : 0.0;
+    int t = 1;
+    while (t < 32 && 4 * t < mean) t *= 2;
+    return o.max_len > 64 * t ? 32 : t;
+}
+
+// Calls f with the lanes as a std::integral_constant.
+template <class F>
+void with_lanes(int t, F&& f) {
+    switch (t) {
+        case 1: f(std::integral_constant<int, 1>{}); break;
+        case 2: f(std::integral_constant<int, 2>{}); break;
+        case 4: f(std::integral_constant<int, 4>{}); break;
+        case 8: f(std::integral_constant<int, 8>{}); break;
+        case 16: f(std::integral_constant<int, 16>{}); break;
+        default: f(std::integral_constant<int, 32>{}); break;
+    }
+}
+
+// y = A x / norm of the row's instance on the scaled FP64 values.
+void power_spmv(nir_pdhg* h, const Orient& o, int lanes, const double* x, const double* norm, const int* inst_of,
+                double* y) {
+    with_lanes(lanes, [&](auto t) {
+        constexpr int T = decltype(t)::value;
+        nir::k_power_spmv<T><<<grid_for((long long)o.rows * T), nir::kBlock, 0, h->stream>>>(o.rows, o.rp, o.ci, o.v64, x,
+                                                                                            norm, inst_of, y);
+    });
+}
+
+// Double-double sums per instance (k_setup.cuh), Q results each, copied to
+// `out` on the host: launch(G, part) leaves G partial sums per instance.
+// base: what each sum starts from (device), or null.
+template <class F>
+void dd_sums(nir_pdhg* h, int count, int Q, const double* base, double* out, F&& launch) {
+    // enough CTAs for the device, at most 128 per instance
+    const int G = std::max(1, std::min(128, 4 * h->sms / count));
+    const size_t need = size_t(count) * G * Q;
+    if (need > h->dd_len) {
+        h->release(h->dd_part);
+        h->dd_part = h->alloc<nir::vfy::DD>(need);
+        h->dd_len = need;
+    }
+    const size_t res = size_t(count) * Q;
+    if (res > h->dd_out_len) {
+        h->release(h->dd_out);
+        h->dd_out = h->alloc<double>(res);
+        h->dd_out_len = res;
+    }
+    launch(G, h->dd_part);
+    nir::k_dd_finish<<<grid_for((long long)res), nir::kBlock, 0, h->stream>>>(count, G, Q, h->dd_part, base, h->dd_out);
+    NIR_LAUNCHED();
+    h->launches += 2;
+    d2h(h, out, h->dd_out, res * sizeof(double));
+}
+
+// The norms of each instance: ||c||, ||c scaled||, ||b||, ||b scaled||
+// (after a preconditioning, which set the scales).
+void lp_norms(nir_pdhg* h, int count, const int* row_off, const int* col_off, double* out) {
+    dd_sums(h, count, nir::kDdNorms, nullptr, out, [&](int G, nir::vfy::DD* part) {
+        nir::k_dd_norms<<<unsigned(count) * unsigned(G), nir::kBlock, 0, h->stream>>>(G, row_off, col_off, h->c, h->dc,
+                                                                                     h->rl, h->ru, h->dr, part);
+    });
+    for (int k = 0; k < count * nir::kDdNorms; ++k) out[k] = std::sqrt(out[k]);
+}
+
+// Each instance's objective at the point x on the device.
+void lp_objectives(nir_pdhg* h, int count, const int* col_off, const double* offsets, const double* x, double* out) {
+    dd_sums(h, count, 1, offsets, out, [&](int G, nir::vfy::DD* part) {
+        nir::k_dd_objective<<<unsigned(count) * unsigned(G), nir::kBlock, 0, h->stream>>>(G, col_off, h->c, x, part);
+    });
+}
+
+// One LP's offsets for the instance-wise kernels.
+void one_instance(nir_pdhg* h) {
+    if (h->one_row) return;
+    int* p = h->alloc<int>(4);
+    const int o[4] = {0, h->m, 0, h->n};
+    h2d(h, p, o, sizeof(o));
+    h->one_row = p;
+    h->one_col = p + 2;
+}
+
 void precondition(nir_pdhg* h, const nir_pdhg_params& p, bool enable) {
     cudaStream_t s = h->stream;
     const int n = h->n, m = h->m;
@@ -1363,12 +1461,26 @@ void precondition(nir_pdhg* h, const nir_pdhg_params& p, bool enable) {
     NIR_LAUNCHED();
     if (enable) {
         const unsigned gwm = grid_for((long long)m * 32), gwn = grid_for((long long)n * 32);
+        const int lm = row_lanes(h->A), ln = row_lanes(h->At);
         for (int it = 0; it < p.ruiz_iters + (p.pock_chambolle ? 1 : 0); ++it) {
             const int mode = it < p.ruiz_iters ? 0 : 1;  // 0 = l-inf (Ruiz), 1 = l1 (Pock-Chambolle)
-            nir::k_row_stat<<<std::max(gwm, 1u), nir::kBlock, 0, s>>>(m, h->A.rp, h->A.ci, h->A.v_orig, h->dr, h->dc, mode,
-                                                                     h->tmp_m);
-            nir::k_row_stat<<<std::max(gwn, 1u), nir::kBlock, 0, s>>>(n, h->At.rp, h->At.ci, h->At.v_orig, h->dc, h->dr,
-                                                                     mode, h->tmp_n);
+            if (mode == 0) {
+                with_lanes(lm, [&](auto t) {
+                    constexpr int T = decltype(t)::value;
+                    nir::k_row_max<T><<<grid_for((long long)m * T), nir::kBlock, 0, s>>>(m, h->A.rp, h->A.ci, h->A.v_orig,
+                                                                                         h->dr, h->dc, h->tmp_m);
+                });
+                with_lanes(ln, [&](auto t) {
+                    constexpr int T = decltype(t)::value;
+                    nir::k_row_max<T><<<grid_for((long long)n * T), nir::kBlock, 0, s>>>(
+                        n, h->At.rp, h->At.ci, h->At.v_orig, h->dc, h->dr, h->tmp_n);
+                });
+            } else {
+                nir::k_row_stat<<<std::max(gwm, 1u), nir::kBlock, 0, s>>>(m, h->A.rp, h->A.ci, h->A.v_orig, h->dr, h->dc,
+                                                                         mode, h->tmp_m);
+                nir::k_row_stat<<<std::max(gwn, 1u), nir::kBlock, 0, s>>>(n, h->At.rp, h->At.ci, h->At.v_orig, h->dc,
+                                                                         h->dr, mode, h->tmp_n);
+            }
             nir::k_apply_stat<<<grid_for(m), nir::kBlock, 0, s>>>(m, h->tmp_m, h->dr);
             nir::k_apply_stat<<<grid_for(n), nir::kBlock, 0, s>>>(n, h->tmp_n, h->dc);
             NIR_LAUNCHED();
@@ -1400,22 +1512,25 @@ double power_norm(nir_pdhg* h, int rounds) {
     auto& sc = h->scaled;
     if (sc.valid && sc.norm_valid && sc.power_iters == rounds) return sc.norm;
     cudaStream_t s = h->stream;
-    const int n = h->n, m = h->m;
+    const int n = h->n;
     const PartLayout L = part_layout(h);
-    const unsigned gwm = grid_for((long long)m * 32), gwn = grid_for((long long)n * 32);
+    double* norm_est = &h->st->ref_norm_est;
+    const int lm = row_lanes(h->A), ln = row_lanes(h->At);
+    one_instance(h);
+    const int G = int(std::min(grid_for(n), 128u));
+    auto measure = [&]() {
+        nir::k_seg_sumsq<<<unsigned(G), nir::kBlock, 0, s>>>(G, h->one_col, h->tmp_n, L.misc);
+        nir::k_seg_norm<<<1, 32, 0, s>>>(1, G, L.misc, norm_est);
+    };
     nir::k_power_start<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->tmp_n);
-    nir::k_sumsq_partials<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->tmp_n, L.misc);
-    nir::k_norm_finalize<<<1, nir::kBlock, 0, s>>>(L.misc, std::max<int>(grid_for(n), 1), h->st);
-    nir::k_scale_by_inv_norm<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->tmp_n, h->st);
+    measure();
     NIR_LAUNCHED();
     for (int r = 0; r < rounds; ++r) {
-        nir::k_spmv_warp64<<<std::max(gwm, 1u), nir::kBlock, 0, s>>>(m, h->A.rp, h->A.ci, h->A.v64, h->tmp_n, h->tmp_m);
-        nir::k_spmv_warp64<<<std::max(gwn, 1u), nir::kBlock, 0, s>>>(n, h->At.rp, h->At.ci, h->At.v64, h->tmp_m, h->tmp_n);
-        nir::k_sumsq_partials<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->tmp_n, L.misc);
-        nir::k_norm_finalize<<<1, nir::kBlock, 0, s>>>(L.misc, std::max<int>(grid_for(n), 1), h->st);
-        nir::k_scale_by_inv_norm<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->tmp_n, h->st);
+        power_spmv(h, h->A, lm, h->tmp_n, norm_est, nullptr, h->tmp_m);
+        power_spmv(h, h->At, ln, h->tmp_m, nullptr, nullptr, h->tmp_n);
+        measure();
         NIR_LAUNCHED();
-        h->launches += 5;
+        h->launches += 4;
     }
     nir::DevState st;
     NIR_CUDA(cudaMemcpyAsync(&st, h->st, sizeof(st), cudaMemcpyDeviceToHost, s));
@@ -1620,13 +1735,16 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
             NIR_CUDA(cudaMemsetAsync(h->gs_err, 0, sizeof(int), s));
         }
     }
-    cfg.bnorm = rhs_norm(h);
-    cfg.cnorm = norm2(h->h_c);
     h->ktime = nir_pdhg_kernel_time{};
 
     NIR_CUDA(cudaMemsetAsync(h->hist, 0, sizeof(double) * 8 * nir::kHist, s));
     precondition(h, p, pdlp && (p.ruiz_iters > 0 || p.pock_chambolle));
     if (!cl) pad_scaled(h);
+    double nrm[nir::kDdNorms];
+    one_instance(h);
+    lp_norms(h, 1, h->one_row, h->one_col, nrm);
+    cfg.cnorm = nrm[0];
+    cfg.bnorm = nrm[2];
     nir::DevState st0{};
     st0.max_iters = p.max_iters;
     st0.best_kkt = INFINITY;
@@ -1637,19 +1755,7 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
         const double sig = power_norm(h, std::max(1, p.power_iters));
         eta = p.step_factor / std::max(sig, 1e-30);
         // primal weight: ||c^|| / ||b^|| in the scaled space
-        std::vector<double> dc(n), dr(m);
-        d2h(h, dc.data(), h->dc, n * sizeof(double));
-        d2h(h, dr.data(), h->dr, m * sizeof(double));
-        DD cs, bs;
-        for (int j = 0; j < n; ++j) cs = dd_add_prod(cs, h->h_c[j] * dc[j], h->h_c[j] * dc[j]);
-        for (int i = 0; i < m; ++i) {
-            double b = 0.0;
-            if (std::isfinite(h->h_rl[i])) b = std::fabs(h->h_rl[i]);
-            if (std::isfinite(h->h_ru[i])) b = std::max(b, std::fabs(h->h_ru[i]));
-            b *= dr[i];
-            bs = dd_add_prod(bs, b, b);
-        }
-        const double cn = std::sqrt(cs.hi + cs.lo), bn = std::sqrt(bs.hi + bs.lo);
+        const double cn = nrm[1], bn = nrm[3];
         omega = (cn > 1e-10 && bn > 1e-10) ? cn / bn : 1.0;
         if (p.omega_init > 0.0) omega = p.omega_init;
         st0.eta = eta;
@@ -1787,12 +1893,9 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
     if (out64) nir::k_unscale_out<double><<<g, nir::kBlock, 0, s>>>(n, m, h->xp64, h->yp64, h->dc, h->dr, h->out_x, h->out_y);
     else nir::k_unscale_out<float><<<g, nir::kBlock, 0, s>>>(n, m, h->xp32, h->yp32, h->dc, h->dr, h->out_x, h->out_y);
     NIR_LAUNCHED();
-    std::vector<double> x(n), y(m);
-    NIR_CUDA(cudaMemcpyAsync(x.data(), h->out_x, n * sizeof(double), cudaMemcpyDeviceToHost, s));
-    NIR_CUDA(cudaMemcpyAsync(y.data(), h->out_y, m * sizeof(double), cudaMemcpyDeviceToHost, s));
-    NIR_CUDA(cudaStreamSynchronize(s));
-    if (x_out) std::memcpy(x_out, x.data(), n * sizeof(double));
-    if (y_out) std::memcpy(y_out, y.data(), m * sizeof(double));
+    if (x_out) NIR_CUDA(cudaMemcpyAsync(x_out, h->out_x, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+    if (y_out) NIR_CUDA(cudaMemcpyAsync(y_out, h->out_y, m * sizeof(double), cudaMemcpyDeviceToHost, s));
+    lp_objectives(h, 1, h->one_col, nullptr, h->out_x, &info->objective);
     h->last_x = h->out_x;
     int status;
     if (st.done) status = st.status;
@@ -1804,7 +1907,6 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
     info->iterations = st.iter;
     h->last_iters = st.iter;
     if (fp64_first) info->iterations_fp64 = st.iter;
-    info->objective = host_objective(h, x);
     info->setup_seconds = t_setup - t0;
     info->solve_seconds = now_sec() - t_setup;
     info->time_to_fp64_seconds = t_switch;

@@ -36,7 +36,7 @@ struct nir_pdhg_batch {
     nir::DevState* insts = nullptr;
     // the running instances and their block prefixes (k_bcompact)
     int *d_act_inst = nullptr, *d_act_off_a = nullptr, *d_act_off_at = nullptr, *d_act_n = nullptr;
-    double *d_bnorm = nullptr, *d_cnorm = nullptr, *d_offset = nullptr, *d_norm = nullptr;
+    double *d_bnorm = nullptr, *d_cnorm = nullptr, *d_offset = nullptr, *d_norm = nullptr, *d_norm_part = nullptr;
     ChunkGraph graphs[2];
     std::unique_ptr<ClusterPlan> cluster;  // engine_cluster.cuh, built by the first solve that can use it
     bool cluster_tried = false;
@@ -355,6 +355,7 @@ void batch_create_impl(nir_pdhg_batch* B, const nir_lp_view* lps, int count, int
     B->d_cnorm = h->alloc<double>(count);
     B->d_offset = h->alloc<double>(count);
     B->d_norm = h->alloc<double>(count);
+    B->d_norm_part = h->alloc<double>(8 * size_t(count));
 }
 
 int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(void*), void* ctx, double* x_out,
@@ -420,37 +421,28 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
     precondition(h, p, p.ruiz_iters > 0 || p.pock_chambolle);
     if (B->cur) batch_pad_values(B);
     // per-instance ||A_i||_2 by power iteration on the block-diagonal matrix
-    const unsigned gwm = grid_for((long long)m * 32), gwn = grid_for((long long)n * 32);
+    constexpr int G = 8;  // CTAs per instance of the norms
+    const int lm = row_lanes(h->A), ln = row_lanes(h->At);
+    auto measure = [&]() {
+        nir::k_seg_sumsq<<<unsigned(I) * G, nir::kBlock, 0, s>>>(G, B->d_col_off, h->tmp_n, B->d_norm_part);
+        nir::k_seg_norm<<<grid_for(I * 32LL), nir::kBlock, 0, s>>>(I, G, B->d_norm_part, B->d_norm);
+    };
     nir::k_power_start_batch<<<grid_for(n), nir::kBlock, 0, s>>>(n, B->d_col_inst, B->d_col_off, h->tmp_n);
-    nir::k_seg_norm<<<I, nir::kBlock, 0, s>>>(B->d_col_off, h->tmp_n, B->d_norm);
-    nir::k_seg_scale<<<grid_for(n), nir::kBlock, 0, s>>>(n, B->d_col_inst, B->d_norm, h->tmp_n);
+    measure();
     for (int r = 0; r < std::max(1, p.power_iters); ++r) {
-        nir::k_spmv_warp64<<<gwm, nir::kBlock, 0, s>>>(m, h->A.rp, h->A.ci, h->A.v64, h->tmp_n, h->tmp_m);
-        nir::k_spmv_warp64<<<gwn, nir::kBlock, 0, s>>>(n, h->At.rp, h->At.ci, h->At.v64, h->tmp_m, h->tmp_n);
-        nir::k_seg_norm<<<I, nir::kBlock, 0, s>>>(B->d_col_off, h->tmp_n, B->d_norm);
-        nir::k_seg_scale<<<grid_for(n), nir::kBlock, 0, s>>>(n, B->d_col_inst, B->d_norm, h->tmp_n);
+        power_spmv(h, h->A, lm, h->tmp_n, B->d_norm, B->d_row_inst, h->tmp_m);
+        power_spmv(h, h->At, ln, h->tmp_m, nullptr, nullptr, h->tmp_n);
+        measure();
     }
     NIR_LAUNCHED();
-    std::vector<double> nrm(I), dc(n), dr(m);
+    std::vector<double> nrm(I), norms(size_t(I) * nir::kDdNorms);
+    lp_norms(h, I, B->d_row_off, B->d_col_off, norms.data());
     d2h(h, nrm.data(), B->d_norm, I * sizeof(double));
-    d2h(h, dc.data(), h->dc, n * sizeof(double));
-    d2h(h, dr.data(), h->dr, m * sizeof(double));
     std::vector<nir::DevState> st0(I);
     std::vector<double> bn(I), cn(I);
     for (int i = 0; i < I; ++i) {
-        DD cs, bs, co, bo;
-        for (int j = B->col_off[i]; j < B->col_off[i + 1]; ++j) {
-            cs = dd_add_prod(cs, h->h_c[j] * dc[j], h->h_c[j] * dc[j]);
-            co = dd_add_prod(co, h->h_c[j], h->h_c[j]);
-        }
-        for (int r = B->row_off[i]; r < B->row_off[i + 1]; ++r) {
-            double b = 0.0;
-            if (std::isfinite(h->h_rl[r])) b = std::fabs(h->h_rl[r]);
-            if (std::isfinite(h->h_ru[r])) b = std::max(b, std::fabs(h->h_ru[r]));
-            bo = dd_add_prod(bo, b, b);
-            bs = dd_add_prod(bs, b * dr[r], b * dr[r]);
-        }
-        const double csn = std::sqrt(cs.hi + cs.lo), bsn = std::sqrt(bs.hi + bs.lo);
+        const double* v = &norms[size_t(i) * nir::kDdNorms];
+        const double csn = v[1], bsn = v[3];
         const double sig = std::sqrt(nrm[i]);
         nir::DevState& d = st0[i];
         d = nir::DevState{};
@@ -461,8 +453,8 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
         d.log_omega0 = std::log(d.omega);
         d.tau = d.eta / d.omega;
         d.sigma = d.eta * d.omega;
-        cn[i] = std::sqrt(co.hi + co.lo);
-        bn[i] = std::sqrt(bo.hi + bo.lo);
+        cn[i] = v[0];
+        bn[i] = v[2];
     }
     h2d(h, B->insts, st0.data(), I * sizeof(nir::DevState));
     if (B->cur) launch_bcompact(B);
@@ -530,12 +522,11 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
         p.precision != NIR_PREC_FP32 ? 1 : 0, h->dc,
         h->dr, h->out_x, h->out_y);
     NIR_LAUNCHED();
-    std::vector<double> x(n), y(m);
-    d2h(h, x.data(), h->out_x, n * sizeof(double));
-    d2h(h, y.data(), h->out_y, m * sizeof(double));
+    if (x_out) NIR_CUDA(cudaMemcpyAsync(x_out, h->out_x, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+    if (y_out) NIR_CUDA(cudaMemcpyAsync(y_out, h->out_y, m * sizeof(double), cudaMemcpyDeviceToHost, s));
+    std::vector<double> obj(I);
+    lp_objectives(h, I, B->d_col_off, B->d_offset, h->out_x, obj.data());
     B->solved = true;
-    if (x_out) std::memcpy(x_out, x.data(), n * sizeof(double));
-    if (y_out) std::memcpy(y_out, y.data(), m * sizeof(double));
     const double t_end = now_sec();
     int worst = NIR_STATUS_OPTIMAL;
     long long iters = 0, iters64 = 0;
@@ -554,11 +545,7 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
         inf.max_rel_row_viol = d.max_rel_row;
         inf.primal_weight = d.omega;
         inf.step_size = d.eta;
-        DD o;
-        o.hi = B->offsets[i];
-        for (int j = B->col_off[i]; j < B->col_off[i + 1]; ++j)
-            if (h->h_c[j] != 0.0 && x[j] != 0.0) o = dd_add_prod(o, h->h_c[j], x[j]);
-        inf.objective = o.hi + o.lo;
+        inf.objective = obj[i];
         inf.setup_seconds = t_setup - t0;
         inf.solve_seconds = t_end - t_setup;
         inf.iterations_to_tol = (inf.status == NIR_STATUS_OPTIMAL) ? inf.iterations : -1;

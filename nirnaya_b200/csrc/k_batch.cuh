@@ -377,24 +377,6 @@ __global__ void k_bsnap(int count, const DevState* __restrict__ insts, HostSnap*
     __threadfence_system();
 }
 
-// Per-instance norms over contiguous ranges (power iteration).
-__global__ void k_seg_norm(const int* __restrict__ off, const double* __restrict__ w, double* __restrict__ norm) {
-    __shared__ double sh[kWarps];
-    const int i = blockIdx.x;
-    double s = 0.0;
-    for (int j = off[i] + threadIdx.x; j < off[i + 1]; j += kBlock) s += w[j] * w[j];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) norm[i] = sqrt(s);
-}
-
-__global__ void k_seg_scale(int n, const int* __restrict__ inst_of, const double* __restrict__ norm,
-                            double* __restrict__ w) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const double d = norm[inst_of[j]];
-    w[j] = d > 0.0 ? w[j] / d : 0.0;
-}
-
 // Output of a batch: each instance from the precision it ended in.
 __global__ void k_bunscale_out(int n, int m, const int* __restrict__ col_inst, const int* __restrict__ row_inst,
                                const DevState* __restrict__ insts, const float* __restrict__ xp32,

@@ -5,6 +5,7 @@
 #pragma once
 
 #include "dev_common.cuh"
+#include "k_verify.cuh"
 
 namespace nir {
 
@@ -76,6 +77,27 @@ __global__ void k_row_stat(int rows, const int* __restrict__ rp, const int* __re
     }
     acc = mode == 0 ? warp_max(acc) : warp_sum(acc);
     if (lane == 0) out[warp] = acc;
+}
+
+// The same maximum with T lanes per row, for rows too short to fill a warp
+// (a maximum does not depend on the order; the sum of mode 1 keeps the warp's
+// tree, because its last bit can decide the rounding to a power of two).
+// 16M nonzeros in rows of 10 and 25: 130 us a pass against 330 with a warp
+// per row.
+template <int T>
+__global__ void k_row_max(int rows, const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ v,
+                          const double* __restrict__ d_row, const double* __restrict__ d_col, double* __restrict__ out) {
+    const int r = int((blockIdx.x * (long long)blockDim.x + threadIdx.x) / T), t = threadIdx.x % T;
+    double acc = 0.0;
+    if (r < rows) {
+        const double dr = d_row[r];
+        const int e = rp[r + 1];
+#pragma unroll 4
+        for (int k = rp[r] + t; k < e; k += T) acc = fmax(acc, fabs(v[k]) * dr * d_col[ci[k]]);
+    }
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) acc = fmax(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    if (r < rows && t == 0) out[r] = acc;
 }
 
 // d[i] /= sqrt(stat[i]) where stat > 0.
@@ -176,40 +198,134 @@ __global__ void k_power_start_batch(int n, const int* __restrict__ col_inst, con
     u[j] = power_start_value(j - col_off[col_inst[j]]);
 }
 
-// One warp per row FP64 SpMV (setup only).
-__global__ void k_spmv_warp64(int rows, const int* __restrict__ rp, const int* __restrict__ ci,
-                              const double* __restrict__ v, const double* __restrict__ x, double* __restrict__ y) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= rows) return;
+// FP64 SpMV of the power iteration with T lanes per row: y = A x / norm of
+// the row's instance (norm null: 1; a zero norm gives 0).  T near a quarter
+// of the mean row length: with a warp per row, rows of 10 entries left two
+// thirds of the lanes idle (16M nonzeros: 220 us a product, 75 with 4 and 8
+// lanes).  The division stands for a pass that scaled x.
+template <int T>
+__global__ void k_power_spmv(int rows, const int* __restrict__ rp, const int* __restrict__ ci,
+                             const double* __restrict__ v, const double* __restrict__ x, const double* __restrict__ norm,
+                             const int* __restrict__ inst_of, double* __restrict__ y) {
+    const int r = int((blockIdx.x * (long long)blockDim.x + threadIdx.x) / T), t = threadIdx.x % T;
     double acc = 0.0;
-    for (int k = rp[warp] + lane; k < rp[warp + 1]; k += 32) acc += v[k] * x[ci[k]];
-    acc = warp_sum(acc);
-    if (lane == 0) y[warp] = acc;
+    if (r < rows) {
+        const int e = rp[r + 1];
+#pragma unroll 4
+        for (int k = rp[r] + t; k < e; k += T) acc += v[k] * x[ci[k]];
+    }
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (r < rows && t == 0) {
+        if (norm) {
+            const double d = norm[inst_of ? inst_of[r] : 0];
+            acc = d > 0.0 ? acc / d : 0.0;
+        }
+        y[r] = acc;
+    }
 }
 
-// Per-block partial sums of squares.
-__global__ void k_sumsq_partials(int n, const double* __restrict__ w, double* __restrict__ part) {
+// Norms of an instance's part of w, in two steps: G CTAs per instance leave
+// partial sums of squares, then one warp per instance adds them in a fixed
+// order.
+__global__ void k_seg_sumsq(int G, const int* __restrict__ off, const double* __restrict__ w, double* __restrict__ part) {
     __shared__ double sh[kWarps];
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    double v = (j < n) ? w[j] * w[j] : 0.0;
-    v = block_sum(v, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = v;
+    const int i = blockIdx.x / G, g = blockIdx.x % G;
+    double s = 0.0;
+    for (int j = off[i] + g * kBlock + int(threadIdx.x); j < off[i + 1]; j += G * kBlock) s += w[j] * w[j];
+    s = block_sum(s, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = s;
+}
+__global__ void k_seg_norm(int count, int G, const double* __restrict__ part, double* __restrict__ norm) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= count) return;
+    double s = 0.0;
+    for (int g = lane; g < G; g += 32) s += part[i * G + g];
+    s = warp_sum(s);
+    if (lane == 0) norm[i] = sqrt(s);
 }
 
-// norm = sqrt(sum part); stores it in st->ref_norm_est; the estimate of
-// ||A||_2 after the round is sqrt(norm) for a unit start vector.
-__global__ void k_norm_finalize(const double* __restrict__ part, int nblk, DevState* st) {
-    __shared__ double sh[kWarps];
-    double s = block_sum_array(part, nblk, sh);
-    if (threadIdx.x == 0) st->ref_norm_est = sqrt(s);
+// ---------------------------------------------------------------- double-double sums
+
+// Sums in double-double over an instance's entries (the reference's dd_real
+// steps, k_verify.cuh): the objective c'x + offset of Model::eval_objective
+// (src/model/model.hpp:73-98) and the norms of b and c, given and scaled.
+// Each thread adds its entries, then the threads, then the G CTAs of an
+// instance; the order differs from a loop's, the rounding is 2^-104 relative
+// to the terms either way.  On the host these sums took 16 ms of a 256-
+// iteration solve of 16M nonzeros, with another 18 MB copied back for them.
+__device__ inline vfy::DD dd_warp(vfy::DD d) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double h = __shfl_down_sync(0xffffffffu, d.hi, o), l = __shfl_down_sync(0xffffffffu, d.lo, o);
+        vfy::add_dd(d, h, l);
+    }
+    return d;
+}
+// The CTA's sum in thread 0.
+__device__ inline vfy::DD dd_block(vfy::DD d, vfy::DD* sh /* kWarps */) {
+    d = dd_warp(d);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = d;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = 1; k < kWarps; ++k) vfy::add_dd(d, sh[k].hi, sh[k].lo);
+    return d;
 }
 
-__global__ void k_scale_by_inv_norm(int n, double* __restrict__ w, const DevState* __restrict__ st) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    double nrm = st->ref_norm_est;
-    w[j] = nrm > 0.0 ? w[j] / nrm : 0.0;
+constexpr int kDdNorms = 4;  // c, c scaled, b, b scaled (b_i: the larger finite bound of row i in magnitude)
+
+__global__ void __launch_bounds__(kBlock) k_dd_norms(int G, const int* __restrict__ row_off, const int* __restrict__ col_off,
+                                                     const double* __restrict__ c, const double* __restrict__ dc,
+                                                     const double* __restrict__ rl, const double* __restrict__ ru,
+                                                     const double* __restrict__ dr, vfy::DD* __restrict__ part) {
+    __shared__ vfy::DD sh[kWarps];
+    const int i = blockIdx.x / G, g = blockIdx.x % G;
+    vfy::DD s[kDdNorms] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    for (int j = col_off[i] + g * kBlock + int(threadIdx.x); j < col_off[i + 1]; j += G * kBlock) {
+        const double a = c[j], b = vfy::mul(a, dc[j]);
+        vfy::add_prod(s[0], a, a);
+        vfy::add_prod(s[1], b, b);
+    }
+    for (int r = row_off[i] + g * kBlock + int(threadIdx.x); r < row_off[i + 1]; r += G * kBlock) {
+        double a = 0.0;
+        if (isfinite(rl[r])) a = fabs(rl[r]);
+        if (isfinite(ru[r])) a = fmax(a, fabs(ru[r]));
+        const double b = vfy::mul(a, dr[r]);
+        vfy::add_prod(s[2], a, a);
+        vfy::add_prod(s[3], b, b);
+    }
+#pragma unroll
+    for (int q = 0; q < kDdNorms; ++q) {
+        const vfy::DD d = dd_block(s[q], sh);
+        if (threadIdx.x == 0) part[blockIdx.x * kDdNorms + q] = d;
+    }
+}
+
+__global__ void __launch_bounds__(kBlock) k_dd_objective(int G, const int* __restrict__ col_off,
+                                                         const double* __restrict__ c, const double* __restrict__ x,
+                                                         vfy::DD* __restrict__ part) {
+    __shared__ vfy::DD sh[kWarps];
+    const int i = blockIdx.x / G, g = blockIdx.x % G;
+    vfy::DD s{0.0, 0.0};
+    for (int j = col_off[i] + g * kBlock + int(threadIdx.x); j < col_off[i + 1]; j += G * kBlock)
+        if (c[j] != 0.0 && x[j] != 0.0) vfy::add_prod(s, c[j], x[j]);
+    const vfy::DD d = dd_block(s, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = d;
+}
+
+// out[i Q + q] = base[i] (or 0) plus the G partial sums, in order.
+__global__ void k_dd_finish(int count, int G, int Q, const vfy::DD* __restrict__ part, const double* __restrict__ base,
+                            double* __restrict__ out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= count * Q) return;
+    const int i = t / Q, q = t % Q;
+    vfy::DD s{base ? base[i] : 0.0, 0.0};
+    for (int g = 0; g < G; ++g) {
+        const vfy::DD p = part[(size_t(i) * G + g) * Q + q];
+        vfy::add_dd(s, p.hi, p.lo);
+    }
+    out[t] = vfy::add(s.hi, s.lo);
 }
 
 // ---------------------------------------------------------------- iterate setup
