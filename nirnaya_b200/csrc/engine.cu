@@ -100,9 +100,68 @@ inline DD dd_add_prod(DD a, double x, double y) {
     return dd_add(a, p);
 }
 
-struct DevBuf {
-    void* p = nullptr;
-    size_t bytes = 0;
+// Device memory in chunks that allocations are carved from: large ones
+// reserved beforehand for what is known to come, small ones on demand, and
+// a block of its own for what is large and fits none.  A cudaMalloc takes
+// 20 us below 64 KB, 70 at 300 KB and 330 from 2 MB on, its cudaFree as
+// long, and a handle holds about 60 arrays.
+struct DevArena {
+    static constexpr size_t kAlign = 256, kOwn = size_t(1) << 20, kSmallChunk = size_t(128) << 10;
+    static size_t aligned(size_t bytes) { return (std::max<size_t>(1, bytes) + kAlign - 1) / kAlign * kAlign; }
+    struct Block {
+        char* p;
+        size_t size, used;
+        bool carved;  // a chunk; false: one allocation
+    };
+    std::vector<Block> blocks;
+    int cur = -1;  // the chunk being carved
+    long long bytes = 0;
+
+    char* block(size_t size, bool carved) {
+        blocks.reserve(blocks.size() + 1);
+        void* p = nullptr;
+        NIR_CUDA(cudaMalloc(&p, size));
+        blocks.push_back({static_cast<char*>(p), size, 0, carved});
+        bytes += (long long)size;
+        return static_cast<char*>(p);
+    }
+    void reserve(size_t size) {
+        block(size, true);
+        cur = int(blocks.size()) - 1;
+    }
+    void* alloc(size_t size) {
+        size = aligned(size);
+        if (cur < 0 || blocks[size_t(cur)].size - blocks[size_t(cur)].used < size) {
+            if (size >= kOwn) return block(size, false);
+            reserve(std::max(size, kSmallChunk));
+        }
+        Block& c = blocks[size_t(cur)];
+        char* p = c.p + c.used;
+        c.used += size;
+        return p;
+    }
+    // Frees a block of its own; a carved allocation stays with its chunk.
+    void release(void* p) {
+        for (size_t i = 0; i < blocks.size(); ++i)
+            if (blocks[i].p == p && !blocks[i].carved) {
+                cudaFree(p);
+                bytes -= (long long)blocks[i].size;
+                blocks.erase(blocks.begin() + long(i));
+                if (cur > int(i)) --cur;
+                return;
+            }
+    }
+    // Scratch carved last is given back by rewinding to the mark before it.
+    size_t mark() const { return cur < 0 ? 0 : blocks[size_t(cur)].used; }
+    void rewind(size_t m) {
+        if (cur >= 0) blocks[size_t(cur)].used = m;
+    }
+    void clear() {
+        for (auto& b : blocks) cudaFree(b.p);
+        blocks.clear();
+        cur = -1;
+        bytes = 0;
+    }
 };
 
 // The per-orientation layout choice of a solve.
@@ -178,6 +237,47 @@ struct ChunkGraph {
 
 struct ClusterPlan;  // engine_cluster.cuh
 
+namespace {
+
+// Status rings in host-mapped memory, kept for the next handle: taking one
+// from the driver costs 1 to 3 ms, giving it back 0.4.  At most kSnapKeep
+// of 8 KB are kept, for the life of the process; any thread may take and
+// give (a ring belongs to one handle in between, whose stream has ended
+// when it is given back).
+constexpr size_t kSnapKeep = 16;
+std::mutex g_snap_mu;
+std::vector<nir::HostSnap*> g_snap_free;
+
+nir::HostSnap* snap_ring_take() {
+    {
+        std::lock_guard<std::mutex> g(g_snap_mu);
+        if (!g_snap_free.empty()) {
+            nir::HostSnap* r = g_snap_free.back();
+            g_snap_free.pop_back();
+            return r;
+        }
+    }
+    void* p = nullptr;
+    NIR_CUDA(cudaHostAlloc(&p, sizeof(nir::HostSnap) * nir::kSnapRing, cudaHostAllocMapped | cudaHostAllocPortable));
+    return static_cast<nir::HostSnap*>(p);
+}
+
+void snap_ring_put(nir::HostSnap* r) {
+    {
+        std::lock_guard<std::mutex> g(g_snap_mu);
+        if (g_snap_free.size() < kSnapKeep) {
+            try {
+                g_snap_free.push_back(r);
+                return;
+            } catch (const std::bad_alloc&) {
+            }
+        }
+    }
+    cudaFreeHost(r);
+}
+
+}  // namespace
+
 struct nir_pdhg {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -220,8 +320,6 @@ struct nir_pdhg {
     size_t flush_bytes = 0;
     double* ceil_out = nullptr;        // one running sum per thread of the ceiling kernels
     nir::DevState* st_time = nullptr;  // running copy of the state for nir_pdhg_time_iteration
-    std::vector<DevBuf> bufs;
-    long long device_bytes = 0;
     ChunkGraph graphs[3];
     long long last_iters = 0;
     LayChoice tuned[3];                    // autotuned layouts per NIR_PREC_*
@@ -269,6 +367,8 @@ struct nir_pdhg {
         int *row_off = nullptr, *col_off = nullptr;  // one instance: {0, m}, {0, n}
     } vfy;
 
+    DevArena mem;
+
     // zero-filled allocation with `pad` spare elements past the end (the
     // row-block copies read 16-byte windows that may reach past the end)
     template <typename T>
@@ -280,33 +380,20 @@ struct nir_pdhg {
 
     template <typename T>
     T* alloc(size_t count) {
-        void* p = nullptr;
-        size_t bytes = std::max<size_t>(1, count) * sizeof(T);
-        NIR_CUDA(cudaMalloc(&p, bytes));
-        bufs.push_back({p, bytes});
-        device_bytes += (long long)bytes;
-        return static_cast<T*>(p);
+        return static_cast<T*>(mem.alloc(count * sizeof(T)));
     }
-
-    void release(void* p) {
-        for (auto it = bufs.begin(); it != bufs.end(); ++it)
-            if (it->p == p) {
-                device_bytes -= (long long)it->bytes;
-                cudaFree(it->p);
-                bufs.erase(it);
-                return;
-            }
-    }
+    void release(void* p) { mem.release(p); }
 
     ~nir_pdhg() {
         if (device >= 0) cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
+        cluster.reset();
         for (auto& g : graphs) {
             if (g.ge) cudaGraphExecDestroy(g.ge);
             if (g.g) cudaGraphDestroy(g.g);
         }
-        for (auto& b : bufs) cudaFree(b.p);
-        if (snap.ring) cudaFreeHost(snap.ring);
+        mem.clear();
+        if (snap.ring) snap_ring_put(snap.ring);
         if (stream) cudaStreamDestroy(stream);
         inner.reset();
     }
@@ -554,6 +641,11 @@ void upload_vectors(nir_pdhg* h, const double* cost, const double* collo, const 
     NIR_CUDA(cudaStreamSynchronize(h->stream));
 }
 
+int max_grid(const nir_pdhg* h) { return 8 * h->sms; }  // 2048 threads per SM / kBlock
+size_t partials_len(const nir_pdhg* h) {
+    return 12 * size_t(max_grid(h)) + size_t(grid_for(std::max(h->m, h->n))) + 16;
+}
+
 void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0)
@@ -571,6 +663,24 @@ void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
     h->offset = lp->obj_offset;
     cudaStream_t s = h->stream;
 
+    // One chunk for everything below: the two orientations (with allocz's
+    // spare entries), then the transpose's scratch, whose place the vectors
+    // take.
+    int end_bit = 1;
+    while ((1LL << end_bit) <= (long long)m) ++end_bit;
+    size_t tmp_bytes = 0;
+    NIR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (const int*)nullptr, (int*)nullptr, (const int*)nullptr,
+                                             (int*)nullptr, (int)nnz, 0, end_bit, s));
+    {
+        auto al = [](size_t count, size_t size) { return DevArena::aligned(count * size); };
+        const size_t Z = size_t(nnz), N = size_t(n), M = size_t(m);
+        const size_t matrix = al(N + 9, 4) + al(M + 9, 4) + 2 * (al(Z + 8, 4) + 2 * al(Z + 8, 8) + al(Z + 8, 4));
+        const size_t scratch = al(N + 1, 8) + 4 * al(Z, 4) + al(tmp_bytes, 1);
+        const size_t vectors = 14 * al(N, 8) + 10 * al(N, 4) + 12 * al(M, 8) + 9 * al(M, 4) + al(8 * nir::kHist, 8) +
+                               al(partials_len(h), 8) + 64 * DevArena::kAlign;
+        h->mem.reserve(matrix + std::max(scratch, vectors));
+    }
+
     // A' = CSC of A read as rows.
     Orient& T = h->At;
     T.rows = n;
@@ -581,6 +691,17 @@ void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
     T.v_orig = h->allocz<double>(nnz);
     T.v64 = h->allocz<double>(nnz);
     T.v32 = h->allocz<float>(nnz);
+    // A's arrays come before the scratch
+    Orient& R = h->A;
+    R.rows = m;
+    R.cols = n;
+    R.nnz = nnz;
+    R.rp = h->allocz<int>(m + 1);
+    R.ci = h->allocz<int>(nnz);
+    R.v_orig = h->allocz<double>(nnz);
+    R.v64 = h->allocz<double>(nnz);
+    R.v32 = h->allocz<float>(nnz);
+    const size_t scratch_mark = h->mem.mark();
     long long* d_start = h->alloc<long long>(n + 1);
     NIR_CUDA(cudaMemcpyAsync(d_start, lp->col_start, (n + 1) * sizeof(long long), cudaMemcpyHostToDevice, s));
     NIR_CUDA(cudaMemcpyAsync(T.ci, lp->row_index, nnz * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -592,15 +713,6 @@ void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
 
     // A: stable radix sort of the CSC entries by row keeps each row's
     // entries in ascending column order (the reference's scatter order).
-    Orient& R = h->A;
-    R.rows = m;
-    R.cols = n;
-    R.nnz = nnz;
-    R.rp = h->allocz<int>(m + 1);
-    R.ci = h->allocz<int>(nnz);
-    R.v_orig = h->allocz<double>(nnz);
-    R.v64 = h->allocz<double>(nnz);
-    R.v32 = h->allocz<float>(nnz);
     {
         int* col_of = h->alloc<int>(nnz);
         int* ids = h->alloc<int>(nnz);
@@ -610,10 +722,6 @@ void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
         NIR_LAUNCHED();
         nir::k_iota<<<grid_for(nnz), nir::kBlock, 0, s>>>(nnz, ids);
         NIR_LAUNCHED();
-        int end_bit = 1;
-        while ((1LL << end_bit) <= (long long)m) ++end_bit;
-        size_t tmp_bytes = 0;
-        NIR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, T.ci, keys_out, ids, perm, (int)nnz, 0, end_bit, s));
         void* tmp = h->alloc<unsigned char>(tmp_bytes);
         NIR_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, T.ci, keys_out, ids, perm, (int)nnz, 0, end_bit, s));
         nir::k_row_ptr_from_sorted<<<grid_for(m + 1), nir::kBlock, 0, s>>>(m, nnz, keys_out, R.rp);
@@ -623,8 +731,7 @@ void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
         R.h_rp.resize(m + 1);
         NIR_CUDA(cudaMemcpyAsync(R.h_rp.data(), R.rp, (m + 1) * sizeof(int), cudaMemcpyDeviceToHost, s));
         NIR_CUDA(cudaStreamSynchronize(s));
-        // scratch of the transpose is released right away
-        for (void* p : {(void*)col_of, (void*)ids, (void*)perm, (void*)keys_out, tmp, (void*)d_start}) h->release(p);
+        h->mem.rewind(scratch_mark);  // the vectors take the scratch's place
     }
 
     // vectors
@@ -673,7 +780,7 @@ void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
     h->gs_gen = h->allocz<unsigned>(1);
     h->gs_err = h->allocz<int>(1);
     NIR_CUDA(cudaMemsetAsync(h->snap.d_seq, 0, sizeof(long long), s));
-    NIR_CUDA(cudaHostAlloc((void**)&h->snap.ring, sizeof(nir::HostSnap) * nir::kSnapRing, cudaHostAllocMapped));
+    h->snap.ring = snap_ring_take();
     std::memset(h->snap.ring, 0, sizeof(nir::HostSnap) * nir::kSnapRing);
     NIR_CUDA(cudaStreamSynchronize(s));
 }
@@ -717,11 +824,9 @@ LaunchCfg warp_cfg(nir_pdhg* h, K* kernel, int nblk) {
     return {std::min(need, per * h->sms), smem};
 }
 
-int max_grid(const nir_pdhg* h) { return 8 * h->sms; }  // 2048 threads per SM / kBlock
-
 // Partial-sum area large enough for any kernel of this handle.
 void ensure_partials(nir_pdhg* h) {
-    size_t need = 12 * size_t(max_grid(h)) + size_t(grid_for(std::max(h->m, h->n))) + 16;
+    size_t need = partials_len(h);
     if (h->part && h->part_len >= need) return;
     h->part = h->alloc<double>(need);
     h->part_len = need;
@@ -2619,7 +2724,7 @@ int nir_pdhg_get_layout(nir_pdhg* h, nir_pdhg_layout* out) {
     out->blocks_at = src->At.lay >= 0 ? lay_nblk(src->At) : 0;
     out->block_nnz = src->A.lay == nir::kLayCta ? kCtaCap : src->A.cap;
     out->block_nnz_at = src->At.lay == nir::kLayCta ? kCtaCap : src->At.cap;
-    out->device_bytes = h->device_bytes;
+    out->device_bytes = h->mem.bytes + (h->cluster ? h->cluster->mem.bytes : 0);
     return 0;
 }
 

@@ -43,7 +43,11 @@ struct nir_pdhg_batch {
     const unsigned char* in_cluster = nullptr;  // [instance], device: solved by the plan in use (null: none)
     bool solved = false;  // h->out_x holds the points the last batch solve returned
     ~nir_pdhg_batch() {
-        if (h && h->device >= 0) cudaSetDevice(h->device);
+        if (h && h->device >= 0) {
+            cudaSetDevice(h->device);
+            if (h->stream) cudaStreamSynchronize(h->stream);
+        }
+        cluster.reset();
         for (auto& g : graphs) {
             if (g.ge) cudaGraphExecDestroy(g.ge);
             if (g.g) cudaGraphDestroy(g.g);

@@ -35,7 +35,8 @@ struct ClusterPlan {
     size_t smem[2] = {};    // dynamic shared memory of a launch
     bool resident[2] = {true, true};  // every member has all of it in shared memory
     long long values_of = -1;  // the scaling whose values the streams hold
-    std::vector<DevBuf> bufs;
+    DevArena mem;
+    ~ClusterPlan() { mem.clear(); }
 };
 
 namespace {
@@ -46,22 +47,15 @@ static_assert(nir::kClPlanWarps == nir::kClWarps, "the plan deals slices to the 
 constexpr size_t kClSmemMax = 220 * 1024;
 
 template <typename T>
-T* cl_alloc(nir_pdhg* h, ClusterPlan& P, size_t count) {
-    T* p = h->alloc<T>(count);
-    P.bufs.push_back({p, 0});
-    return p;
+T* cl_alloc(ClusterPlan& P, size_t count) {
+    return static_cast<T*>(P.mem.alloc(count * sizeof(T)));
 }
 
 template <typename T>
 T* cl_upload(nir_pdhg* h, ClusterPlan& P, const std::vector<T>& v) {
-    T* p = cl_alloc<T>(h, P, v.size());
+    T* p = cl_alloc<T>(P, v.size());
     if (!v.empty()) NIR_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream));
     return p;
-}
-
-void cl_free(nir_pdhg* h, ClusterPlan& P) {
-    for (auto& b : P.bufs) h->release(b.p);
-    P.bufs.clear();
 }
 
 // What the kernel sees of one side.
@@ -123,12 +117,19 @@ std::unique_ptr<ClusterPlan> cl_build(nir_pdhg* h, int C, const std::vector<int>
     P.col_off = col_off;
     P.d_row_off = d_row_off;
     P.d_col_off = d_col_off;
-    try {
+    {
+        size_t total = 0;
         for (ClusterPlan::Side* t : {&P.row, &P.col}) {
             const bool is_row = t == &P.row;
             const Orient& o = is_row ? h->A : h->At;
             t->rows = o.rows;
             nir::cl_build_side(is_row ? row_off : col_off, o.h_rp, C, t->h);
+            total += size_t(o.rows) * size_t(4 + 4 + 1 + 2 + 2 * C) + t->h.slices.size() * 20 + size_t(P.count) * C * 40;
+        }
+        P.mem.reserve(total + 64 * DevArena::kAlign);
+        for (ClusterPlan::Side* t : {&P.row, &P.col}) {
+            const bool is_row = t == &P.row;
+            const Orient& o = is_row ? h->A : h->At;
             t->order = cl_upload(h, P, t->h.order);
             t->pos = cl_upload(h, P, t->h.pos);
             t->rank = cl_upload(h, P, t->h.rank);
@@ -137,12 +138,12 @@ std::unique_ptr<ClusterPlan> cl_build(nir_pdhg* h, int C, const std::vector<int>
             t->base = cl_upload(h, P, t->h.base);
             t->slices = cl_upload(h, P, t->h.slices);
             t->owner = cl_upload(h, P, t->h.owner);
-            t->need = cl_alloc<unsigned short>(h, P, size_t(o.rows));
-            t->slot = cl_alloc<unsigned short>(h, P, size_t(o.rows) * C);
-            t->ghost_rank = cl_alloc<int>(h, P, size_t(P.count) * C);
-            t->bytes = cl_alloc<int>(h, P, size_t(P.count) * C);
-            t->all = cl_alloc<unsigned short>(h, P, size_t(P.count) * C);
-            t->bulk = cl_alloc<unsigned short>(h, P, size_t(P.count) * C);
+            t->need = cl_alloc<unsigned short>(P, size_t(o.rows));
+            t->slot = cl_alloc<unsigned short>(P, size_t(o.rows) * C);
+            t->ghost_rank = cl_alloc<int>(P, size_t(P.count) * C);
+            t->bytes = cl_alloc<int>(P, size_t(P.count) * C);
+            t->all = cl_alloc<unsigned short>(P, size_t(P.count) * C);
+            t->bulk = cl_alloc<unsigned short>(P, size_t(P.count) * C);
         }
         std::vector<int> gr(size_t(P.count) * C);
         for (ClusterPlan::Side* t : {&P.row, &P.col}) {
@@ -186,18 +187,21 @@ std::unique_ptr<ClusterPlan> cl_build(nir_pdhg* h, int C, const std::vector<int>
         P.members = int(list.size());
         if (P.members == 0) {
             NIR_CUDA(cudaStreamSynchronize(s));
-            cl_free(h, P);
             return nullptr;
         }
         P.d_list = cl_upload(h, P, list);
         P.d_member = cl_upload(h, P, P.member);
         for (int q = 0; q < 2; ++q) P.d_flags[q] = cl_upload(h, P, flags[q]);
+        size_t streams = 0;
+        for (ClusterPlan::Side* t : {&P.row, &P.col})
+            streams += size_t(t->h.base.back()) * nir::kClUnit * 14 + size_t(t->rows) * 80 + 4 * DevArena::kAlign;
+        P.mem.reserve(streams);
         for (ClusterPlan::Side* t : {&P.row, &P.col}) {
             const size_t e = size_t(t->h.base.back()) * nir::kClUnit;
-            t->idx = cl_alloc<unsigned short>(h, P, e);
-            t->v32 = cl_alloc<float>(h, P, e);
-            t->v64 = cl_alloc<double>(h, P, e);
-            t->vec = cl_alloc<double>(h, P, size_t(t->rows) * 10);
+            t->idx = cl_alloc<unsigned short>(P, e);
+            t->v32 = cl_alloc<float>(P, e);
+            t->v64 = cl_alloc<double>(P, e);
+            t->vec = cl_alloc<double>(P, size_t(t->rows) * 10);
         }
         for (int t = 0; t < 2; ++t) {
             const Orient& o = t ? h->At : h->A;
@@ -210,9 +214,6 @@ std::unique_ptr<ClusterPlan> cl_build(nir_pdhg* h, int C, const std::vector<int>
             NIR_LAUNCHED();
         }
         NIR_CUDA(cudaStreamSynchronize(s));  // the uploads read the vectors above
-    } catch (...) {
-        cl_free(h, P);
-        throw;
     }
     return up;
 }
@@ -405,8 +406,6 @@ ClusterPlan* cl_single(nir_pdhg* h, const nir_pdhg_params& p) {
             if (P && (f >= 0 || cl_time(nnz, cl_arrivals(*P, 0), C) < kClMargin * cl_launch_time(nnz))) {
                 h->cluster = std::move(P);
                 h->cluster_size = C;
-            } else if (P) {
-                cl_free(h, *P);
             }
         }
     }
@@ -452,12 +451,7 @@ std::unique_ptr<ClusterPlan> cl_batch(nir_pdhg* h, const std::vector<int>& row_o
     for (int k = first; k < 5; ++k) {
         std::unique_ptr<ClusterPlan> P =
             cl_build(h, sizes[k], row_off, col_off, d_row_off, d_col_off, d_row_inst, d_col_inst);
-        if (P && (!best || P->members > best->members)) {
-            if (best) cl_free(h, *best);
-            best = std::move(P);
-        } else if (P) {
-            cl_free(h, *P);
-        }
+        if (P && (!best || P->members > best->members)) best = std::move(P);
         if (f > 0 || (best && best->members == count)) break;
     }
     return best;
