@@ -63,8 +63,7 @@ void verify_impl(nir_pdhg* h, int count, const int* d_row_off, const int* d_col_
     auto* g = static_cast<nir::vfy::Rec*>(v.g);
     nir::vfy::k_vfy_cols<<<count, nir::vfy::kVfyBlock, 0, s>>>(d_col_off, d_x, h->l, h->u, d_vt, v.fb, b, g);
     NIR_LAUNCHED();
-    const long long threads = (long long)count + h->m;
-    const unsigned grid = unsigned((threads + nir::vfy::kVfyBlock - 1) / nir::vfy::kVfyBlock);
+    const unsigned grid = unsigned(count) + unsigned((h->m + nir::vfy::kVfyBlock - 1) / nir::vfy::kVfyBlock);
     nir::vfy::k_vfy_rows<<<grid, nir::vfy::kVfyBlock, 0, s>>>(count, h->m, d_row_off, d_col_off, d_row_inst, h->A.rp,
                                                               h->A.ci, h->A.v_orig, d_x, h->rl, h->ru, h->c, v.offset,
                                                               v.fb, h->d_row_orig, v.rv, v.rs, v.obj);
