@@ -59,6 +59,14 @@ struct DevState {
     double bnorm, cnorm;   // ||b||, ||c|| of the original LP: the relative KKT's denominators
 };
 
+// Programmatic dependent launch.  A kernel launched that way starts while
+// the one before it still runs: it may read what no kernel of the chunk
+// writes (matrix, descriptors, solver state), and waits before the rest.
+// pdl_release lets the next kernel start likewise.  Without the launch
+// attribute both do nothing.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Deterministic block-wide sum / max over kBlock threads: a fixed shuffle
 // tree inside each warp, then warp 0 combines the warp results in order.
 template <typename T>

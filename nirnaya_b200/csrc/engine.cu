@@ -1021,6 +1021,23 @@ struct SolveCfg {
     int barrier_test = 0;  // persistent launch whose barrier cannot complete (bounded-wait test)
 };
 
+// Launches a kernel on the handle's stream; `early`: it may start while the
+// kernel before it still runs (pdl_wait).
+template <typename... P, typename... A>
+void launch_kernel(nir_pdhg* h, bool early, void (*k)(P...), int grid, size_t smem, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(nir::kBlock);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    NIR_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...));
+}
+
 // Optional event timing of the first iteration of a chunk.
 struct ChunkTimer {
     cudaEvent_t e[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -1096,25 +1113,19 @@ void launch_fast_chunk_l(nir_pdhg* h, const SolveCfg& cfg, int phase, ChunkTimer
         nir::IterArgs ad{la, L.D, h->st, i, cfg.halpern, phase, cfg.p.reflection};
         const bool timed = tm && tm->armed && i == 0 && !cfg.persistent;
         if (timed) NIR_CUDA(cudaEventRecord(tm->e[0], s));
-        if (check)
-            nir::k_primal<LP, TV, TX, true><<<gp1, nir::kBlock, sp, s>>>(
-                ap, valAt, Vec<TX>::y(h), Vec<TX>::x(h), Vec<TX>::xb(h), Vec<TX>::xp(h), Vec<TX>::c(h), Vec<TX>::l(h),
-                Vec<TX>::u(h), Vec<TX>::x0(h));
-        else
-            nir::k_primal<LP, TV, TX, false><<<gp0, nir::kBlock, sp, s>>>(
-                ap, valAt, Vec<TX>::y(h), Vec<TX>::x(h), Vec<TX>::xb(h), Vec<TX>::xp(h), Vec<TX>::c(h), Vec<TX>::l(h),
-                Vec<TX>::u(h), Vec<TX>::x0(h));
-        NIR_LAUNCHED();
+        // Every kernel of the chunk but the first may start before the one
+        // ahead of it has ended: its descriptors and first matrix entries
+        // are then in registers when the vectors are complete.  The first
+        // follows the controller, whose state it reads.  Timed launches
+        // run one by one.
+        const bool early = !timed && !(tm && tm->armed);
+        const auto kp = check ? nir::k_primal<LP, TV, TX, true> : nir::k_primal<LP, TV, TX, false>;
+        launch_kernel(h, early && i > i_first, kp, check ? gp1 : gp0, sp, ap, valAt, Vec<TX>::y(h), Vec<TX>::x(h),
+                      Vec<TX>::xb(h), Vec<TX>::xp(h), Vec<TX>::c(h), Vec<TX>::l(h), Vec<TX>::u(h), Vec<TX>::x0(h));
         if (timed) NIR_CUDA(cudaEventRecord(tm->e[1], s));
-        if (check)
-            nir::k_dual<LD, TV, TX, true><<<gd1, nir::kBlock, sd, s>>>(ad, valA, Vec<TX>::xb(h), Vec<TX>::y(h),
-                                                                       Vec<TX>::yp(h), Vec<TX>::rl(h), Vec<TX>::ru(h),
-                                                                       Vec<TX>::y0(h));
-        else
-            nir::k_dual<LD, TV, TX, false><<<gd0, nir::kBlock, sd, s>>>(ad, valA, Vec<TX>::xb(h), Vec<TX>::y(h),
-                                                                        Vec<TX>::yp(h), Vec<TX>::rl(h), Vec<TX>::ru(h),
-                                                                        Vec<TX>::y0(h));
-        NIR_LAUNCHED();
+        const auto kd = check ? nir::k_dual<LD, TV, TX, true> : nir::k_dual<LD, TV, TX, false>;
+        launch_kernel(h, early, kd, check ? gd1 : gd0, sd, ad, valA, Vec<TX>::xb(h), Vec<TX>::y(h), Vec<TX>::yp(h),
+                      Vec<TX>::rl(h), Vec<TX>::ru(h), Vec<TX>::y0(h));
         if (timed) NIR_CUDA(cudaEventRecord(tm->e[2], s));
         h->launches += 2;
     }
@@ -2595,15 +2606,13 @@ void time_iteration_l(nir_pdhg* h, int reps, double* primal_us, double* dual_us,
     nir::IterArgs ad{lay_of(h->A), L.D, h->st_time, 1, 1, 0, 1.0};
     const TV* valAt = vals_of<TV>(h->At);
     const TV* valA = vals_of<TV>(h->A);
-    auto primal = [&]() {
-        nir::k_primal<LP, TV, TX, false><<<gp, nir::kBlock, sp, s>>>(
-            ap, valAt, Vec<TX>::y(h), Vec<TX>::x(h), Vec<TX>::xb(h), Vec<TX>::xp(h), Vec<TX>::c(h), Vec<TX>::l(h),
-            Vec<TX>::u(h), Vec<TX>::x0(h));
+    auto primal = [&](bool early) {
+        launch_kernel(h, early, nir::k_primal<LP, TV, TX, false>, gp, sp, ap, valAt, Vec<TX>::y(h), Vec<TX>::x(h),
+                      Vec<TX>::xb(h), Vec<TX>::xp(h), Vec<TX>::c(h), Vec<TX>::l(h), Vec<TX>::u(h), Vec<TX>::x0(h));
     };
-    auto dual = [&]() {
-        nir::k_dual<LD, TV, TX, false><<<gd, nir::kBlock, sd, s>>>(ad, valA, Vec<TX>::xb(h), Vec<TX>::y(h),
-                                                                   Vec<TX>::yp(h), Vec<TX>::rl(h), Vec<TX>::ru(h),
-                                                                   Vec<TX>::y0(h));
+    auto dual = [&](bool early) {
+        launch_kernel(h, early, nir::k_dual<LD, TV, TX, false>, gd, sd, ad, valA, Vec<TX>::xb(h), Vec<TX>::y(h),
+                      Vec<TX>::yp(h), Vec<TX>::rl(h), Vec<TX>::ru(h), Vec<TX>::y0(h));
     };
     cudaEvent_t a, b;
     NIR_CUDA(cudaEventCreate(&a));
@@ -2613,8 +2622,8 @@ void time_iteration_l(nir_pdhg* h, int reps, double* primal_us, double* dual_us,
         cudaGraphExec_t ge = nullptr;
         NIR_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         for (int r = 0; r < reps; ++r) {
-            if (which != 1) primal();
-            if (which != 0) dual();
+            if (which != 1) primal(r > 0);
+            if (which != 0) dual(r > 0 || which == 2);
         }
         const cudaError_t launched = cudaGetLastError();
         const cudaError_t ended = cudaStreamEndCapture(s, &g);

@@ -210,24 +210,13 @@ void launch_batch_chunk_l(nir_pdhg_batch* B, const SolveCfg& cfg, int phase) {
         const bool check = (i == K - 1);
         nir::BatchArgs ap = bargs(B, true, P, i, cfg.halpern, phase, cfg.p.reflection);
         nir::BatchArgs ad = bargs(B, false, D, i, cfg.halpern, phase, cfg.p.reflection);
-        if (check)
-            nir::k_bprimal<LP, TV, TX, true><<<gp1, nir::kBlock, sp, s>>>(
-                ap, bvals<TV>(LT), Vec<TX>::y(h), Vec<TX>::x(h), Vec<TX>::xb(h), Vec<TX>::xp(h), Vec<TX>::c(h),
-                Vec<TX>::l(h), Vec<TX>::u(h), Vec<TX>::x0(h));
-        else
-            nir::k_bprimal<LP, TV, TX, false><<<gp0, nir::kBlock, sp, s>>>(
-                ap, bvals<TV>(LT), Vec<TX>::y(h), Vec<TX>::x(h), Vec<TX>::xb(h), Vec<TX>::xp(h), Vec<TX>::c(h),
-                Vec<TX>::l(h), Vec<TX>::u(h), Vec<TX>::x0(h));
-        NIR_LAUNCHED();
-        if (check)
-            nir::k_bdual<LD, TV, TX, true><<<gd1, nir::kBlock, sd, s>>>(ad, bvals<TV>(LA), Vec<TX>::xb(h),
-                                                                        Vec<TX>::y(h), Vec<TX>::yp(h), Vec<TX>::rl(h),
-                                                                        Vec<TX>::ru(h), Vec<TX>::y0(h));
-        else
-            nir::k_bdual<LD, TV, TX, false><<<gd0, nir::kBlock, sd, s>>>(ad, bvals<TV>(LA), Vec<TX>::xb(h),
-                                                                         Vec<TX>::y(h), Vec<TX>::yp(h), Vec<TX>::rl(h),
-                                                                         Vec<TX>::ru(h), Vec<TX>::y0(h));
-        NIR_LAUNCHED();
+        // as for one LP: all but the first start before the kernel ahead has ended
+        const auto kp = check ? nir::k_bprimal<LP, TV, TX, true> : nir::k_bprimal<LP, TV, TX, false>;
+        launch_kernel(h, i > i_first, kp, check ? gp1 : gp0, sp, ap, bvals<TV>(LT), Vec<TX>::y(h), Vec<TX>::x(h),
+                      Vec<TX>::xb(h), Vec<TX>::xp(h), Vec<TX>::c(h), Vec<TX>::l(h), Vec<TX>::u(h), Vec<TX>::x0(h));
+        const auto kd = check ? nir::k_bdual<LD, TV, TX, true> : nir::k_bdual<LD, TV, TX, false>;
+        launch_kernel(h, true, kd, check ? gd1 : gd0, sd, ad, bvals<TV>(LA), Vec<TX>::xb(h), Vec<TX>::y(h),
+                      Vec<TX>::yp(h), Vec<TX>::rl(h), Vec<TX>::ru(h), Vec<TX>::y0(h));
         h->launches += 2;
     }
     nir::BatchArgs kr = bargs(B, false, KR, 0, 0, phase, 0.0);

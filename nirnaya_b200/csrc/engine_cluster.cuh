@@ -359,7 +359,7 @@ double cl_time(double nnz, double entries, int C) {
     const double per = 0.35 + 0.04 * std::log2(double(C));
     return (C >= 16 ? 2.9 : 2.4) + 1e-3 * per * nnz / C + (C > 1 ? 0.2e-3 * entries : 0.0);
 }
-double cl_launch_time(double nnz) { return 7.8 + 7.5e-6 * nnz; }
+double cl_launch_time(double nnz) { return 5.3 + 7e-6 * nnz; }
 // Clusters must be this much faster by the estimate, whose error is about
 // as large.
 constexpr double kClMargin = 0.9;
@@ -384,11 +384,12 @@ double cl_arrivals(const ClusterPlan& P, int i) {
 // The plan a single LP's solve runs on, or null for the per-launch kernels.
 // The cluster is as large as shortens an iteration: 16 CTAs, fewer on an LP
 // whose rows do not fill them.  Built where clusters are faster even with
-// nothing to exchange (below about 160,000 nonzeros), kept where they still
-// are with what the plan exchanges: 4.8 against 8.1 us an iteration on a
-// random 2,000 x 5,000 LP of 40,000 nonzeros, 6.3 against 8.5 on a
-// multiperiod one of 126,000, but 9.1 against 9.3 on one of 200,000 and 10
-// against 9 on a blending LP of 100,000 whose ranks need nearly all entries.
+// nothing to exchange (below about 70,000 nonzeros), kept where they still
+// are with what the plan exchanges: 2.7 against 5.4 us an iteration on a
+// 60 x 150 LP, 4.8 against 5.9 on a random 2,000 x 5,000 one of 40,000
+// nonzeros, 3.5 against 5.2 on a multiperiod one of 15,000, but 6.3 against
+// 6.3 on one of 126,000 and 10 against 6.9 on a blending LP of 100,000 whose
+// ranks need nearly all entries.
 ClusterPlan* cl_single(nir_pdhg* h, const nir_pdhg_params& p) {
     if (!cl_takes(h, p) || h->m < 1 || h->n < 1) return nullptr;
     if (h->cluster_size < 0) {

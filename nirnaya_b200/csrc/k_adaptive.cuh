@@ -42,12 +42,13 @@ namespace nir {
 #endif
 // Gathers of the multiplied vector.  A kernel that runs several
 // iterations (the persistent chunk kernel) rewrites that vector between
-// its grid barriers, so it must gather through L2 (coherent, ld.global.cg)
-// rather than through the read-only path, which may serve a stale line.
+// its grid barriers, so it must gather through L2 (coherent, ld.global.cg).
+// The others gather through L1, but not by the read-only path: a kernel
+// launched early overlaps the one that writes the vector.
 template <bool COH, typename T>
 __device__ __forceinline__ T gather_ld(const T* p) {
     if (COH) return __ldcg(p);
-    return __ldg(p);
+    return __ldca(p);
 }
 
 // Same choice for the per-row operands of the iteration epilogues (cost,
@@ -218,7 +219,10 @@ __device__ __forceinline__ void rowblock_spmv(const int2* __restrict__ blk, int 
     TA* s_prod = reinterpret_cast<TA*>(nir_smem) + w * kWarpCapMax;
     const int G = gridDim.x * kWarps;
     int b = blockIdx.x * kWarps + w;
-    if (b >= nblk) return;
+    if (b >= nblk) {
+        pdl_wait();
+        return;
+    }
     int2 d0 = __ldg(blk + b), d1 = __ldg(blk + b + 1);
     int c[kWarpU];
     TV v[kWarpU];
@@ -228,6 +232,7 @@ __device__ __forceinline__ void rowblock_spmv(const int2* __restrict__ blk, int 
         n0 = __ldg(blk + b + G);
         n1 = __ldg(blk + b + G + 1);
     }
+    pdl_wait();  // descriptors and matrix are constant; the vectors come from the kernel before
     for (;;) {
         const bool has_next = b + G < nblk;
         int cn[kWarpU];

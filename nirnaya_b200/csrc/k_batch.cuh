@@ -148,7 +148,10 @@ __device__ __forceinline__ void lay_spmv_batch(const BatchArgs& a, const TV* __r
         const int nact = __ldg(a.act_n);
         const int total = nact > 0 ? __ldg(a.act_off + nact) : 0;
         int pos = blockIdx.x * kWarps + w;
-        if (pos >= total) return;
+        if (pos >= total) {
+            pdl_wait();
+            return;
+        }
         int inst = 0;
         int b = visited_block(a, pos, nact, inst);
         int2 d0 = __ldg(blk + b), d1 = __ldg(blk + b + 1);
@@ -156,6 +159,7 @@ __device__ __forceinline__ void lay_spmv_batch(const BatchArgs& a, const TV* __r
         int c[kWarpU];
         TV v[kWarpU];
         stream_load<TV>(d0, d1, act ? L.cap : -1, L.ci, val, c, v);
+        pdl_wait();  // lists, states and matrix do not change during a chunk
         for (;;) {
             const int pn = pos + G;
             const bool has_next = pn < total;
@@ -195,6 +199,7 @@ __device__ __forceinline__ void lay_spmv_batch(const BatchArgs& a, const TV* __r
         int k = 0;
         const int nact = __ldg(a.act_n);
         const int total = nact > 0 ? __ldg(a.act_off + nact) : 0;
+        pdl_wait();
         for (int pos = blockIdx.x; pos < total; pos += gridDim.x) {
             int inst = 0;
             const int b = visited_block(a, pos, nact, inst);
@@ -215,6 +220,7 @@ __global__ void __launch_bounds__(kBlock, (lay_min_blocks<LAY, TV, TX, true>()))
               TX* __restrict__ xbar, TX* __restrict__ xplus, const TX* __restrict__ c, const TX* __restrict__ lo,
               const TX* __restrict__ up, const TX* __restrict__ x0) {
     __shared__ double s_red[kWarps];
+    pdl_release();
     PrimalEpi<TX, CHECK> epi;
     epi.x = x;
     epi.xbar = xbar;
@@ -234,6 +240,7 @@ __global__ void __launch_bounds__(kBlock, (lay_min_blocks<LAY, TV, TX, true>()))
     k_bdual(BatchArgs a, const TV* __restrict__ val, const TX* __restrict__ xbar, TX* __restrict__ y,
             TX* __restrict__ yplus, const TX* __restrict__ rl, const TX* __restrict__ ru, const TX* __restrict__ y0) {
     __shared__ double s_red[kWarps];
+    pdl_release();
     DualEpi<TX, CHECK> epi;
     epi.y = y;
     epi.yplus = yplus;

@@ -1,7 +1,7 @@
 // Chunks of iterations inside one thread-block cluster per LP.
 //
 // A small or medium LP spends its iteration on latency, not on bandwidth:
-// two kernels of a CUDA graph take about 6.5 us on a 2,000 x 5,000 LP of
+// two kernels of a CUDA graph take about 5.9 us on a 2,000 x 5,000 LP of
 // 40,000 nonzeros whose arithmetic takes a tenth of that, and a batch of
 // such LPs gathers from a vector that would fit in shared memory.  Here a
 // cluster of C CTAs (C = 1, 2, 4, 8 or 16) takes one LP through a whole
@@ -27,9 +27,8 @@
 //     the slots to store to, and the matrix itself.
 //
 // Measured on B200 (us per iteration, checks included, against the
-// per-launch kernels): 2.6 against 7.5 on a 60 x 150 LP, 4.8 against 8.1 on
-// the 2,000 x 5,000 one (16 CTAs), 6.3 against 8.5 on a 5,000 x 12,500
-// multiperiod LP of 126,000 nonzeros; 97 against 204 for a batch of 128
+// per-launch kernels): 2.7 against 5.4 on a 60 x 150 LP, 4.8 against 5.9 on
+// the 2,000 x 5,000 one (16 CTAs); 85 against 180 for a batch of 128
 // multiperiod LPs of 500 to 20,000 rows (16M nonzeros, clusters of 4), 5.5
 // against 12.6 for 96 LPs of 50 to 400 rows (clusters of 1).  Small LPs are
 // bound by the latency of a pass, about 1,300 cycles from the last arrival

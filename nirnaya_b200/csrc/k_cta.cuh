@@ -102,12 +102,13 @@ __device__ __forceinline__ void ld_val(const float* __restrict__ p, int pos, int
     }
 }
 
-// Gathers of the multiplied vector: the read-only path, or L2 (coherent)
-// for a kernel that rewrites the vector between grid barriers.
+// Gathers of the multiplied vector: through L1 (not the read-only path: a
+// kernel launched early overlaps the one that writes it), or through L2
+// (coherent) for a kernel that rewrites the vector between grid barriers.
 template <bool COH, typename T>
 __device__ __forceinline__ T cta_gather(const T* p) {
     if (COH) return __ldcg(p);
-    return __ldg(p);
+    return __ldca(p);
 }
 
 // ---------------------------------------------------------------- block state
@@ -271,6 +272,7 @@ __device__ __forceinline__ void cta_spmv(const int4* __restrict__ blk, int nblk,
                                          const int* __restrict__ ci, const TV* __restrict__ val,
                                          const TX* __restrict__ x, Epi& epi, CtaShared<TA>* sm) {
     int k = 0;
+    pdl_wait();
     for (int b = blockIdx.x; b < nblk; b += gridDim.x, ++k) {
         const int4 d0 = __ldg(blk + b), d1 = __ldg(blk + b + 1);
         cta_block<TA, TV, TX, E, Epi, COH>(d0, d1, rp, ci, val, x, epi, sm[k & 1]);
