@@ -352,17 +352,17 @@ int cl_forced() {
 // What an iteration costs, in microseconds, as measured on B200 for LPs of
 // 1,200 to 500,000 nonzeros on clusters of 1 to 16: the latency of two
 // passes, the gathers of an SM (0.35 per 1,000 nonzeros, and more the more
-// ranks wait for the slowest) and the entries that come from other ranks.
+// ranks wait for the slowest) and the entries that come from other ranks
+// (0.6 for 6,500 on the 2,000 x 5,000 LP, 1.9 for 9,800, 3.9 for 16,400).
 // Against it the two launches of the per-launch kernels while the LP lies
 // in L2.
 double cl_time(double nnz, double entries, int C) {
-    const double per = 0.35 + 0.04 * std::log2(double(C));
-    return (C >= 16 ? 2.9 : 2.4) + 1e-3 * per * nnz / C + (C > 1 ? 0.2e-3 * entries : 0.0);
+    const double per = 0.35 + 0.04 * std::log2(double(C)), k = 1e-3 * entries;
+    return (C >= 16 ? 2.9 : 2.4) + 1e-3 * per * nnz / C + (C > 1 ? k * (0.04 + 0.0125 * k) : 0.0);
 }
 double cl_launch_time(double nnz) { return 5.3 + 7e-6 * nnz; }
-// Clusters must be this much faster by the estimate, whose error is about
-// as large.
-constexpr double kClMargin = 0.9;
+// Clusters must be this much faster by the estimate.
+constexpr double kClMargin = 0.95;
 
 void cl_prepare_kernels() {
     cl_prepare_kernel<false, float>();
@@ -384,7 +384,7 @@ double cl_arrivals(const ClusterPlan& P, int i) {
 // The plan a single LP's solve runs on, or null for the per-launch kernels.
 // The cluster is as large as shortens an iteration: 16 CTAs, fewer on an LP
 // whose rows do not fill them.  Built where clusters are faster even with
-// nothing to exchange (below about 70,000 nonzeros), kept where they still
+// nothing to exchange (below about 85,000 nonzeros), kept where they still
 // are with what the plan exchanges: 2.7 against 5.4 us an iteration on a
 // 60 x 150 LP, 4.8 against 5.9 on a random 2,000 x 5,000 one of 40,000
 // nonzeros, 3.5 against 5.2 on a multiperiod one of 15,000, but 6.3 against
