@@ -1222,18 +1222,26 @@ struct RefProbe {
 void launch_ref_chunk(nir_pdhg* h, int K, const RefProbe* probe) {
     cudaStream_t s = h->stream;
     const PartLayout L = part_layout(h);
-    const unsigned gm = grid_for(h->m), gn = grid_for(h->n);
+    auto ctas = [](const Orient& o) { return std::max(1, (o.nblk + nir::kWarps - 1) / nir::kWarps); };
+    const int gn = ctas(h->At), gm = ctas(h->A);
     for (int i = 0; i < K; ++i) {
-        nir::k_ref_primal<<<std::max(gn, 1u), nir::kBlock, 0, s>>>(h->n, h->At.rp, h->At.ci, h->At.v_orig, h->y64, h->c,
-                                                                    h->l, h->u, h->x64, h->xb64, h->st, i);
-        NIR_LAUNCHED();
-        nir::k_ref_dual<<<std::max(gm, 1u), nir::kBlock, 0, s>>>(h->m, h->A.rp, h->A.ci, h->A.v_orig, h->xb64, h->rl,
-                                                                  h->ru, h->y64, L.misc, h->st, i);
-        NIR_LAUNCHED();
-        nir::k_ref_stop<<<1, nir::kBlock, 0, s>>>(L.misc, std::max<int>(gm, 1), h->st, i, K);
-        NIR_LAUNCHED();
-        h->launches += 3;
+        // the first step of the chunk and the one after the stop test read
+        // the state a kernel before them wrote; the others start early
+        launch_kernel(h, i > 1, nir::k_refb_primal, gn, 0, (const int2*)h->At.blk, h->At.nblk, h->At.cap, h->At.rp,
+                      h->At.ci, h->At.v_orig, h->y64, h->c, h->l, h->u, h->x64, h->xb64, h->st, i);
+        launch_kernel(h, true, i == 0 ? nir::k_refb_dual<true> : nir::k_refb_dual<false>, gm, 0, (const int2*)h->A.blk,
+                      h->A.nblk, h->A.cap, h->A.rp, h->A.ci, h->A.v_orig, h->xb64, h->rl, h->ru, h->y64, h->tmp_m, h->st, i);
+        h->launches += 2;
+        if (i == 0) {
+            // one maximum per CTA, at most one CTA per row
+            nir::k_refb_test<<<1, nir::kBlock, 0, s>>>(h->tmp_m, gm, h->st);
+            NIR_LAUNCHED();
+            h->launches += 1;
+        }
     }
+    nir::k_refb_end<<<1, 32, 0, s>>>(h->st, K);
+    NIR_LAUNCHED();
+    h->launches += 1;
     if (probe) {
         // KKT of (x, y) on the unscaled matrix (dr = dc = 1): reads only
         int gkr = 0, gkc = 0;
@@ -1285,7 +1293,7 @@ struct LoopResult {
     double t_switch = 0.0;
 };
 
-int launches_per_chunk(int K, bool ref) { return ref ? 3 * K + 1 : 2 * K + 5; }
+int launches_per_chunk(int K, bool ref) { return ref ? 2 * K + 3 : 2 * K + 5; }
 
 // Runs chunks until the device reports done, the phase changes, or the
 // caller's poll / time limit stops it.  Keeps `depth` chunks in flight.
@@ -1380,6 +1388,8 @@ int solve_reference(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), v
     cudaStream_t s = h->stream;
     const double t0 = now_sec();
     ensure_partials(h);
+    // row blocks of both orientations (the order of a row's sum does not depend on them)
+    for (Orient* o : {&h->A, &h->At}) set_blocks(h, *o, auto_cap(h->nnz, o->rows));
     const int n = h->n, m = h->m;
     nir::DevState st0{};
     st0.max_iters = p.max_iters;
@@ -1405,7 +1415,7 @@ int solve_reference(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), v
     for (int r = 0; r < 12; ++r) {
         nir::k_ref_spmv<<<std::max(grid_for(m), 1u), nir::kBlock, 0, s>>>(m, h->A.rp, h->A.ci, h->A.v_orig, h->tmp_n, h->tmp_m);
         nir::k_ref_spmv<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->At.rp, h->At.ci, h->At.v_orig, h->tmp_m, h->tmp_n);
-        nir::k_ref_norm<<<1, 32, 0, s>>>(n, h->tmp_n, h->st);
+        nir::k_ref_norm<<<1, nir::kBlock, 0, s>>>(n, h->tmp_n, h->st);
         nir::k_ref_div<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->tmp_n, h->st);
         NIR_LAUNCHED();
         h->launches += 4;
@@ -1424,7 +1434,7 @@ int solve_reference(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), v
             KeyHash key;
             key.add(1000).add(probing).add(probe.bnorm).add(probe.cnorm).add(probe.tol).add(h->offset);
             if (probing) key.add(lay_of(h->A).blk).add(lay_of(h->At).blk).add(h->A.lay).add(h->At.lay);
-            key.add(h->part);
+            key.add(h->part).add(h->A.blk).add(h->A.cap).add(h->At.blk).add(h->At.cap);
             cudaGraphExec_t ge = chunk_graph(h, 0, key.h, launch);
             const int per = launches_per_chunk(K, true) + (probing ? 3 : 0);
             R = run_chunks(h, p, poll, ctx, t0, 0, per, [&]() { NIR_CUDA(cudaGraphLaunch(ge, s)); }, nullptr);
@@ -1886,7 +1896,7 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
         for (int r = 0; r < 12; ++r) {
             nir::k_ref_spmv<<<std::max(grid_for(m), 1u), nir::kBlock, 0, s>>>(m, h->A.rp, h->A.ci, h->A.v_orig, h->tmp_n, h->tmp_m);
             nir::k_ref_spmv<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->At.rp, h->At.ci, h->At.v_orig, h->tmp_m, h->tmp_n);
-            nir::k_ref_norm<<<1, 32, 0, s>>>(n, h->tmp_n, h->st);
+            nir::k_ref_norm<<<1, nir::kBlock, 0, s>>>(n, h->tmp_n, h->st);
             nir::k_ref_div<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->tmp_n, h->st);
         }
         nir::k_ref_steps<<<1, 32, 0, s>>>(h->st);
@@ -2823,7 +2833,7 @@ extern "C" int nir_pdhg_reference_solve_noalloc(const nir_csr_dev* A, const nir_
         for (int r = 0; r < 12; ++r) {
             nir::k_ref_spmv<<<gm, nir::kBlock, 0, s>>>(mi, A->row_ptr, A->col_idx, A->value, u, v);
             nir::k_ref_spmv<<<gn, nir::kBlock, 0, s>>>(ni, At->row_ptr, At->col_idx, At->value, v, u);
-            nir::k_ref_norm<<<1, 32, 0, s>>>(ni, u, st);
+            nir::k_ref_norm<<<1, nir::kBlock, 0, s>>>(ni, u, st);
             nir::k_ref_div<<<gn, nir::kBlock, 0, s>>>(ni, u, st);
         }
         nir::k_ref_steps<<<1, 32, 0, s>>>(st);

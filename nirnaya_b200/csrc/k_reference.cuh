@@ -10,6 +10,7 @@
 #pragma once
 
 #include "dev_common.cuh"
+#include "row_blocks.hpp"
 
 namespace nir {
 
@@ -23,13 +24,35 @@ __global__ void k_ref_spmv(int rows, const int* __restrict__ rp, const int* __re
     y[r] = s;
 }
 
-// Power-iteration norm, src/gpu/pdhg_solver.hpp:38-41: one thread adds
-// u_j^2 in index order, then norm_est = sqrt(max(1e-12, n2)).
-__global__ void k_ref_norm(int n, const double* __restrict__ u, DevState* st) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+// Power-iteration norm, src/gpu/pdhg_solver.hpp:38-41: u_j^2 added in index
+// order, then norm_est = sqrt(max(1e-12, n2)).  One CTA: the sum is one
+// chain, so one thread carries it and the other warps keep the squares ready
+// in shared memory, a tile ahead (5,000 terms: 195 us with the loads on the
+// chain, 40 without).
+constexpr int kRefTile = kBlock - 32;
+__global__ void __launch_bounds__(kBlock) k_ref_norm(int n, const double* __restrict__ u, DevState* st) {
+    __shared__ double sq[2][kRefTile];
+    if (blockIdx.x != 0) return;
+    auto fill = [&](int base, int b) {
+        const int k = int(threadIdx.x) - 32;
+        if (k < 0) return;
+        const double v = base + k < n ? u[base + k] : 0.0;
+        sq[b][k] = __dmul_rn(v, v);
+    };
     double n2 = 0.0;
-    for (int j = 0; j < n; ++j) n2 = __dadd_rn(n2, __dmul_rn(u[j], u[j]));
-    st->ref_norm_est = __dsqrt_rn(smax(1e-12, n2));
+    fill(0, 0);
+    __syncthreads();
+    for (int base = 0, t = 0; base < n; base += kRefTile, ++t) {
+        const int b = t & 1;
+        if (base + kRefTile < n) fill(base + kRefTile, b ^ 1);
+        if (threadIdx.x == 0) {
+            // n2 >= 0, so the zeros past the end change nothing
+#pragma unroll 8
+            for (int k = 0; k < kRefTile; ++k) n2 = __dadd_rn(n2, sq[b][k]);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) st->ref_norm_est = __dsqrt_rn(smax(1e-12, n2));
 }
 
 __global__ void k_ref_div(int n, double* __restrict__ u, const DevState* __restrict__ st) {
@@ -107,6 +130,157 @@ __global__ void k_ref_dual(int m, const int* __restrict__ rp, const int* __restr
     // max is order-independent, so the tree gives the reference's value
     double bm = block_max(viol, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = bm;
+}
+
+// ---- the same steps over warp row blocks (row_blocks.hpp)
+//
+// With a thread per row a warp's loads of 32 rows scatter over as many cache
+// lines, and every term waits for its loads.  Over row blocks a warp reads
+// the block's entries with consecutive lanes, gathers and multiplies them
+// all at once, and leaves the rounded products in shared memory; each row's
+// products are then added in their order by the row's own lane.  The bits
+// are the same; only the additions are left on the chain.  A row longer than
+// the block capacity is added by one lane, 256 products at a time.
+
+// One warp's block: fin(row, sum) on the row's lane.
+template <class Fin>
+__device__ __forceinline__ void ref_block(int2 d0, int2 d1, int cap, const int* __restrict__ rp,
+                                          const int* __restrict__ ci, const double* __restrict__ val,
+                                          const double* __restrict__ x, double* s_prod, Fin fin) {
+    const int lane = threadIdx.x & 31;
+    const int r0 = d0.x, p0 = d0.y, nrows = d1.x - d0.x, nnzb = d1.y - d0.y;
+    const int r = r0 + lane;
+    int ra = 0, re = 0;
+    if (nnzb <= cap && lane < nrows) {
+        ra = max(__ldg(rp + r) - p0, 0);
+        re = min(__ldg(rp + r + 1) - p0, nnzb);
+    }
+    double s = 0.0;
+    for (int base = 0; base < nnzb; base += kWarpCapMax) {
+        int c[kWarpU];
+        double v[kWarpU];
+#pragma unroll
+        for (int q = 0; q < kWarpU; ++q) {
+            const int k = base + lane + 32 * q;
+            c[q] = k < nnzb ? __ldg(ci + p0 + k) : 0;
+            v[q] = k < nnzb ? __ldg(val + p0 + k) : 0.0;
+        }
+        if (base == 0) pdl_wait();
+#pragma unroll
+        for (int q = 0; q < kWarpU; ++q) {
+            const int k = base + lane + 32 * q;
+            if (k < nnzb) s_prod[lane + 32 * q] = __dmul_rn(v[q], __ldca(x + c[q]));
+        }
+        __syncwarp();
+        if (nnzb <= cap) {
+            for (int k = ra; k < re; ++k) s = __dadd_rn(s, s_prod[k]);
+        } else if (lane == 0) {
+            const int n = min(kWarpCapMax, nnzb - base);
+#pragma unroll 4
+            for (int k = 0; k < n; ++k) s = __dadd_rn(s, s_prod[k]);
+        }
+        __syncwarp();
+    }
+    if (nnzb == 0) pdl_wait();
+    if (lane < nrows) fin(r, s);
+}
+
+__device__ __forceinline__ bool ref_over(const DevState* st, int i_in_chunk) {
+    return st->done || st->iter + i_in_chunk >= st->max_iters;
+}
+
+// Primal step, src/gpu/pdhg_solver.hpp:69-78.
+__global__ void __launch_bounds__(kBlock) k_refb_primal(const int2* __restrict__ blk, int nblk, int cap,
+                                                        const int* __restrict__ rp, const int* __restrict__ ci,
+                                                        const double* __restrict__ v, const double* __restrict__ y,
+                                                        const double* __restrict__ cost, const double* __restrict__ lo,
+                                                        const double* __restrict__ up, double* __restrict__ x,
+                                                        double* __restrict__ xbar, const DevState* __restrict__ st,
+                                                        int i_in_chunk) {
+    __shared__ double prod[kWarps][kWarpCapMax];
+    pdl_release();
+    const int w = threadIdx.x >> 5, b = blockIdx.x * kWarps + w;
+    // the first kernel of a chunk is launched after the one that wrote the state
+    if (b >= nblk || ref_over(st, i_in_chunk)) {
+        pdl_wait();
+        return;
+    }
+    const double tau = st->tau;
+    ref_block(blk[b], blk[b + 1], cap, rp, ci, v, y, prod[w], [&](int j, double s) {
+        const double xj = x[j], l = lo[j], u = up[j];
+        double cand = __dsub_rn(xj, __dmul_rn(tau, __dsub_rn(cost[j], s)));
+        if (fin_bound(l)) cand = smax(l, cand);
+        if (fin_bound(u)) cand = smin(u, cand);
+        xbar[j] = __dsub_rn(__dmul_rn(2.0, cand), xj);
+        x[j] = cand;
+    });
+}
+
+// Dual step, src/gpu/pdhg_solver.hpp:80-95; TEST: also each CTA's violation
+// maximum to part[] (the stop test reads it every 32nd iteration only).
+template <bool TEST>
+__global__ void __launch_bounds__(kBlock) k_refb_dual(const int2* __restrict__ blk, int nblk, int cap,
+                                                      const int* __restrict__ rp, const int* __restrict__ ci,
+                                                      const double* __restrict__ v, const double* __restrict__ xbar,
+                                                      const double* __restrict__ rlo, const double* __restrict__ rup,
+                                                      double* __restrict__ y, double* __restrict__ part,
+                                                      const DevState* __restrict__ st, int i_in_chunk) {
+    __shared__ double prod[kWarps][kWarpCapMax];
+    __shared__ double sh[kWarps];
+    pdl_release();
+    const int w = threadIdx.x >> 5, b = blockIdx.x * kWarps + w;
+    if (ref_over(st, i_in_chunk)) {
+        pdl_wait();
+        return;
+    }
+    double viol = 0.0;
+    if (b < nblk) {
+        const double sigma = st->sigma;
+        ref_block(blk[b], blk[b + 1], cap, rp, ci, v, xbar, prod[w], [&](int i, double a) {
+            const double yi = y[i], lo = rlo[i], hi = rup[i];
+            double r = __dsub_rn(a, __ddiv_rn(yi, sigma));
+            if (fin_bound(lo)) r = smax(lo, r);
+            if (fin_bound(hi)) r = smin(hi, r);
+            y[i] = __dadd_rn(yi, __dmul_rn(sigma, __dsub_rn(r, a)));
+            if (TEST) {
+                if (fin_bound(lo)) viol = smax(viol, __dsub_rn(lo, a));
+                if (fin_bound(hi)) viol = smax(viol, __dsub_rn(a, hi));
+            }
+        });
+    } else {
+        pdl_wait();
+    }
+    if (TEST) {
+        const double bm = block_max(viol, sh);
+        if (threadIdx.x == 0) part[blockIdx.x] = bm;
+    }
+}
+
+// The stop test after a chunk's first iteration (chunks start at multiples
+// of 32, their length) and the end of a chunk: k_ref_stop's outcomes with
+// two launches a chunk instead of one an iteration.
+__global__ void k_refb_test(const double* __restrict__ part, int nblk, DevState* st) {
+    __shared__ double sh[kWarps];
+    const long long it = st->iter;
+    if (st->done || it >= st->max_iters || it <= 20) return;
+    const double mx = block_max_array(part, nblk, sh);
+    if (threadIdx.x == 0 && mx <= 1e-6) {
+        st->done = 1;
+        st->ref_stopped = 1;
+        st->status = 0;
+        st->ref_iterations = it + 1;
+    }
+}
+__global__ void k_refb_end(DevState* st, int K) {
+    if (threadIdx.x != 0 || st->done) return;
+    if (st->iter + K >= st->max_iters) {
+        st->done = 1;
+        st->status = 6;  // NIR_STATUS_ITERATION_LIMIT
+        st->ref_iterations = st->max_iters;
+        return;
+    }
+    st->iter += K;
+    st->ref_iterations = st->iter;
 }
 
 // Stop test after iteration `it`, src/gpu/pdhg_solver.hpp:97-100, and the
