@@ -1,5 +1,5 @@
-// Warm-start network: hand-written BF16 tensor-core GEMMs (mma.sync
-// m16n8k16, FP32 accumulation), fused epilogues, Adam, all on one stream.
+// Warm-start network: hand-written BF16 tensor-core GEMMs (tcgen05, FP32
+// accumulation), fused epilogues, Adam, all on one stream.
 // C ABI: include/nir_mlp.h.
 //
 // GEMM.  C[M x N] = sum_k A(m, k) * B(n, k).  Each operand is stored either
@@ -8,22 +8,26 @@
 //   forward   Y  = X * W^T      A = X  K-major,  B = W  K-major
 //   input grad dX = dY * W      A = dY K-major,  B = W  MN-major
 //   weight grad dW = dY^T * X   A = dY MN-major, B = X  MN-major
-// A CTA (8 warps) computes a 128 x 128 tile in steps of 32 along K; tiles
-// stream global -> shared with 16-byte cp.async (zero-filled outside the
-// matrix) through a 3-stage pipeline; warps read fragments with ldmatrix
-// (.trans for MN-major tiles) from XOR-swizzled rows (no bank conflicts)
-// and issue 16 mma.sync per 16-wide K step on a 64 x 32 warp tile.
-// Products with few output tiles and a long K split K over blockIdx.z into
-// FP32 partials that a second kernel sums in a fixed order (deterministic)
-// before the epilogue.
+// A CTA computes a tile of 128 rows and 64 or 128 columns: TMA brings the
+// operands into shared memory stage by stage, 64 of K each, one thread issues
+// tcgen05.mma on them, the FP32 accumulators lie in tensor memory, and 8
+// warps finish the tile (bias, ReLU, mask) and store it.
+// A product with few output tiles and a long K is a sum of splits of K, added
+// in order: a CTA keeps an accumulator for each, or the CTAs of a thread-block
+// cluster compute them side by side and add them through each other's shared
+// memory (deterministic).
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <random>
 #include <stdexcept>
 #include <string>
@@ -45,9 +49,7 @@ thread_local std::string g_err;
 
 using bf16 = __nv_bfloat16;
 
-constexpr int BM = 128, BN = 128, BK = 32, STAGES = 3, THREADS = 256;
-constexpr int TILE_BYTES = BM * BK * 2;                 // one operand tile, 8 KB
-constexpr int SMEM_BYTES = STAGES * 2 * TILE_BYTES;     // 48 KB
+constexpr int BM = 128, BN = 128, BK = 32;  // BM x BN: the tiles the splits of K are counted by
 
 enum Epi : int { EPI_BIAS_RELU_BF16 = 0, EPI_BIAS_F32 = 1, EPI_MASK_BF16 = 2, EPI_F32 = 3 };
 
@@ -58,7 +60,7 @@ struct GemmArgs {
     int ldb;
     int M, N, K;
     int kps;           // K range per split (multiple of BK)
-    int splits;        // gridDim.z; > 1: partials to ws
+    int splits;        // partial sums of kps each, added in order
     int epi;
     const float* bias;
     bf16* out_bf;
@@ -66,182 +68,376 @@ struct GemmArgs {
     int ldc;
     const bf16* mask;  // EPI_MASK_BF16: multiply by (mask > 0)
     int ldm;
-    float* ws;         // splits x M x N partials
+    bool wide;         // rows of whole, aligned groups of 8 columns
 };
 
-// Byte offset of 16-byte chunk c of row r in a swizzled tile.
-__device__ __forceinline__ int kmaj_off(int r, int c) { return r * 64 + ((c ^ ((r >> 1) & 3)) << 4); }   // 128 x 32
-__device__ __forceinline__ int mnmaj_off(int r, int c) { return r * 256 + ((c ^ (r & 7)) << 4); }       // 32 x 128
+// Programmatic dependent launch: with the launch attribute a kernel starts
+// while the one before still runs and waits for it before it reads what
+// that wrote; without it both do nothing.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
-    const int n = valid ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n));
-}
-
-__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-
-__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// One operand tile (rows r0.., K range k0..k0+BK) into shared memory.
-// K-major: 128 rows x 4 chunks; MN-major: 32 K-rows x 16 chunks.
-template <bool KMAJ>
-__device__ __forceinline__ void load_tile(uint32_t sbase, const bf16* __restrict__ P, int ld, int rows, int r0,
-                                          int k0, int kend) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int idx = threadIdx.x + i * THREADS;
-        if (KMAJ) {
-            const int r = idx >> 2, c = idx & 3;
-            const int gr = r0 + r, gk = k0 + c * 8;
-            const bool ok = gr < rows && gk < kend;
-            cp_async16(sbase + kmaj_off(r, c), ok ? (const void*)(P + (size_t)gr * ld + gk) : (const void*)P, ok);
-        } else {
-            const int r = idx >> 4, c = idx & 15;
-            const int gk = k0 + r, gr = r0 + c * 8;
-            const bool ok = gk < kend && gr < rows;
-            cp_async16(sbase + mnmaj_off(r, c), ok ? (const void*)(P + (size_t)gk * ld + gr) : (const void*)P, ok);
-        }
+// The epilogue of one element, and of 8 neighbouring columns (col a multiple
+// of 8), which are read and stored together where the rows allow it.
+__device__ __forceinline__ void epilogue1(const GemmArgs& g, int row, int col, float v) {
+    const size_t o = (size_t)row * g.ldc + col;
+    switch (g.epi) {
+        case EPI_BIAS_RELU_BF16: g.out_bf[o] = __float2bfloat16_rn(fmaxf(v + g.bias[col], 0.f)); break;
+        case EPI_BIAS_F32: g.out_f[o] = v + g.bias[col]; break;
+        case EPI_MASK_BF16:
+            g.out_bf[o] = __float2bfloat16_rn(__bfloat162float(g.mask[(size_t)row * g.ldm + col]) > 0.f ? v : 0.f);
+            break;
+        default: g.out_f[o] = v; break;
     }
 }
+__device__ __forceinline__ void epilogue8(const GemmArgs& g, int row, int col, const float (&in)[8]) {
+    if (!g.wide) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (col + j < g.N) epilogue1(g, row, col + j, in[j]);
+        return;
+    }
+    const size_t o = (size_t)row * g.ldc + col;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = in[j];
+    if (g.epi == EPI_BIAS_RELU_BF16 || g.epi == EPI_BIAS_F32) {
+        const float4* b = reinterpret_cast<const float4*>(g.bias + col);
+        const float4 b0 = b[0], b1 = b[1];
+        v[0] += b0.x, v[1] += b0.y, v[2] += b0.z, v[3] += b0.w;
+        v[4] += b1.x, v[5] += b1.y, v[6] += b1.z, v[7] += b1.w;
+    }
+    if (g.epi == EPI_BIAS_F32 || g.epi == EPI_F32) {
+        float4* q = reinterpret_cast<float4*>(g.out_f + o);
+        q[0] = make_float4(v[0], v[1], v[2], v[3]);
+        q[1] = make_float4(v[4], v[5], v[6], v[7]);
+        return;
+    }
+    union Pack {
+        uint4 q;
+        bf16 e[8];
+        __device__ Pack() {}
+    } out, m;
+    if (g.epi == EPI_MASK_BF16) {
+        m.q = *reinterpret_cast<const uint4*>(g.mask + (size_t)row * g.ldm + col);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) out.e[j] = __float2bfloat16_rn(__bfloat162float(m.e[j]) > 0.f ? v[j] : 0.f);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) out.e[j] = __float2bfloat16_rn(fmaxf(v[j], 0.f));
+    }
+    *reinterpret_cast<uint4*>(g.out_bf + o) = out.q;
+}
 
+// ---- the GEMM kernel
+//
+// A CTA of 8 warps computes a 128 x TN tile in tensor memory, 64 of K a
+// stage.  One thread has the operands brought into shared memory by TMA, in
+// the 128-byte swizzle that the tensor core reads, several stages ahead;
+// another issues each stage's tcgen05.mma (K = 16 each, in order).  A CTA
+// computes G.accs splits one after another, each in its own accumulator, and
+// adds them in order as it reads them; or (G.rank_bits > 0) the CTAs of a
+// cluster share the tile: in each round a rank computes one split and leaves
+// it in shared memory, where the stages were, and every rank adds its share
+// of the tile's rows over the splits in order, reading the other ranks'
+// shared memory.  Neither the tile nor the ranks decide the order of any sum.
+// One launch takes a group of independent products (the weight gradients of
+// all layers).
+// Small products are bound by their latency (load, multiply, read back,
+// store), large ones by the loads: with 128 x 128 tiles a stage's 32 KB from
+// L2 take longer than its 256 cycles of multiplication.  In TFLOP/s, with
+// mma.sync on 128 x 128 tiles and splits added by another kernel before:
+// 8192^3 280 -> 1290, 4096^3 327 -> 1110, 65536 x 512 x 512 222 -> 490,
+// 8192 x 512 x 512 75 -> 420, 1024 x 512 x 512 29 -> 80.
+constexpr int GROUP_MAX = 17;  // layers
+constexpr int RANK_BITS_MAX = 4;
+constexpr int STAGES_MAX = 6;
+constexpr int SK = 64;         // K of a stage
+constexpr int TMEM_COLUMNS = 512;  // of an SM
+constexpr int GEMM_WAIT_MAX = 1 << 20;
+
+template <int TN>
+struct GTile {
+    static constexpr int threads = 256;
+    static constexpr int bytes_a = 128 * SK * 2, bytes_b = TN * SK * 2;
+    static constexpr int stage = bytes_a + bytes_b;      // 24 or 32 KB
+    static constexpr int ld = TN + 4;                    // floats per row of the finished tile
+    // dynamic shared memory, from a multiple of 1024: the stages, or the tile
+    static constexpr int tile = 128 * ld * 4;
+    static int smem(int stages) { return std::max(stages * stage, tile) + 1024; }
+};
+
+struct GemmOne {
+    alignas(64) CUtensorMap a, b;
+    GemmArgs g;
+};
+template <int MAX>
+struct GemmGroupOf {
+    GemmOne g[MAX];
+    int first[MAX + 1];  // first tile of each product
+    int count;
+    int rank_bits;       // 2^rank_bits CTAs per tile
+    int accs;            // splits that a CTA computes one after another, each in its own accumulator (one CTA per tile)
+    int stages;          // at most STAGES_MAX
+    uint32_t tmem;       // columns of tensor memory for them, a power of two
+    int* fault;          // set if a wait of the kernel gives up
+};
+// Weight gradients come in groups, the other products one by one (the
+// arguments of a launch are copied by the host).
 template <bool AK, bool BKM>
-__global__ void __launch_bounds__(THREADS) k_gemm(GemmArgs g) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    const uint32_t sb = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp >> 2, wn = warp & 3;  // 2 x 4 warps, 64 x 32 each
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int kbeg = blockIdx.z * g.kps;
-    const int kend = min(g.K, kbeg + g.kps);
-    const int KT = (kend > kbeg) ? (kend - kbeg + BK - 1) / BK : 0;
+using GemmGroup = GemmGroupOf<(!AK && !BKM) ? GROUP_MAX : 1>;
 
-    float acc[4][4][4];
+// A stage's operand: K-major ROWS rows of 64 k (128 bytes); MN-major 64
+// K-rows of 64 rows (128 bytes), 64 ROWS after 64 ROWS.
+template <int ROWS, bool KMAJ>
+__device__ __forceinline__ void load_operand(uint32_t dst, const CUtensorMap* map, int r0, int k0, uint32_t bar) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
-
-    auto stageA = [&](int s) { return sb + s * 2 * TILE_BYTES; };
-    auto stageB = [&](int s) { return sb + s * 2 * TILE_BYTES + TILE_BYTES; };
-
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < KT) {
-            load_tile<AK>(stageA(s), g.A, g.lda, g.M, m0, kbeg + s * BK, kend);
-            load_tile<BKM>(stageB(s), g.B, g.ldb, g.N, n0, kbeg + s * BK, kend);
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-    }
-
-    for (int kt = 0; kt < KT; ++kt) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
-        __syncthreads();
-        const int nk = kt + STAGES - 1;
-        if (nk < KT) {
-            load_tile<AK>(stageA(nk % STAGES), g.A, g.lda, g.M, m0, kbeg + nk * BK, kend);
-            load_tile<BKM>(stageB(nk % STAGES), g.B, g.ldb, g.N, n0, kbeg + nk * BK, kend);
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-        const uint32_t sa = stageA(kt % STAGES), sbb = stageB(kt % STAGES);
-#pragma unroll
-        for (int kk = 0; kk < BK; kk += 16) {
-            uint32_t af[4][4];
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi) {
-                const int mb = wm * 64 + mi * 16;
-                if (AK) {
-                    const int r = mb + (lane & 15), c = (kk >> 3) + (lane >> 4);
-                    ldsm_x4(sa + kmaj_off(r, c), af[mi]);
-                } else {
-                    const int j = lane >> 3;
-                    const int r = kk + (j >> 1) * 8 + (lane & 7), c = (mb + (j & 1) * 8) >> 3;
-                    ldsm_x4_t(sa + mnmaj_off(r, c), af[mi]);
-                }
-            }
-            uint32_t bfr[2][4];
-#pragma unroll
-            for (int np = 0; np < 2; ++np) {
-                const int nb = wn * 32 + np * 16;
-                const int j = lane >> 3;
-                if (BKM) {
-                    const int r = nb + (j >> 1) * 8 + (lane & 7), c = (kk >> 3) + (j & 1);
-                    ldsm_x4(sbb + kmaj_off(r, c), bfr[np]);
-                } else {
-                    const int r = kk + (j & 1) * 8 + (lane & 7), c = (nb + (j >> 1) * 8) >> 3;
-                    ldsm_x4_t(sbb + mnmaj_off(r, c), bfr[np]);
-                }
-            }
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-                    mma_bf16(acc[mi][ni], af[mi], bfr[ni >> 1][(ni & 1) * 2], bfr[ni >> 1][(ni & 1) * 2 + 1]);
-        }
-    }
-    asm volatile("cp.async.wait_group 0;\n" ::);
-
-    const int gq = lane >> 2, tq = lane & 3;
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int row = m0 + wm * 64 + mi * 16 + gq + (e >> 1) * 8;
-                const int col = n0 + wn * 32 + ni * 8 + tq * 2 + (e & 1);
-                if (row >= g.M || col >= g.N) continue;
-                const float v = acc[mi][ni][e];
-                if (g.splits > 1) {
-                    g.ws[((size_t)blockIdx.z * g.M + row) * g.N + col] = v;
-                    continue;
-                }
-                const size_t o = (size_t)row * g.ldc + col;
-                switch (g.epi) {
-                    case EPI_BIAS_RELU_BF16: g.out_bf[o] = __float2bfloat16_rn(fmaxf(v + g.bias[col], 0.f)); break;
-                    case EPI_BIAS_F32: g.out_f[o] = v + g.bias[col]; break;
-                    case EPI_MASK_BF16:
-                        g.out_bf[o] = __float2bfloat16_rn(__bfloat162float(g.mask[(size_t)row * g.ldm + col]) > 0.f ? v : 0.f);
-                        break;
-                    default: g.out_f[o] = v; break;
-                }
-            }
+    for (int i = 0; i < (KMAJ ? 1 : ROWS / 64); ++i)
+        asm volatile(
+            "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
+            "[%4];" ::"r"(dst + i * (SK * 128)),
+            "l"(map), "r"(KMAJ ? k0 : r0 + i * 64), "r"(KMAJ ? r0 : k0), "r"(bar)
+            : "memory");
 }
 
-// Sums the split-K partials in split order and applies the epilogue.
-__global__ void k_splitk_reduce(GemmArgs g) {
-    const size_t total = (size_t)g.M * g.N;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        float v = 0.f;
-        for (int z = 0; z < g.splits; ++z) v += g.ws[(size_t)z * total + i];
-        const int row = int(i / g.N), col = int(i % g.N);
-        const size_t o = (size_t)row * g.ldc + col;
-        switch (g.epi) {
-            case EPI_BIAS_RELU_BF16: g.out_bf[o] = __float2bfloat16_rn(fmaxf(v + g.bias[col], 0.f)); break;
-            case EPI_BIAS_F32: g.out_f[o] = v + g.bias[col]; break;
-            case EPI_MASK_BF16:
-                g.out_bf[o] = __float2bfloat16_rn(__bfloat162float(g.mask[(size_t)row * g.ldm + col]) > 0.f ? v : 0.f);
-                break;
-            default: g.out_f[o] = v; break;
+// Shared-memory descriptor of an operand at `addr` in the 128-byte swizzle:
+// groups of 8 rows (K-major) or 8 K-rows (MN-major) 1024 bytes apart; MN-major
+// the next 64 rows after SK K-rows.
+template <bool KMAJ>
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+    const uint64_t lead = KMAJ ? 1 : (SK * 128) >> 4;
+    return uint64_t((addr >> 4) & 0x3fff) | (lead << 16) | (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) |
+           (uint64_t(2) << 61);
+}
+
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
+    for (int i = 0; i < GEMM_WAIT_MAX; ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// 8 floats of a rank's shared memory, added to v.
+__device__ __forceinline__ void add_rank8(uint32_t addr, int rank, float (&v)[8]) {
+    uint32_t a;
+    float w[8];
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3])
+                 : "r"(a)
+                 : "memory");
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(w[4]), "=f"(w[5]), "=f"(w[6]), "=f"(w[7])
+                 : "r"(a + 16)
+                 : "memory");
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] += w[j];
+}
+
+// Arrives at `bar` when this thread's multiplications so far are done.
+__device__ __forceinline__ void mma_arrive(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// 16 columns of this warp's 32 rows of tensor memory.
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+          "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+        : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+template <int TN, bool AK, bool BKM>
+__global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGroup<AK, BKM> G) {
+    using L = GTile<TN>;
+    const int S = G.stages;
+    constexpr int GROUPS = TN / 8;                 // 8-column groups of a row
+    constexpr int SUMS = 128 * GROUPS / 2 / 256;   // groups that a thread adds, for two ranks
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ uint32_t tmem_at;
+    __shared__ __align__(8) unsigned long long bars[2 * STAGES_MAX + 1];  // stage full, stage free, round multiplied
+    pdl_release();
+    const uint32_t sb = (static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + 1023u) & ~1023u;
+    const uint32_t full = static_cast<uint32_t>(__cvta_generic_to_shared(bars)), free = full + 8 * STAGES_MAX,
+                   all = free + 8 * STAGES_MAX;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(&tmem_at))),
+                     "r"(G.tmem)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    } else if (tid == 32) {
+        for (int i = 0; i <= 2 * STAGES_MAX; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + i * 8) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const int tile = blockIdx.x >> G.rank_bits, ranks = 1 << G.rank_bits, rank = blockIdx.x & (ranks - 1);
+    int p = 0;
+    while (p + 1 < G.count && tile >= G.first[p + 1]) ++p;
+    const GemmOne& o = G.g[p];
+    const GemmArgs& g = o.g;
+    const int tn = (g.N + TN - 1) / TN, t = tile - G.first[p];
+    const int m0 = (t / tn) * 128, n0 = (t % tn) * TN;
+    const bool split = G.rank_bits > 0 && g.splits > 1;  // over the ranks
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_at;
+    // BF16 operands (K-major or MN-major), FP32 accumulator, 128 x TN
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (AK ? 0u : 1u << 15) | (BKM ? 0u : 1u << 16) |
+                               (uint32_t(TN / 8) << 17) | (8u << 24);
+    constexpr uint32_t step_a = AK ? 32 : 2048, step_b = BKM ? 32 : 2048;  // 16 of K
+    bool ok = true;
+    int rounds = 0;        // multiplied so far
+    int s = 0, phase = 0;  // of the loading and of the multiplying thread: the next stage, and how often all were passed
+    float sum[SUMS][8];
+#pragma unroll
+    for (int i = 0; i < SUMS; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[i][j] = 0.f;
+    pdl_wait();  // the operands come from the kernels before
+
+    for (int round = 0; round < g.splits; round += ranks * G.accs) {
+        // this CTA's splits of the round, their stages one after another
+        const int z0 = round + rank * G.accs, z1 = min(z0 + G.accs, g.splits);
+        if (tid == 32) {
+            for (int z = z0; z < z1; ++z)
+                for (int k = z * g.kps; k < min(g.K, (z + 1) * g.kps); k += SK) {
+                    if (phase > 0) ok = ok && bar_wait(free + s * 8, (phase - 1) & 1);
+                    if (!ok) break;
+                    const uint32_t at = sb + s * L::stage;
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + s * 8),
+                                 "r"(uint32_t(L::stage))
+                                 : "memory");
+                    load_operand<128, AK>(at, &o.a, m0, k, full + s * 8);
+                    load_operand<TN, BKM>(at + L::bytes_a, &o.b, n0, k, full + s * 8);
+                    if (++s == S) s = 0, ++phase;
+                }
+            // given up: what was started still arrives before this CTA ends
+            if (!ok)
+                for (int j = 0; j < S; ++j)
+                    if (j < s || phase > 0) bar_wait(full + j * 8, (j < s ? phase : phase - 1) & 1);
+        } else if (tid == 0 && z1 > z0) {
+            for (int z = z0; z < z1; ++z) {
+                const int kbeg = z * g.kps, kend = min(g.K, kbeg + g.kps);
+                const uint32_t acc = tmem + (z - z0) * TN;
+                for (int k = kbeg; k < kend; k += SK) {
+                    ok = ok && bar_wait(full + s * 8, phase & 1);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t at = sb + s * L::stage;
+                    const uint64_t da = smem_desc<AK>(at), db = smem_desc<BKM>(at + L::bytes_a);
+                    // whole steps of BK, zero-filled past the end of K
+                    const int steps = min(SK, (kend - k + BK - 1) / BK * BK) / 16;
+#pragma unroll
+                    for (int q = 0; q < SK / 16; ++q)
+                        if (q < steps)
+                            asm volatile(
+                                "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
+                                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(acc),
+                                "l"(da + ((q * step_a) >> 4)), "l"(db + ((q * step_b) >> 4)), "r"(idesc),
+                                "r"(uint32_t(k > kbeg || q > 0))
+                                : "memory");
+                    mma_arrive(free + s * 8);
+                    if (++s == S) s = 0, ++phase;
+                }
+            }
+            mma_arrive(all);
+        }
+        __syncwarp();
+        if (z1 > z0) {
+            ok = bar_wait(all, rounds & 1) && ok;
+            ++rounds;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        __syncthreads();  // the finished tile lies where the stages were
+        if (z1 > z0) {
+            // warp w holds rows 32 (w % 4).. and half of the columns
+            const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * (TN / 2);
+            const uint32_t to = sb + uint32_t(r * L::ld + c0) * 4u;
+            const uint32_t from = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(c0);
+#pragma unroll
+            for (int c = 0; c < TN / 2; c += 16) {
+                float v[16];
+                tmem_ld16(from + c, v);
+                if (G.accs > 1 && g.splits > 1) {  // add this CTA's splits in order
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = 0.f + v[j];
+                    for (int z = 1; z < g.splits; ++z) {
+                        float w[16];
+                        tmem_ld16(from + z * TN + c, w);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] += w[j];
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j += 4)
+                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + (c + j) * 4), "f"(v[j]),
+                                 "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3])
+                                 : "memory");
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (!split) {
+            __syncthreads();
+            for (int e = tid; e < (rank == 0 ? 128 * GROUPS : 0); e += 256) {
+                const int r = e / GROUPS, c = 8 * (e % GROUPS);
+                if (m0 + r >= g.M || n0 + c >= g.N) continue;
+                float v[8];
+                const uint32_t at = sb + uint32_t(r * L::ld + c) * 4u;
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                             : "r"(at)
+                             : "memory");
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                             : "r"(at + 16)
+                             : "memory");
+                epilogue8(g, m0 + r, n0 + c, v);
+            }
+        } else {
+            cluster_arrive();
+            cluster_wait();
+            const int have = min(ranks, g.splits - round);
+            const int per = 128 >> G.rank_bits, mine = per * GROUPS;
+#pragma unroll
+            for (int i = 0; i < SUMS; ++i) {
+                const int e = tid + i * 256;
+                if (e < mine) {
+                    const uint32_t at = sb + uint32_t((rank * per + e / GROUPS) * L::ld + 8 * (e % GROUPS)) * 4u;
+#pragma unroll 4
+                    for (int q = 0; q < have; ++q) add_rank8(at, q, sum[i]);
+                }
+            }
+            // no rank leaves or fills its stages while another reads its tile
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            cluster_arrive();
+            if (round + ranks >= g.splits) {
+#pragma unroll
+                for (int i = 0; i < SUMS; ++i) {
+                    const int e = tid + i * 256;
+                    const int r = rank * per + e / GROUPS, c = 8 * (e % GROUPS);
+                    if (e < mine && m0 + r < g.M && n0 + c < g.N) epilogue8(g, m0 + r, n0 + c, sum[i]);
+                }
+            }
+            cluster_wait();
         }
     }
+    if (!ok) *G.fault = 1;
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(G.tmem));
 }
 
 // ------------------------------------------------------------ elementwise
@@ -297,6 +493,8 @@ __global__ void k_loss(int rows, int cols, const float* __restrict__ pred, const
     __shared__ float sh[32];
     const size_t total = (size_t)rows * cols;
     float s = 0.f;
+    pdl_release();
+    pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const float wc = w[i % cols];
         const float d = pred[i] - tgt[i];
@@ -307,12 +505,15 @@ __global__ void k_loss(int rows, int cols, const float* __restrict__ pred, const
     if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-__global__ void k_sum_partials(int n, const float* __restrict__ part, float mul, float* __restrict__ out, int slot) {
+// out[slot] = mul * the sum of the slot's n partials, one CTA per slot (all
+// steps of an epoch at once).
+__global__ void k_sum_partials(int n, const float* __restrict__ part, float mul, float* __restrict__ out) {
     __shared__ float sh[32];
+    const float* p = part + (size_t)blockIdx.x * n;
     float s = 0.f;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) s += p[i];
     s = block_sum_f(s, sh);
-    if (threadIdx.x == 0) out[slot] = s * mul;
+    if (threadIdx.x == 0) out[blockIdx.x] = s * mul;
 }
 
 // db[c] = sum over rows of dY[r][c] in two deterministic passes: chunk z
@@ -320,36 +521,97 @@ __global__ void k_sum_partials(int n, const float* __restrict__ part, float mul,
 // order.
 constexpr int kColChunkRows = 128;
 
-__global__ void k_colsum_part(int rows, int cols, const bf16* __restrict__ dy, float* __restrict__ part) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    const int r0 = blockIdx.y * kColChunkRows, r1 = min(rows, r0 + kColChunkRows);
+// The chunks of every layer in one launch.
+struct ColsumTable {
+    const bf16* dy[GROUP_MAX];
+    float* part[GROUP_MAX];
+    int cols[GROUP_MAX];
+    int first[GROUP_MAX + 1];  // first CTA of each layer
+    int count, rows;
+};
+// A CTA takes 64 columns of a chunk: all threads load it, then a thread per
+// column adds its 128 values in order out of shared memory.
+constexpr int kColsumCols = 64;
+__global__ void __launch_bounds__(256) k_colsum_part(const __grid_constant__ ColsumTable t) {
+    __shared__ __align__(16) bf16 sh[kColChunkRows][kColsumCols];
+    pdl_release();
+    int l = 0;
+    while (l + 1 < t.count && int(blockIdx.x) >= t.first[l + 1]) ++l;
+    const int cols = t.cols[l], cb = (cols + kColsumCols - 1) / kColsumCols, b = int(blockIdx.x) - t.first[l];
+    const int c0 = (b % cb) * kColsumCols, z = b / cb;
+    const int r0 = z * kColChunkRows, n = min(t.rows - r0, kColChunkRows);
+    pdl_wait();
+    // 8 columns (16 bytes) at a time; cols is a multiple of 8
+    for (int i = threadIdx.x; i < n * (kColsumCols / 8); i += 256) {
+        const int r = i / (kColsumCols / 8), c = 8 * (i % (kColsumCols / 8));
+        if (c0 + c < cols)
+            *reinterpret_cast<uint4*>(&sh[r][c]) =
+                *reinterpret_cast<const uint4*>(t.dy[l] + (size_t)(r0 + r) * cols + c0 + c);
+    }
+    __syncthreads();
+    const int c = threadIdx.x;
+    if (c >= kColsumCols || c0 + c >= cols) return;
     float s = 0.f;
-    for (int r = r0; r < r1; ++r) s += __bfloat162float(dy[(size_t)r * cols + c]);
-    part[(size_t)blockIdx.y * cols + c] = s;
+#pragma unroll 16
+    for (int r = 0; r < n; ++r) s += __bfloat162float(sh[r][c]);
+    t.part[l][(size_t)z * cols + c0 + c] = s;
+}
+
+__device__ __forceinline__ float colsum_total(int chunks, int cols, int c, const float* __restrict__ part) {
+    float s = 0.f;
+    for (int z = 0; z < chunks; ++z) s += part[(size_t)z * cols + c];
+    return s;
 }
 
 __global__ void k_colsum_final(int chunks, int cols, const float* __restrict__ part, float* __restrict__ db) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.f;
-    for (int z = 0; z < chunks; ++z) s += part[(size_t)z * cols + c];
-    db[c] = s;
+    if (c < cols) db[c] = colsum_total(chunks, cols, c, part);
 }
 
-__global__ void k_adam(size_t n, float* __restrict__ w, bf16* __restrict__ wb, const float* __restrict__ g,
-                       float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2, float eps, float bc1,
-                       float bc2) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float wi = w[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-        w[i] = wi;
-        if (wb) wb[i] = __float2bfloat16_rn(wi);
+// Adam over the weights and biases of every layer in one launch, one element
+// per thread; a bias' gradient is added up from its chunks here.
+struct AdamTable {
+    struct Layer {
+        float *w, *gw, *mw, *vw, *b, *gb, *mb, *vb;
+        bf16* wb;
+        const float* part;
+        int nw, nb;
+    } l[GROUP_MAX];
+    int first[GROUP_MAX + 1];  // first CTA of each layer
+    int count, chunks;
+    const float2* bc;  // the step's bias corrections
+    float lr, b1, b2, eps;
+};
+__global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamTable t) {
+    pdl_release();
+    int l = 0;
+    while (l + 1 < t.count && int(blockIdx.x) >= t.first[l + 1]) ++l;
+    const AdamTable::Layer& y = t.l[l];
+    const int i = (int(blockIdx.x) - t.first[l]) * 256 + int(threadIdx.x);
+    pdl_wait();
+    if (i >= y.nw + y.nb) return;
+    const bool weight = i < y.nw;
+    const int j = weight ? i : i - y.nw;
+    float* m = weight ? y.mw : y.mb;
+    float* v = weight ? y.vw : y.vb;
+    float* w = weight ? y.w : y.b;
+    float gi;
+    if (weight) {
+        gi = y.gw[j];
+    } else {
+        gi = colsum_total(t.chunks, y.nb, j, y.part);
+        y.gb[j] = gi;
     }
+    // the roundings are spelled out, so that they do not depend on what the
+    // compiler contracts here
+    const float mi = __fmaf_rn(1.f - t.b1, gi, __fmul_rn(t.b1, m[j]));
+    const float vi = __fmaf_rn(__fmul_rn(1.f - t.b2, gi), gi, __fmul_rn(t.b2, v[j]));
+    m[j] = mi;
+    v[j] = vi;
+    const float2 bc = __ldg(t.bc);
+    const float wi = w[j] - t.lr * (mi / bc.x) / (sqrtf(vi / bc.y) + t.eps);
+    w[j] = wi;
+    if (weight) y.wb[j] = __float2bfloat16_rn(wi);
 }
 
 // Uniform(-a, a) from a counter hash (splitmix64) of (seed, index).
@@ -375,6 +637,47 @@ unsigned grid1d(size_t n, int cap = 148 * 16) {
 
 // ------------------------------------------------------------ the handle
 
+namespace {
+// Flags in mapped host memory that a kernel sets when one of its waits gives
+// up: the host reads them after a synchronisation at no cost.  A page of them
+// serves the handles of the process, taken on the first use and kept (a
+// pinned allocation for each handle took 2.5 ms of the 4.4 its creation did);
+// handles beyond the page's flags have their own.
+struct FaultFlags {
+    static constexpr int kFlags = 1024;
+    std::mutex mu;
+    int* page = nullptr;
+    std::vector<int*> spare;
+
+    static int* allocate(int n) {
+        int* p = nullptr;
+        MLP_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), n * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+        return p;
+    }
+    int* take() {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!page) {
+            spare.reserve(kFlags);
+            page = allocate(kFlags);
+            for (int i = 0; i < kFlags; ++i) spare.push_back(page + i);
+        }
+        int* f = spare.empty() ? allocate(1) : spare.back();
+        if (!spare.empty()) spare.pop_back();
+        *f = 0;
+        return f;
+    }
+    void give(int* f) {
+        std::lock_guard<std::mutex> lock(mu);
+        if (f >= page && f < page + kFlags) spare.push_back(f);
+        else cudaFreeHost(f);
+    }
+};
+FaultFlags& fault_flags() {
+    static FaultFlags* flags = new FaultFlags;  // outlives every handle
+    return *flags;
+}
+}  // namespace
+
 struct nir_mlp {
     nir_mlp_config cfg{};
     int device = 0;
@@ -397,12 +700,16 @@ struct nir_mlp {
     float* pred = nullptr;
     float* tgt = nullptr;
     bf16* dy = nullptr;
-    bf16 *g0 = nullptr, *g1 = nullptr;  // hidden-size gradient ping-pong
-    float* ws = nullptr;
-    size_t ws_len = 0;
-    float* colsum_ws = nullptr;
-    size_t colsum_len = 0;
-    float* part = nullptr;
+    std::vector<bf16*> grad;            // masked gradients at the hidden outputs
+    bf16* ep_x = nullptr;               // the epoch's samples in its order
+    float* ep_y = nullptr;
+    int ep_len = 0;
+    float2* bc = nullptr;               // Adam's bias corrections of the epoch's steps
+    int bc_len = 0;
+    int cap_back = 0;
+    float* colsum_ws = nullptr;  // every layer's chunks, one after another
+    float* part = nullptr;       // loss partials, loss_blocks() per step
+    size_t part_len = 0;
     float* losses = nullptr;  // device loss per step
     int losses_len = 0;
     // training set
@@ -415,6 +722,8 @@ struct nir_mlp {
     float* stage = nullptr;  // FP32 staging of uploaded rows, grown on demand
     size_t stage_len = 0;
     // output map of nir_mlp_predict_device_affine
+    bool gemm_ready[8] = {};  // GEMM kernels prepared for launches
+    int* fault = nullptr;     // mapped host memory, set if a wait inside a GEMM gives up
     int aff_n = 0, aff_col = 0;
     double aff_lo = 0.0, aff_hi = 0.0;
     double *aff_scale = nullptr, *aff_shift = nullptr, *aff_out = nullptr;
@@ -438,6 +747,7 @@ struct nir_mlp {
     ~nir_mlp() {
         cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
+        if (fault) fault_flags().give(fault);
         for (void* p : allocs)
             if (p) cudaFree(p);
         if (stream) cudaStreamDestroy(stream);
@@ -450,10 +760,12 @@ void check_mult8(int v, const char* what) {
     if (v <= 0 || v % 8 != 0) throw std::invalid_argument(std::string(what) + " must be a positive multiple of 8");
 }
 
-// C = op(A) op(B)^T with the given storage (see the file header).
-void gemm(nir_mlp* h, bool a_kmaj, bool b_kmaj, const bf16* A, int lda, const bf16* B, int ldb, int M, int N, int K,
-          int epi, const float* bias, bf16* out_bf, float* out_f, int ldc, const bf16* mask, int ldm) {
-    if (M <= 0 || N <= 0) return;
+// Arguments of C = op(A) op(B)^T with the given storage (see the file
+// header): the splits of K depend on the sizes alone, so the order of the
+// sums does not depend on the kernel that takes the product.
+GemmArgs gemm_args(const nir_mlp* h, bool a_kmaj, bool b_kmaj, const bf16* A, int lda, const bf16* B, int ldb, int M,
+                   int N, int K, int epi, const float* bias, bf16* out_bf, float* out_f, int ldc, const bf16* mask,
+                   int ldm) {
     if (K % 8 != 0 || (!a_kmaj && M % 8 != 0) || (!b_kmaj && N % 8 != 0) || lda % 8 != 0 || ldb % 8 != 0)
         throw std::invalid_argument("gemm: contiguous extents must be multiples of 8");
     GemmArgs g{};
@@ -471,6 +783,8 @@ void gemm(nir_mlp* h, bool a_kmaj, bool b_kmaj, const bf16* A, int lda, const bf
     g.ldc = ldc;
     g.mask = mask;
     g.ldm = ldm;
+    auto aligned = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
+    g.wide = (N | ldc | ldm) % 8 == 0 && aligned(bias) && aligned(out_bf) && aligned(out_f) && aligned(mask);
     const int tm = (M + BM - 1) / BM, tn = (N + BN - 1) / BN;
     const int KT = (K + BK - 1) / BK;
     int splits = 1;
@@ -478,52 +792,199 @@ void gemm(nir_mlp* h, bool a_kmaj, bool b_kmaj, const bf16* A, int lda, const bf
     if (tm * tn < want && KT >= 16) splits = std::min(KT / 8, (want + tm * tn - 1) / (tm * tn));
     splits = std::max(splits, 1);
     g.kps = ((KT + splits - 1) / splits) * BK;
-    splits = (K + g.kps - 1) / g.kps;
-    g.splits = splits;
-    if (splits > 1) {
-        const size_t need = (size_t)splits * M * N;
-        if (need > h->ws_len) {
-            h->release(h->ws);
-            h->ws = h->alloc<float>(need);
-            h->ws_len = need;
-        }
-        g.ws = h->ws;
+    g.splits = (K + g.kps - 1) / g.kps;
+    return g;
+}
+
+template <typename... P, typename... A>
+void launch_early(nir_mlp* h, void (*k)(P...), dim3 grid, int threads, size_t smem, int cluster, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = unsigned(cluster);
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    MLP_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...));
+}
+
+// The tensor map of an operand of `rows` rows for stages of `tile` of them.
+CUtensorMap operand_map(const bf16* P, int ld, int rows, int K, bool kmaj, int tile) {
+    static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        MLP_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q));
+        if (!f) throw std::runtime_error("the driver has no cuTensorMapEncodeTiled");
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
+    }();
+    CUtensorMap m;
+    const cuuint64_t dims[2] = {cuuint64_t(kmaj ? K : rows), cuuint64_t(kmaj ? rows : K)};
+    // (the stride of a single row is not used, but checked)
+    const cuuint64_t strides[1] = {dims[1] > 1 ? cuuint64_t(ld) * sizeof(bf16) : (dims[0] + 7) / 8 * 16};
+    const cuuint32_t box[2] = {64, cuuint32_t(kmaj ? tile : SK)}, one[2] = {1, 1};
+    if (encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(P), dims, strides, box, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        throw std::invalid_argument("an operand's rows must start at multiples of 16 bytes");
+    return m;
+}
+
+// How a launch is cut: 128 x tn tiles, 2^bits CTAs each.
+struct GemmPlan {
+    double time = 1e300;
+    int tn = 64, bits = 0, stages = 0;
+    uint32_t tmem = 0;
+};
+// Estimated time (us) of a group, from runs over M 128..65536, N 16..8192 and
+// K 64..52000.  A CTA's start, first load and epilogue take 4 (tn = 64) or 5
+// us, a stage of 64 of K 0.4 us with 64 columns; with 128 it takes 0.36 us,
+// and 0.5 where two CTAs share an SM.  Splits that one CTA takes one after
+// another cost nothing more (1024 x 512 x 512 in two splits: 6.7 us), but
+// more CTAs share the stages (512 x 512 x 1024 in four: 9.7 us by one CTA a
+// tile, 7.5 by four).  An exchange between the CTAs of a cluster takes 1.5 to
+// 2.5 us with an SM for each, 5 to 8 where they share SMs, and the round
+// after it loads anew.  Two CTAs fit on an SM unless their tensor memory or
+// their stages do not; clusters of 16 fill about half of the SMs, and those
+// of 8 and more find an SM for each CTA only while half of the SMs do.
+GemmPlan gemm_plan(const nir_mlp* h, const GemmArgs* gs, int count, int splits, int tn, int bits) {
+    const int ranks = 1 << bits;
+    long long ctas = 0;
+    for (int i = 0; i < count; ++i) ctas += (long long)((gs[i].M + 127) / 128) * ((gs[i].N + tn - 1) / tn) * ranks;
+    GemmPlan p;
+    p.tn = tn;
+    p.bits = bits;
+    p.tmem = tn;
+    while (bits == 0 && p.tmem < uint32_t(tn * splits)) p.tmem *= 2;
+    const int slots = bits == RANK_BITS_MAX || 2 * p.tmem > TMEM_COLUMNS ? h->sms : 2 * h->sms;
+    // one CTA to an SM, with all of its memory
+    const bool alone = ctas <= (bits >= 3 ? h->sms / 2 : h->sms) || 2 * p.tmem > TMEM_COLUMNS;
+    p.stages = alone ? 6 : tn == 64 ? 4 : 3;
+    const double there = double(std::min<long long>(ctas, slots));
+    const double stage = tn == 64 ? 0.4 : alone ? 0.36 : 0.5;
+    const double swap = alone ? (tn == 64 ? 0.8 + 0.3 * bits + 0.004 * there : 1.5 + 0.6 * bits + 0.005 * there)
+                              : (tn == 64 ? 2.3 + 0.5 * bits + 0.012 * there : 3.0 + 1.5 * bits + 0.03 * there);
+    const double again = !alone ? 0.0 : tn == 64 ? 1.0 : 1.8;
+    double longest = 0.0;
+    for (int i = 0; i < count; ++i) {
+        const double split = (std::min(gs[i].kps, gs[i].K) + SK - 1) / SK * stage;
+        const int rounds = (gs[i].splits + ranks - 1) / ranks;
+        longest = std::max(longest, bits ? rounds * (split + swap) + (rounds - 1) * again : gs[i].splits * split);
     }
-    dim3 grid(tn, tm, splits);
-    auto launch = [&](auto kern) {
-        MLP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        kern<<<grid, THREADS, SMEM_BYTES, h->stream>>>(g);
-    };
-    if (a_kmaj && b_kmaj) launch(k_gemm<true, true>);
-    else if (a_kmaj && !b_kmaj) launch(k_gemm<true, false>);
-    else if (!a_kmaj && !b_kmaj) launch(k_gemm<false, false>);
-    else launch(k_gemm<false, true>);
+    p.time = double((ctas + slots - 1) / slots) * ((tn == 64 ? 4.0 : 5.0) + longest);
+    return p;
+}
+
+// Once per handle and kernel that it uses: what a launch may ask for.
+template <int TN, bool AK, bool BKM>
+void prepare_gemm(nir_mlp* h) {
+    bool& ready = h->gemm_ready[(TN == 128) * 4 + AK * 2 + BKM];
+    if (ready) return;
+    MLP_CUDA(cudaFuncSetAttribute(k_gemm<TN, AK, BKM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  GTile<TN>::smem(STAGES_MAX)));
+    MLP_CUDA(cudaFuncSetAttribute(k_gemm<TN, AK, BKM>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    ready = true;
+}
+
+template <int TN, bool AK, bool BKM>
+void launch_tiles(nir_mlp* h, const GemmArgs* gs, int count, int splits, const GemmPlan& plan) {
+    prepare_gemm<TN, AK, BKM>(h);
+    GemmGroup<AK, BKM> G{};
+    int tiles = 0;
+    for (int i = 0; i < count; ++i) {
+        G.g[i].g = gs[i];
+        G.g[i].a = operand_map(gs[i].A, gs[i].lda, gs[i].M, gs[i].K, AK, 128);
+        G.g[i].b = operand_map(gs[i].B, gs[i].ldb, gs[i].N, gs[i].K, BKM, TN);
+        G.first[i] = tiles;
+        tiles += ((gs[i].M + 127) / 128) * ((gs[i].N + TN - 1) / TN);
+    }
+    G.first[count] = tiles;
+    G.count = count;
+    G.fault = h->fault;
+    G.rank_bits = plan.bits;
+    G.accs = plan.bits ? 1 : splits;
+    G.tmem = plan.tmem;
+    G.stages = plan.stages;
+    launch_early(h, k_gemm<TN, AK, BKM>, dim3(unsigned(tiles) << G.rank_bits), GTile<TN>::threads,
+                 GTile<TN>::smem(G.stages), 1 << G.rank_bits, G);
     MLP_LAUNCHED();
-    if (splits > 1) {
-        k_splitk_reduce<<<grid1d((size_t)M * N), 256, 0, h->stream>>>(g);
-        MLP_LAUNCHED();
+}
+
+// Independent products of one storage kind in one launch.
+template <bool AK, bool BKM>
+void launch_gemm(nir_mlp* h, const GemmArgs* gs, int count) {
+    int splits = 1;
+    for (int i = 0; i < count; ++i) splits = std::max(splits, gs[i].splits);
+    GemmPlan best;
+    for (int tn : {64, 128})
+        for (int bits = splits * tn > TMEM_COLUMNS; bits == 0 || (bits <= RANK_BITS_MAX && (1 << bits) < 2 * splits);
+             ++bits) {
+            const GemmPlan p = gemm_plan(h, gs, count, splits, tn, bits);
+            if (p.time < best.time) best = p;
+        }
+    if (best.tn == 64) launch_tiles<64, AK, BKM>(h, gs, count, splits, best);
+    else launch_tiles<128, AK, BKM>(h, gs, count, splits, best);
+}
+
+void gemm(nir_mlp* h, bool a_kmaj, bool b_kmaj, const bf16* A, int lda, const bf16* B, int ldb, int M, int N, int K,
+          int epi, const float* bias, bf16* out_bf, float* out_f, int ldc, const bf16* mask, int ldm) {
+    if (M <= 0 || N <= 0) return;
+    const GemmArgs g =
+        gemm_args(h, a_kmaj, b_kmaj, A, lda, B, ldb, M, N, K, epi, bias, out_bf, out_f, ldc, mask, ldm);
+    if (a_kmaj && b_kmaj) launch_gemm<true, true>(h, &g, 1);
+    else if (a_kmaj && !b_kmaj) launch_gemm<true, false>(h, &g, 1);
+    else if (!a_kmaj && !b_kmaj) launch_gemm<false, false>(h, &g, 1);
+    else launch_gemm<false, true>(h, &g, 1);
+}
+
+// Waits for the stream; an error if a kernel could not finish its work.
+void finish(nir_mlp* h) {
+    MLP_CUDA(cudaStreamSynchronize(h->stream));
+    if (h->fault && *reinterpret_cast<volatile int*>(h->fault)) {
+        *h->fault = 0;
+        throw std::runtime_error("a wait inside a GEMM kernel gave up");
     }
 }
 
 void ensure_rows(nir_mlp* h, int rows) {
     if (rows <= h->cap_rows) return;
     for (bf16* p : h->act) h->release(p);
-    for (void* p : {(void*)h->x, (void*)h->pred, (void*)h->tgt, (void*)h->dy, (void*)h->g0, (void*)h->g1})
+    for (void* p : {(void*)h->x, (void*)h->pred})
         if (p) h->release(p);
-    const int din = h->cfg.d_in, dout = h->cfg.d_out, wmax = h->cfg.width;
+    const int din = h->cfg.d_in, dout = h->cfg.d_out;
     h->x = h->alloc<bf16>((size_t)rows * din);
     h->act.assign(h->cfg.depth, nullptr);
     for (auto& a : h->act) a = h->alloc<bf16>((size_t)rows * h->cfg.width);
     h->pred = h->alloc<float>((size_t)rows * dout);
-    h->tgt = h->alloc<float>((size_t)rows * dout);
-    h->dy = h->alloc<bf16>((size_t)rows * dout);
-    h->g0 = h->alloc<bf16>((size_t)rows * wmax);
-    h->g1 = h->alloc<bf16>((size_t)rows * wmax);
     h->cap_rows = rows;
 }
 
-void forward(nir_mlp* h, int rows) {
-    const bf16* in = h->x;
+// The buffers of a backward pass over `rows` samples (a forward pass alone
+// needs none of them).
+void ensure_backward(nir_mlp* h, int rows) {
+    if (rows <= h->cap_back) return;
+    for (bf16* p : h->grad) h->release(p);
+    for (void* p : {(void*)h->tgt, (void*)h->dy, (void*)h->colsum_ws, (void*)h->part})
+        if (p) h->release(p);
+    const int dout = h->cfg.d_out;
+    h->tgt = h->alloc<float>((size_t)rows * dout);
+    h->dy = h->alloc<bf16>((size_t)rows * dout);
+    h->grad.assign(h->cfg.depth, nullptr);
+    for (auto& g : h->grad) g = h->alloc<bf16>((size_t)rows * h->cfg.width);
+    size_t cols = 0;
+    for (auto& ly : h->layers) cols += (size_t)ly.out;
+    h->colsum_ws = h->alloc<float>((size_t)((rows + kColChunkRows - 1) / kColChunkRows) * cols);
+    h->part = nullptr;
+    h->part_len = 0;
+    h->cap_back = rows;
+}
+
+void forward(nir_mlp* h, int rows, const bf16* in) {
     const int L = int(h->layers.size());
     for (int l = 0; l < L; ++l) {
         auto& ly = h->layers[l];
@@ -538,55 +999,86 @@ void forward(nir_mlp* h, int rows) {
     }
 }
 
-// Loss (device slot) and dY, then every layer's gradients.
-void backward(nir_mlp* h, int rows, int loss_slot) {
-    const int dout = h->cfg.d_out;
-    const float denom = float(rows) * std::max(h->outw_sum, 1.f);
-    const unsigned gb = grid1d((size_t)rows * dout, 1024);
-    k_loss<<<gb, 256, 0, h->stream>>>(rows, dout, h->pred, h->tgt, h->outw, 2.f / denom, h->dy, h->part);
-    k_sum_partials<<<1, 256, 0, h->stream>>>(int(gb), h->part, 1.f / denom, h->losses, loss_slot);
-    MLP_LAUNCHED();
-    const int L = int(h->layers.size());
-    const bf16* g = h->dy;
-    for (int l = L - 1; l >= 0; --l) {
-        auto& ly = h->layers[l];
-        const bf16* in = (l == 0) ? h->x : h->act[l - 1];
-        // dW = g^T in   (out x in), contraction over the rows
-        gemm(h, false, false, g, ly.out, in, ly.in, ly.out, ly.in, rows, EPI_F32, nullptr, nullptr, ly.gW, ly.in,
-             nullptr, 0);
-        {
-            const int chunks = (rows + kColChunkRows - 1) / kColChunkRows;
-            const size_t need = (size_t)chunks * ly.out;
-            if (need > h->colsum_len) {
-                h->release(h->colsum_ws);
-                h->colsum_ws = h->alloc<float>(need);
-                h->colsum_len = need;
-            }
-            k_colsum_part<<<dim3((ly.out + 255) / 256, chunks), 256, 0, h->stream>>>(rows, ly.out, g, h->colsum_ws);
-            k_colsum_final<<<(ly.out + 255) / 256, 256, 0, h->stream>>>(chunks, ly.out, h->colsum_ws, ly.gb);
-            MLP_LAUNCHED();
-        }
-        if (l > 0) {
-            bf16* gn = (g == h->g0) ? h->g1 : h->g0;
-            // d(in) = g W, masked by the ReLU of the layer below
-            gemm(h, true, false, g, ly.out, ly.Wb, ly.in, rows, ly.in, ly.out, EPI_MASK_BF16, nullptr, gn, nullptr,
-                 ly.in, h->act[l - 1], ly.in);
-            g = gn;
-        }
-    }
+unsigned loss_blocks(const nir_mlp* h, int rows) { return grid1d((size_t)rows * h->cfg.d_out, 1024); }
+
+void ensure_parts(nir_mlp* h, size_t len) {
+    if (len <= h->part_len) return;
+    if (h->part) h->release(h->part);
+    h->part = h->alloc<float>(len);
+    h->part_len = len;
 }
 
-void adam(nir_mlp* h) {
-    h->adam_t += 1;
-    const float b1 = h->cfg.beta1, b2 = h->cfg.beta2;
-    const float bc1 = 1.f - std::pow(b1, float(h->adam_t)), bc2 = 1.f - std::pow(b2, float(h->adam_t));
-    for (auto& ly : h->layers) {
-        const size_t nw = (size_t)ly.in * ly.out;
-        k_adam<<<grid1d(nw), 256, 0, h->stream>>>(nw, ly.W, ly.Wb, ly.gW, ly.mW, ly.vW, h->cfg.lr, b1, b2, h->cfg.eps,
-                                                   bc1, bc2);
-        k_adam<<<grid1d(ly.out), 256, 0, h->stream>>>(ly.out, ly.b, nullptr, ly.gb, ly.mb, ly.vb, h->cfg.lr, b1, b2,
-                                                       h->cfg.eps, bc1, bc2);
+// The losses of `steps` steps of `rows` samples from their partials.
+void finish_losses(nir_mlp* h, int rows, int steps) {
+    const float denom = float(rows) * std::max(h->outw_sum, 1.f);
+    k_sum_partials<<<unsigned(steps), 256, 0, h->stream>>>(int(loss_blocks(h, rows)), h->part, 1.f / denom, h->losses);
+    MLP_LAUNCHED();
+}
+
+// The column sums of every layer's output gradient, chunk by chunk.
+int colsum_chunks(int rows) { return (rows + kColChunkRows - 1) / kColChunkRows; }
+float* colsum_of(nir_mlp* h, int rows, int l) {
+    size_t o = 0;
+    for (int k = 0; k < l; ++k) o += (size_t)h->layers[k].out;
+    return h->colsum_ws + o * (size_t)colsum_chunks(rows);
+}
+
+// Loss partials (of step `slot`) and dY, the gradients down the layers, then
+// every layer's weight gradient in one launch and every bias' column sums in
+// another: they depend on nothing after them, and a step's launches, not its
+// arithmetic, are what it spends its time on (1024 samples of 16 -> 3 x 512
+// -> 8: 258 us with 40 launches, 68 us with 11).
+void backward(nir_mlp* h, int rows, const bf16* x, const float* tgt, int slot) {
+    const int dout = h->cfg.d_out;
+    const float denom = float(rows) * std::max(h->outw_sum, 1.f);
+    const unsigned gb = loss_blocks(h, rows);
+    launch_early(h, k_loss, dim3(gb), 256, 0, 1, rows, dout, (const float*)h->pred, tgt, (const float*)h->outw,
+                 2.f / denom, h->dy, h->part + (size_t)slot * gb);
+    const int L = int(h->layers.size());
+    auto grad_of = [&](int l) { return l == L - 1 ? h->dy : h->grad[l]; };
+    for (int l = L - 1; l > 0; --l) {
+        auto& ly = h->layers[l];
+        // d(in) = g W, masked by the ReLU of the layer below
+        gemm(h, true, false, grad_of(l), ly.out, ly.Wb, ly.in, rows, ly.in, ly.out, EPI_MASK_BF16, nullptr, h->grad[l - 1],
+             nullptr, ly.in, h->act[l - 1], ly.in);
     }
+    GemmArgs gs[GROUP_MAX];
+    ColsumTable ct{};
+    for (int l = 0; l < L; ++l) {
+        auto& ly = h->layers[l];
+        const bf16* in = (l == 0) ? x : h->act[l - 1];
+        // dW = g^T in   (out x in), contraction over the rows
+        gs[l] = gemm_args(h, false, false, grad_of(l), ly.out, in, ly.in, ly.out, ly.in, rows, EPI_F32, nullptr, nullptr,
+                          ly.gW, ly.in, nullptr, 0);
+        ct.dy[l] = grad_of(l);
+        ct.part[l] = colsum_of(h, rows, l);
+        ct.cols[l] = ly.out;
+        ct.first[l + 1] = ct.first[l] + colsum_chunks(rows) * ((ly.out + kColsumCols - 1) / kColsumCols);
+    }
+    launch_gemm<false, false>(h, gs, L);
+    ct.count = L;
+    ct.rows = rows;
+    launch_early(h, k_colsum_part, dim3(unsigned(ct.first[L])), 256, 0, 1, ct);
+    MLP_LAUNCHED();
+}
+
+void adam(nir_mlp* h, int rows, int slot) {
+    AdamTable t{};
+    const int L = int(h->layers.size());
+    for (int l = 0; l < L; ++l) {
+        auto& y = h->layers[l];
+        const int nw = y.in * y.out;
+        t.l[l] = AdamTable::Layer{y.W, y.gW, y.mW, y.vW, y.b, y.gb, y.mb, y.vb, y.Wb, colsum_of(h, rows, l), nw, y.out};
+        t.first[l + 1] = t.first[l] + (nw + y.out + 255) / 256;
+    }
+    t.count = L;
+    t.chunks = colsum_chunks(rows);
+    t.bc = h->bc + slot;
+    t.lr = h->cfg.lr;
+    t.b1 = h->cfg.beta1;
+    t.b2 = h->cfg.beta2;
+    t.eps = h->cfg.eps;
+    launch_early(h, k_adam, dim3(unsigned(t.first[L])), 256, 0, 1, t);
     MLP_LAUNCHED();
 }
 
@@ -609,7 +1101,7 @@ void upload_rows(nir_mlp* h, const float* x, int rows, bf16* dst, int cols) {
     MLP_CUDA(cudaMemcpyAsync(h->stage, x, len * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     k_to_bf16<<<grid1d(len), 256, 0, h->stream>>>(len, h->stage, dst);
     MLP_LAUNCHED();
-    MLP_CUDA(cudaStreamSynchronize(h->stream));
+    finish(h);
 }
 
 int fail(const std::exception& e, bool input) {
@@ -664,13 +1156,13 @@ int nir_mlp_create(const nir_mlp_config* cfg, int device, nir_mlp** out) {
             MLP_LAUNCHED();
             h->layers.push_back(ly);
         }
+        h->fault = fault_flags().take();
         h->outw = h->alloc<float>(cfg->d_out);
         std::vector<float> ones(cfg->d_out, 1.f);
         MLP_CUDA(cudaMemcpyAsync(h->outw, ones.data(), ones.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
         h->outw_sum = float(cfg->d_out);
-        h->part = h->alloc<float>(1024);
         ensure_losses(h.get(), 1024);
-        MLP_CUDA(cudaStreamSynchronize(h->stream));
+        finish(h.get());
     } catch (const std::invalid_argument& e) {
         return fail(e, true);
     } catch (const std::exception& e) {
@@ -701,7 +1193,7 @@ int nir_mlp_get_params(nir_mlp* h, float* out) {
             MLP_CUDA(cudaMemcpyAsync(out + o, ly.b, ly.out * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
             o += ly.out;
         }
-        MLP_CUDA(cudaStreamSynchronize(h->stream));
+        finish(h);
     } catch (const std::exception& e) {
         return fail(e, false);
     }
@@ -727,7 +1219,7 @@ int nir_mlp_set_params(nir_mlp* h, const float* in) {
             MLP_CUDA(cudaMemsetAsync(ly.vb, 0, ly.out * sizeof(float), h->stream));
         }
         h->adam_t = 0;
-        MLP_CUDA(cudaStreamSynchronize(h->stream));
+        finish(h);
     } catch (const std::exception& e) {
         return fail(e, false);
     }
@@ -744,7 +1236,7 @@ int nir_mlp_set_output_weights(nir_mlp* h, const float* w) {
             s += w[i];
         }
         MLP_CUDA(cudaMemcpyAsync(h->outw, w, h->cfg.d_out * sizeof(float), cudaMemcpyHostToDevice, h->stream));
-        MLP_CUDA(cudaStreamSynchronize(h->stream));
+        finish(h);
         h->outw_sum = float(s);
     } catch (const std::invalid_argument& e) {
         return fail(e, true);
@@ -776,7 +1268,7 @@ int nir_mlp_set_data(nir_mlp* h, const float* x, const float* targets, int32_t n
         }
         MLP_CUDA(cudaMemcpyAsync(h->data_y, targets, (size_t)n * dout * sizeof(float), cudaMemcpyHostToDevice,
                                  h->stream));
-        MLP_CUDA(cudaStreamSynchronize(h->stream));
+        finish(h);
         h->n_data = n;
     } catch (const std::exception& e) {
         return fail(e, false);
@@ -796,11 +1288,26 @@ int nir_mlp_train(nir_mlp* h, int32_t epochs, int32_t batch, float* epoch_loss) 
     try {
         MLP_CUDA(cudaSetDevice(h->device));
         ensure_rows(h, batch);
-        const int steps = h->n_data / batch;
+        ensure_backward(h, batch);
+        const int steps = h->n_data / batch, used = steps * batch;
         ensure_losses(h, steps);
+        ensure_parts(h, (size_t)steps * loss_blocks(h, batch));
+        if (used > h->ep_len) {
+            h->release(h->ep_x);
+            h->release(h->ep_y);
+            h->ep_x = h->alloc<bf16>((size_t)used * h->cfg.d_in);
+            h->ep_y = h->alloc<float>((size_t)used * h->cfg.d_out);
+            h->ep_len = used;
+        }
         std::mt19937_64 rng(h->cfg.seed ^ 0x5bd1e995ULL ^ (uint64_t)h->adam_t);
         std::vector<int> perm(h->n_data);
         std::vector<float> lossv(steps);
+        std::vector<float2> bcv(steps);
+        if (steps > h->bc_len) {
+            if (h->bc) h->release(h->bc);
+            h->bc = h->alloc<float2>(steps);
+            h->bc_len = steps;
+        }
         cudaEvent_t e0, e1;
         MLP_CUDA(cudaEventCreate(&e0));
         MLP_CUDA(cudaEventCreate(&e1));
@@ -812,21 +1319,29 @@ int nir_mlp_train(nir_mlp* h, int32_t epochs, int32_t batch, float* epoch_loss) 
             MLP_CUDA(cudaMemcpyAsync(h->perm, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice,
                                      h->stream));
             MLP_CUDA(cudaEventRecord(e0, h->stream));
+            // the epoch's samples in its order, at once
+            k_gather_rows<bf16><<<grid1d((size_t)used * h->cfg.d_in), 256, 0, h->stream>>>(h->perm, used, h->cfg.d_in,
+                                                                                           h->data_x, h->ep_x);
+            k_gather_rows<float><<<grid1d((size_t)used * h->cfg.d_out), 256, 0, h->stream>>>(h->perm, used, h->cfg.d_out,
+                                                                                             h->data_y, h->ep_y);
+            MLP_LAUNCHED();
             for (int s = 0; s < steps; ++s) {
-                const int* idx = h->perm + (size_t)s * batch;
-                k_gather_rows<bf16><<<grid1d((size_t)batch * h->cfg.d_in), 256, 0, h->stream>>>(
-                    idx, batch, h->cfg.d_in, h->data_x, h->x);
-                k_gather_rows<float><<<grid1d((size_t)batch * h->cfg.d_out), 256, 0, h->stream>>>(
-                    idx, batch, h->cfg.d_out, h->data_y, h->tgt);
-                MLP_LAUNCHED();
-                forward(h, batch);
-                backward(h, batch, s);
-                adam(h);
+                h->adam_t += 1;
+                bcv[size_t(s)] = make_float2(1.f - std::pow(h->cfg.beta1, float(h->adam_t)),
+                                             1.f - std::pow(h->cfg.beta2, float(h->adam_t)));
             }
+            MLP_CUDA(cudaMemcpyAsync(h->bc, bcv.data(), bcv.size() * sizeof(float2), cudaMemcpyHostToDevice, h->stream));
+            for (int s = 0; s < steps; ++s) {
+                const bf16* x = h->ep_x + (size_t)s * batch * h->cfg.d_in;
+                forward(h, batch, x);
+                backward(h, batch, x, h->ep_y + (size_t)s * batch * h->cfg.d_out, s);
+                adam(h, batch, s);
+            }
+            finish_losses(h, batch, steps);
             MLP_CUDA(cudaEventRecord(e1, h->stream));
             MLP_CUDA(cudaMemcpyAsync(lossv.data(), h->losses, steps * sizeof(float), cudaMemcpyDeviceToHost,
                                      h->stream));
-            MLP_CUDA(cudaStreamSynchronize(h->stream));
+            finish(h);
             float ms = 0.f;
             MLP_CUDA(cudaEventElapsedTime(&ms, e0, e1));
             total_ms += ms;
@@ -864,10 +1379,10 @@ int nir_mlp_predict(nir_mlp* h, const float* x, int32_t n, float* y) {
         for (int r = 0; r < n; r += chunk) {
             const int k = std::min(chunk, n - r);  // a multiple of 8
             upload_rows(h, x + (size_t)r * h->cfg.d_in, k, h->x, h->cfg.d_in);
-            forward(h, k);
+            forward(h, k, h->x);
             MLP_CUDA(cudaMemcpyAsync(y + (size_t)r * h->cfg.d_out, h->pred, (size_t)k * h->cfg.d_out * sizeof(float),
                                      cudaMemcpyDeviceToHost, h->stream));
-            MLP_CUDA(cudaStreamSynchronize(h->stream));
+            finish(h);
         }
     } catch (const std::exception& e) {
         return fail(e, false);
@@ -889,10 +1404,10 @@ int nir_mlp_predict_device(nir_mlp* h, const float* x_dev, int32_t n, float* y) 
             const size_t len = (size_t)k * h->cfg.d_in;
             k_to_bf16<<<grid1d(len), 256, 0, h->stream>>>(len, x_dev + (size_t)r * h->cfg.d_in, h->x);
             MLP_LAUNCHED();
-            forward(h, k);
+            forward(h, k, h->x);
             MLP_CUDA(cudaMemcpyAsync(y + (size_t)r * h->cfg.d_out, h->pred, (size_t)k * h->cfg.d_out * sizeof(float),
                                      cudaMemcpyDeviceToHost, h->stream));
-            MLP_CUDA(cudaStreamSynchronize(h->stream));
+            finish(h);
         }
     } catch (const std::exception& e) {
         return fail(e, false);
@@ -923,7 +1438,7 @@ int nir_mlp_set_affine(nir_mlp* h, int32_t n, int32_t col, double lo, double hi,
             MLP_CUDA(cudaMemcpyAsync(h->aff_shift, shift, size_t(n) * sizeof(double), cudaMemcpyHostToDevice,
                                      h->stream));
         }
-        MLP_CUDA(cudaStreamSynchronize(h->stream));
+        finish(h);
         h->aff_n = n;
         h->aff_col = col;
         h->aff_lo = lo;
@@ -949,13 +1464,13 @@ int nir_mlp_predict_device_affine(nir_mlp* h, const float* x_dev, int32_t n, con
             const size_t len = (size_t)k * h->cfg.d_in;
             k_to_bf16<<<grid1d(len), 256, 0, h->stream>>>(len, x_dev + (size_t)r * h->cfg.d_in, h->x);
             MLP_LAUNCHED();
-            forward(h, k);
+            forward(h, k, h->x);
             k_affine_out<<<unsigned((k + 255) / 256), 256, 0, h->stream>>>(k, r, h->pred, h->cfg.d_out, h->aff_col,
                                                                           h->aff_lo, h->aff_hi, h->aff_scale,
                                                                           h->aff_shift, h->aff_out);
             MLP_LAUNCHED();
         }
-        MLP_CUDA(cudaStreamSynchronize(h->stream));
+        finish(h);
         *out_dev = h->aff_out;
     } catch (const std::exception& e) {
         return fail(e, false);
@@ -971,11 +1486,18 @@ int nir_mlp_gradients(nir_mlp* h, const float* x, const float* targets, int32_t 
     try {
         MLP_CUDA(cudaSetDevice(h->device));
         ensure_rows(h, n);
+        ensure_backward(h, n);
+        ensure_parts(h, loss_blocks(h, n));
         upload_rows(h, x, n, h->x, h->cfg.d_in);
         MLP_CUDA(cudaMemcpyAsync(h->tgt, targets, (size_t)n * h->cfg.d_out * sizeof(float), cudaMemcpyHostToDevice,
                                  h->stream));
-        forward(h, n);
-        backward(h, n, 0);
+        forward(h, n, h->x);
+        backward(h, n, h->x, h->tgt, 0);
+        finish_losses(h, n, 1);
+        for (size_t l = 0; l < h->layers.size(); ++l)
+            k_colsum_final<<<(h->layers[l].out + 255) / 256, 256, 0, h->stream>>>(
+                colsum_chunks(n), h->layers[l].out, colsum_of(h, n, int(l)), h->layers[l].gb);
+        MLP_LAUNCHED();
         float lv = 0.f;
         MLP_CUDA(cudaMemcpyAsync(&lv, h->losses, sizeof(float), cudaMemcpyDeviceToHost, h->stream));
         if (grads) {
@@ -988,7 +1510,7 @@ int nir_mlp_gradients(nir_mlp* h, const float* x, const float* targets, int32_t 
                 o += ly.out;
             }
         }
-        MLP_CUDA(cudaStreamSynchronize(h->stream));
+        finish(h);
         if (loss) *loss = lv;
     } catch (const std::exception& e) {
         return fail(e, false);
@@ -1015,7 +1537,7 @@ int nir_mlp_gemm_check(nir_mlp* h, int a_kmaj, int b_kmaj, int32_t M, int32_t N,
         upload_rows(h, B, 1, db, int(nb));
         gemm(h, a_kmaj != 0, b_kmaj != 0, da, lda, db, ldb, M, N, K, EPI_F32, nullptr, nullptr, dc, N, nullptr, 0);
         MLP_CUDA(cudaMemcpyAsync(C, dc, (size_t)M * N * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-        MLP_CUDA(cudaStreamSynchronize(h->stream));
+        finish(h);
         h->release(da);
         h->release(db);
         h->release(dc);
