@@ -981,21 +981,36 @@ void pad_scaled(nir_pdhg* h) {
     }
 }
 
+// Launches a kernel on the handle's stream; `early`: it may start while the
+// kernel before it still runs (pdl_wait).
+template <typename... P, typename... A>
+void launch_kernel(nir_pdhg* h, bool early, void (*k)(P...), int grid, size_t smem, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(nir::kBlock);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    NIR_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...));
+}
+
 // The two FP64 KKT passes of a check over the layouts in use, at (xp, yp)
 // of type TX; returns their grids (the number of partials each wrote).
 template <typename TX>
 void launch_kkt(nir_pdhg* h, int phase, double* partKR, double* partKC, const TX* xp, const TX* yp, int* gkr,
-                int* gkc) {
-    cudaStream_t s = h->stream;
+                int* gkc, bool early = false) {
     with_lays(h, [&](auto lp, auto ld) {
         constexpr int LP = decltype(lp)::value, LD = decltype(ld)::value;
         *gkr = lay_grid<LD, double>(h, nir::k_kkt_rows<LD, TX>, lay_nblk(h->A));
         *gkc = lay_grid<LP, double>(h, nir::k_kkt_cols<LP, TX>, lay_nblk(h->At));
         nir::KktArgs kr{lay_of(h->A), vals_of<double>(h->A), partKR, h->st, phase};
-        nir::k_kkt_rows<LD, TX><<<*gkr, nir::kBlock, lay_smem<LD, double>(), s>>>(kr, xp, yp, h->dr, h->rl, h->ru);
+        launch_kernel(h, early, nir::k_kkt_rows<LD, TX>, *gkr, lay_smem<LD, double>(), kr, xp, yp, h->dr, h->rl, h->ru);
         nir::KktArgs kc{lay_of(h->At), vals_of<double>(h->At), partKC, h->st, phase};
-        nir::k_kkt_cols<LP, TX><<<*gkc, nir::kBlock, lay_smem<LP, double>(), s>>>(kc, xp, yp, h->dc, h->c, h->l, h->u);
-        NIR_LAUNCHED();
+        launch_kernel(h, early, nir::k_kkt_cols<LP, TX>, *gkc, lay_smem<LP, double>(), kc, xp, yp, h->dc, h->c, h->l, h->u);
     });
     h->launches += 2;
 }
@@ -1020,23 +1035,6 @@ struct SolveCfg {
     int persistent = 0;    // non-check iterations in one cooperative launch per chunk
     int barrier_test = 0;  // persistent launch whose barrier cannot complete (bounded-wait test)
 };
-
-// Launches a kernel on the handle's stream; `early`: it may start while the
-// kernel before it still runs (pdl_wait).
-template <typename... P, typename... A>
-void launch_kernel(nir_pdhg* h, bool early, void (*k)(P...), int grid, size_t smem, A&&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(unsigned(grid));
-    cfg.blockDim = dim3(nir::kBlock);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = h->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = early ? 1 : 0;
-    NIR_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...));
-}
 
 // Optional event timing of the first iteration of a chunk.
 struct ChunkTimer {
@@ -1130,7 +1128,8 @@ void launch_fast_chunk_l(nir_pdhg* h, const SolveCfg& cfg, int phase, ChunkTimer
         h->launches += 2;
     }
     int gkr = 0, gkc = 0;
-    launch_kkt<TX>(h, phase, L.KR, L.KC, Vec<TX>::xp(h), Vec<TX>::yp(h), &gkr, &gkc);
+    const bool early = !(tm && tm->armed);
+    launch_kkt<TX>(h, phase, L.KR, L.KC, Vec<TX>::xp(h), Vec<TX>::yp(h), &gkr, &gkc, early);
     h->launches -= 2;  // counted with the chunk below
     nir::CtlArgs ca = control_args(cfg, phase, h->hist);
     ca.partP = L.P;
@@ -1142,17 +1141,13 @@ void launch_fast_chunk_l(nir_pdhg* h, const SolveCfg& cfg, int phase, ChunkTimer
     ca.nKR = gkr;
     ca.nKC = gkc;
     ca.offset = h->offset;
-    nir::k_control<<<1, nir::kBlock, 0, s>>>(ca, h->st);
-    NIR_LAUNCHED();
-    const int nm = std::max(h->n, h->m);
-    nir::k_apply_restart<TX><<<grid_for(nm), nir::kBlock, 0, s>>>(h->n, h->m, h->st, phase, Vec<TX>::x(h),
-                                                                   Vec<TX>::x0(h), Vec<TX>::xp(h), Vec<TX>::y(h),
-                                                                   Vec<TX>::y0(h), Vec<TX>::yp(h));
-    NIR_LAUNCHED();
-    nir::k_snap<<<1, 32, 0, s>>>(h->st, h->snap.ring, h->snap.d_seq);
-    NIR_LAUNCHED();
+    launch_kernel(h, early, nir::k_control, 1, 0, ca, h->st);
+    const int nm = std::max(1, std::max(h->n, h->m));
+    launch_kernel(h, early, nir::k_apply_restart<TX>, int(grid_for(nm)), 0, h->n, h->m, (const nir::DevState*)h->st, phase,
+                  Vec<TX>::x(h), Vec<TX>::x0(h), Vec<TX>::xp(h), Vec<TX>::y(h), Vec<TX>::y0(h), Vec<TX>::yp(h),
+                  h->snap.ring, h->snap.d_seq);
     if (tm && tm->armed) NIR_CUDA(cudaEventRecord(tm->e[3], s));
-    h->launches += 5;
+    h->launches += 4;
 }
 
 template <typename TV, typename TX>
@@ -1293,7 +1288,7 @@ struct LoopResult {
     double t_switch = 0.0;
 };
 
-int launches_per_chunk(int K, bool ref) { return ref ? 2 * K + 3 : 2 * K + 5; }
+int launches_per_chunk(int K, bool ref) { return ref ? 2 * K + 3 : 2 * K + 4; }
 
 // Runs chunks until the device reports done, the phase changes, or the
 // caller's poll / time limit stops it.  Keeps `depth` chunks in flight.

@@ -296,40 +296,23 @@ struct BatchCtlArgs {
     const unsigned char* skip;  // instances that clusters run, or null
 };
 
-__device__ inline double range_sum(const double* __restrict__ p, int lo, int hi, double* sh) {
-    double s = 0.0;
-    for (int i = lo + threadIdx.x; i < hi; i += kBlock) s += p[i];
-    return block_sum(s, sh);
-}
-
-__device__ inline double range_max(const double* __restrict__ p, int lo, int hi, double* sh) {
-    double s = 0.0;
-    for (int i = lo + threadIdx.x; i < hi; i += kBlock) s = fmax(s, p[i]);
-    return block_max(s, sh);
-}
-
 // One CTA per instance.
 __global__ void __launch_bounds__(kBlock) k_bcontrol(CtlArgs a, BatchCtlArgs b, DevState* insts) {
-    __shared__ double sh[kWarps];
+    __shared__ CtlShared sh;
     const int i = blockIdx.x;
     DevState* st = insts + i;
-    if (st->done || st->phase != a.phase || (b.skip && b.skip[i])) return;
+    ctl_copy_state(&sh.st, st);
+    __syncthreads();
+    if (sh.st.done || sh.st.phase != a.phase || (b.skip && b.skip[i])) return;
     const int p0 = b.at_lo[i], p1 = b.at_lo[i + 1], d0 = b.a_lo[i], d1 = b.a_lo[i + 1];
-    CtlSums s;
-    s.dx2 = range_sum(b.partP, p0, p1, sh);
-    s.dxa2 = range_sum(b.partP + b.nP, p0, p1, sh);
-    s.dy2 = range_sum(b.partD, d0, d1, sh);
-    s.dya2 = range_sum(b.partD + b.nD, d0, d1, sh);
-    s.pres2 = range_sum(b.partKR, d0, d1, sh);
-    s.dobj_r = range_sum(b.partKR + b.nD, d0, d1, sh);
-    s.ywrong2 = range_sum(b.partKR + 2 * b.nD, d0, d1, sh);
-    s.maxrel = range_max(b.partKR + 3 * b.nD, d0, d1, sh);
-    s.dres2 = range_sum(b.partKC, p0, p1, sh);
-    s.dobj_c = range_sum(b.partKC + b.nP, p0, p1, sh);
-    s.pobj_c = range_sum(b.partKC + 2 * b.nP, p0, p1, sh);
-    s.xviol2 = range_sum(b.partKC + 3 * b.nP, p0, p1, sh);
-    if (threadIdx.x != 0) return;
-    control_update(a, st, s, b.bnorm[i], b.cnorm[i], b.offset[i], nullptr);
+    ctl_sums({b.partP, b.nP, p0, p1}, {b.partD, b.nD, d0, d1}, {b.partKR, b.nD, d0, d1}, {b.partKC, b.nP, p0, p1}, sh);
+    if (threadIdx.x == 0) {
+        const double* s = sh.sum;
+        const CtlSums sums{s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], s[8], s[9], s[10], s[11]};
+        control_update(a, &sh.st, sums, b.bnorm[i], b.cnorm[i], b.offset[i], nullptr);
+    }
+    __syncthreads();
+    ctl_copy_state(st, &sh.st);
 }
 
 template <typename T>

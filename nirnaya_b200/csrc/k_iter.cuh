@@ -156,9 +156,10 @@ struct KktArgs {
 
 template <int LAY, typename TX>
 __global__ void __launch_bounds__(kBlock)
-    k_kkt_rows(KktArgs a, const TX* __restrict__ xplus, const TX* __restrict__ yplus, const double* __restrict__ dr,
+    k_kkt_rows(KktArgs a, const TX* xplus, const TX* yplus, const double* __restrict__ dr,
                const double* __restrict__ rl, const double* __restrict__ ru) {
     __shared__ double s_red[kWarps];
+    pdl_release();
     if (a.st->done || a.st->phase != a.phase) return;
     KktRowEpi<TX> epi;
     epi.dr = dr;
@@ -171,9 +172,10 @@ __global__ void __launch_bounds__(kBlock)
 
 template <int LAY, typename TX>
 __global__ void __launch_bounds__(kBlock)
-    k_kkt_cols(KktArgs a, const TX* __restrict__ xplus, const TX* __restrict__ yplus, const double* __restrict__ dc,
+    k_kkt_cols(KktArgs a, const TX* xplus, const TX* yplus, const double* __restrict__ dc,
                const double* __restrict__ c, const double* __restrict__ l, const double* __restrict__ u) {
     __shared__ double s_red[kWarps];
+    pdl_release();
     if (a.st->done || a.st->phase != a.phase) return;
     KktColEpi<TX> epi;
     epi.dc = dc;

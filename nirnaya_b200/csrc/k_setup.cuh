@@ -433,8 +433,8 @@ struct HostSnap {
 
 constexpr int kSnapRing = 64;
 
-__global__ void k_snap(const DevState* __restrict__ st, HostSnap* __restrict__ ring, long long* __restrict__ seq) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// One thread.
+__device__ inline void write_snap(const DevState* st, HostSnap* ring, long long* seq) {
     long long s = *seq + 1;
     *seq = s;
     HostSnap h;
@@ -458,6 +458,10 @@ __global__ void k_snap(const DevState* __restrict__ st, HostSnap* __restrict__ r
     h.pad = 0;
     ring[s % kSnapRing] = h;
     __threadfence_system();
+}
+
+__global__ void k_snap(const DevState* st, HostSnap* ring, long long* seq) {
+    if (threadIdx.x == 0 && blockIdx.x == 0) write_snap(st, ring, seq);
 }
 
 }  // namespace nir
