@@ -207,7 +207,7 @@ __device__ __forceinline__ void lay_spmv_batch(const BatchArgs& a, const TV* __r
             const DevState& s = a.inst[inst];
             if (!inst_active(s, a.phase)) continue;
             set(epi, s);
-            cta_block<TA, TV, TX, LAY, Epi, COH>(d0, d1, L.rp, L.ci, val, x, epi, sm[k & 1]);
+            cta_block<TA, TV, TX, LAY, Epi, COH>(d0, d1, L.rp, L.ci, val, x, epi, sm[k & 1], false);
             ++k;
             if (Epi::NQ > 0) flush_cta_partials(epi, a.part, L.nblk, b, s_red);
         }
