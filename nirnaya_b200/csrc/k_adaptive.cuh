@@ -292,6 +292,7 @@ __global__ void __launch_bounds__(kBlock, iter_min_blocks<TA>()) k_spmv_adaptive
     __shared__ TA s_red[kWarps];
     PlainEpi<TA> epi;
     epi.y = y;
+    pdl_release();
     rowblock_spmv<TA, TV, TX>(blk, nblk, cap, rp, ci, val, x, epi, s_red);
 }
 

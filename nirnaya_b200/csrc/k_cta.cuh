@@ -307,6 +307,7 @@ __global__ void __launch_bounds__(kBlock, cta_min_blocks<TA, E>())
     __shared__ CtaShared<TA> sm[2];
     CtaPlainEpi<TA> epi;
     epi.y = y;
+    pdl_release();
     cta_spmv<TA, TV, TX, E>(blk, nblk, rp, ci, val, x, epi, sm);
 }
 
