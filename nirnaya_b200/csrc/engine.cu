@@ -1503,8 +1503,10 @@ void power_spmv(nir_pdhg* h, const Orient& o, int lanes, const double* x, const 
                 double* y) {
     with_lanes(lanes, [&](auto t) {
         constexpr int T = decltype(t)::value;
-        nir::k_power_spmv<T><<<grid_for((long long)o.rows * T), nir::kBlock, 0, h->stream>>>(o.rows, o.rp, o.ci, o.v64, x,
-                                                                                            norm, inst_of, y);
+        // early where the grid fits the device at once: in the last wave of a
+        // larger one the waiting CTAs would only take room
+        const int grid = int(grid_for((long long)o.rows * T));
+        launch_kernel(h, grid <= max_grid(h), nir::k_power_spmv<T>, grid, 0, o.rows, o.rp, o.ci, o.v64, x, norm, inst_of, y);
     });
 }
 
@@ -1588,23 +1590,22 @@ void precondition(nir_pdhg* h, const nir_pdhg_params& p, bool enable) {
             if (mode == 0) {
                 with_lanes(lm, [&](auto t) {
                     constexpr int T = decltype(t)::value;
-                    nir::k_row_max<T><<<grid_for((long long)m * T), nir::kBlock, 0, s>>>(m, h->A.rp, h->A.ci, h->A.v_orig,
-                                                                                         h->dr, h->dc, h->tmp_m);
+                    launch_kernel(h, it > 0, nir::k_row_max<T>, int(grid_for((long long)m * T)), 0, m, h->A.rp, h->A.ci,
+                                  h->A.v_orig, h->dr, h->dc, h->tmp_m);
                 });
                 with_lanes(ln, [&](auto t) {
                     constexpr int T = decltype(t)::value;
-                    nir::k_row_max<T><<<grid_for((long long)n * T), nir::kBlock, 0, s>>>(
-                        n, h->At.rp, h->At.ci, h->At.v_orig, h->dc, h->dr, h->tmp_n);
+                    launch_kernel(h, true, nir::k_row_max<T>, int(grid_for((long long)n * T)), 0, n, h->At.rp, h->At.ci,
+                                  h->At.v_orig, h->dc, h->dr, h->tmp_n);
                 });
             } else {
-                nir::k_row_stat<<<std::max(gwm, 1u), nir::kBlock, 0, s>>>(m, h->A.rp, h->A.ci, h->A.v_orig, h->dr, h->dc,
-                                                                         mode, h->tmp_m);
-                nir::k_row_stat<<<std::max(gwn, 1u), nir::kBlock, 0, s>>>(n, h->At.rp, h->At.ci, h->At.v_orig, h->dc,
-                                                                         h->dr, mode, h->tmp_n);
+                launch_kernel(h, it > 0, nir::k_row_stat, int(gwm), 0, m, h->A.rp, h->A.ci, h->A.v_orig, h->dr, h->dc, mode,
+                              h->tmp_m);
+                launch_kernel(h, true, nir::k_row_stat, int(gwn), 0, n, h->At.rp, h->At.ci, h->At.v_orig, h->dc, h->dr,
+                              mode, h->tmp_n);
             }
-            nir::k_apply_stat<<<grid_for(m), nir::kBlock, 0, s>>>(m, h->tmp_m, h->dr);
-            nir::k_apply_stat<<<grid_for(n), nir::kBlock, 0, s>>>(n, h->tmp_n, h->dc);
-            NIR_LAUNCHED();
+            launch_kernel(h, true, nir::k_apply_stat, int(grid_for(m)), 0, m, h->tmp_m, h->dr);
+            launch_kernel(h, true, nir::k_apply_stat, int(grid_for(n)), 0, n, h->tmp_n, h->dc);
             h->launches += 4;
         }
         nir::k_round_pow2<<<grid_for(m), nir::kBlock, 0, s>>>(m, h->dr);
@@ -1640,8 +1641,8 @@ double power_norm(nir_pdhg* h, int rounds) {
     one_instance(h);
     const int G = int(std::min(grid_for(n), 128u));
     auto measure = [&]() {
-        nir::k_seg_sumsq<<<unsigned(G), nir::kBlock, 0, s>>>(G, h->one_col, h->tmp_n, L.misc);
-        nir::k_seg_norm<<<1, 32, 0, s>>>(1, G, L.misc, norm_est);
+        launch_kernel(h, true, nir::k_seg_sumsq, G, 0, G, (const int*)h->one_col, h->tmp_n, L.misc);
+        launch_kernel(h, true, nir::k_seg_norm, 1, 0, 1, G, L.misc, norm_est);
     };
     nir::k_power_start<<<std::max(grid_for(n), 1u), nir::kBlock, 0, s>>>(n, h->tmp_n);
     measure();

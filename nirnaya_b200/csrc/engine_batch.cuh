@@ -417,8 +417,8 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
     constexpr int G = 8;  // CTAs per instance of the norms
     const int lm = row_lanes(h->A), ln = row_lanes(h->At);
     auto measure = [&]() {
-        nir::k_seg_sumsq<<<unsigned(I) * G, nir::kBlock, 0, s>>>(G, B->d_col_off, h->tmp_n, B->d_norm_part);
-        nir::k_seg_norm<<<grid_for(I * 32LL), nir::kBlock, 0, s>>>(I, G, B->d_norm_part, B->d_norm);
+        launch_kernel(h, true, nir::k_seg_sumsq, I * G, 0, G, (const int*)B->d_col_off, h->tmp_n, B->d_norm_part);
+        launch_kernel(h, true, nir::k_seg_norm, int(grid_for(I * 32LL)), 0, I, G, B->d_norm_part, B->d_norm);
     };
     nir::k_power_start_batch<<<grid_for(n), nir::kBlock, 0, s>>>(n, B->d_col_inst, B->d_col_off, h->tmp_n);
     measure();
