@@ -12,7 +12,7 @@
  * Layers: d_in -> width (ReLU) -> ... (depth hidden layers) -> d_out.
  * FP32 master weights; activations, weight copies and gradients with
  * respect to activations in BF16; every contraction accumulates in FP32 on
- * the tensor cores (hand-written kernels, mma.sync m16n8k16 BF16).
+ * the tensor cores (hand-written kernels, tcgen05 BF16).
  * Training: mean-squared error over the outputs with weight 1 (outputs
  * with weight 0 are padding), Adam.
  *
