@@ -338,9 +338,10 @@ struct nir_pdhg {
     int* gs_err = nullptr;
     int launches = 0;
     std::shared_ptr<ClusterPlan> cluster;  // one LP's plan (engine_cluster.cuh), built by its first solve in clusters
-    // one LP as the instance-wise kernels see it ({0, m}, {0, n}), and their
-    // partial sums and results (dd_sums)
+    // one LP as the instance-wise kernels see it ({0, m}, {0, n}, the
+    // objective's offset), and their partial sums and results (dd_sums)
     int *one_row = nullptr, *one_col = nullptr;
+    double* one_offset = nullptr;
     nir::vfy::DD* dd_part = nullptr;
     size_t dd_len = 0;
     double* dd_out = nullptr;
@@ -1546,19 +1547,21 @@ void lp_norms(nir_pdhg* h, int count, const int* row_off, const int* col_off, do
     for (int k = 0; k < count * nir::kDdNorms; ++k) out[k] = std::sqrt(out[k]);
 }
 
-// Each instance's objective at the point x on the device.
+// Each instance's objective at the point x on the device, its offset included.
 void lp_objectives(nir_pdhg* h, int count, const int* col_off, const double* offsets, const double* x, double* out) {
     dd_sums(h, count, 1, offsets, out, [&](int G, nir::vfy::DD* part) {
         nir::k_dd_objective<<<unsigned(count) * unsigned(G), nir::kBlock, 0, h->stream>>>(G, col_off, h->c, x, part);
     });
 }
 
-// One LP's offsets for the instance-wise kernels.
+// One LP's row, column and objective offsets for the instance-wise kernels.
 void one_instance(nir_pdhg* h) {
     if (h->one_row) return;
     int* p = h->alloc<int>(4);
     const int o[4] = {0, h->m, 0, h->n};
     h2d(h, p, o, sizeof(o));
+    h->one_offset = h->alloc<double>(1);
+    h2d(h, h->one_offset, &h->offset, sizeof(double));
     h->one_row = p;
     h->one_col = p + 2;
 }
@@ -2028,7 +2031,7 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
     NIR_LAUNCHED();
     if (x_out) NIR_CUDA(cudaMemcpyAsync(x_out, h->out_x, n * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (y_out) NIR_CUDA(cudaMemcpyAsync(y_out, h->out_y, m * sizeof(double), cudaMemcpyDeviceToHost, s));
-    lp_objectives(h, 1, h->one_col, nullptr, h->out_x, &info->objective);
+    lp_objectives(h, 1, h->one_col, h->one_offset, h->out_x, &info->objective);
     h->last_x = h->out_x;
     int status;
     if (st.done) status = st.status;
