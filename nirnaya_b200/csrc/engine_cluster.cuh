@@ -161,7 +161,7 @@ std::unique_ptr<ClusterPlan> cl_build(nir_pdhg* h, int C, const std::vector<int>
             d2h(h, gr.data(), t->ghost_rank, gr.size() * sizeof(int));
             t->come.resize(gr.size());
             d2h(h, t->come.data(), t->bytes, t->come.size() * sizeof(int));
-            t->ghosts.assign(size_t(P.count), 1);  // slot 0 backs the padding's index
+            t->ghosts.assign(size_t(P.count), nir::kClZeroSlots);  // the padding's index
             for (int i = 0; i < P.count; ++i)
                 for (int r = 0; r < C; ++r) t->ghosts[size_t(i)] = std::max(t->ghosts[size_t(i)], gr[size_t(i) * C + r]);
             t->ghost = cl_upload(h, P, t->ghosts);

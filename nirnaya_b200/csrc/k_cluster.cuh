@@ -58,6 +58,11 @@ constexpr int kClSums = 12;          // quantities of a check (CtlSums)
 constexpr int kClWeights = 64;       // iterations whose Halpern weights are tabulated
 constexpr int kClBulkPart = 8;       // a rank that gathers 1/8 of another's entries gets all of them by one copy
 constexpr int kClUnit = 64;          // stream entries of one step pair: 32 lanes x 2
+// Slots 0 and 1 of both sides hold zero throughout: the padding of a slice
+// gathers slot 0, and its product is 0 whatever the iterate holds (a real
+// entry's slot there turned an overflow in it, 0 x inf, into a NaN in every
+// padded row).  Two, so that whole segments stay at even slots.
+constexpr int kClZeroSlots = 2;
 
 // What an instance keeps in shared memory beside the gathered entries and
 // the slices.
@@ -705,8 +710,9 @@ __global__ void k_cl_need(int rows, const int* __restrict__ order, const int* __
 // Slots of one side for rank r = b % C of instance b / C.  The entries of a
 // source rank s that r gathers are numbered in position order; where they
 // are one in kClBulkPart of s's entries or more, and for s = r, all of s's
-// entries get slots, from an even one on, so that one bulk copy brings them.  ghost[b]
-// is the number of slots, bytes[b] what a phase brings from other ranks;
+// entries get slots, from an even one on, so that one bulk copy brings them.  The
+// first kClZeroSlots are nobody's.  ghost[b] is the number of slots, bytes[b]
+// what a phase brings from other ranks;
 // all[b] collects the sources taken whole (bit s).
 __global__ void __launch_bounds__(kBlock) k_cl_slots(int C, const int* __restrict__ off, const int* __restrict__ bound,
                                                      const unsigned short* __restrict__ need,
@@ -717,7 +723,7 @@ __global__ void __launch_bounds__(kBlock) k_cl_slots(int C, const int* __restric
     const int p0 = off[i], n = off[i + 1] - p0;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned short* out = slot + size_t(C) * p0 + size_t(r) * n;
-    int carry = 0, come = 0;
+    int carry = kClZeroSlots, come = 0;
     unsigned whole = 0;
     for (int s = 0; s < C; ++s) {
         const int b0 = bound[i * (C + 1) + s], b1 = bound[i * (C + 1) + s + 1];
@@ -791,8 +797,8 @@ __device__ __forceinline__ int cl_source(const int4 d, int lane, int step, int p
     return e < rp[r + 1] - rp[r] ? rp[r] + e : -1;
 }
 
-// One warp per slice: the slots its entries gather (0 in the padding, whose
-// values are 0).
+// One warp per slice: the slots its entries gather (slot 0, which holds zero,
+// in the padding, whose values are 0).
 __global__ void k_cl_fill_idx(int ns, int C, const int4* __restrict__ slices, const int* __restrict__ owner,
                               ClSide side, ClSide other, const int* __restrict__ order, const int* __restrict__ rp,
                               const int* __restrict__ ci, const int* __restrict__ pos_other,
