@@ -122,7 +122,9 @@ typedef struct nir_pdhg_params {
                                      iteration at 40k nonzeros: two grid barriers cost more
                                      than two graph-launched kernels); 2 = test of the
                                      barrier's bounded wait (one CTA too many: the solve
-                                     must end with NIR_STATUS_INTERNAL_ERROR in ~0.1 s)  (0) */
+                                     must end with NIR_STATUS_INTERNAL_ERROR in ~0.1 s); 3 =
+                                     the same test of the waits in thread-block clusters,
+                                     where the solve runs in them (some seconds)     (0) */
     int32_t pad_;
 } nir_pdhg_params;
 

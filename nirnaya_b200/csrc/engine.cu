@@ -1034,7 +1034,7 @@ struct SolveCfg {
     int mixed = 0;
     double bnorm = 0.0, cnorm = 0.0;
     int persistent = 0;    // non-check iterations in one cooperative launch per chunk
-    int barrier_test = 0;  // persistent launch whose barrier cannot complete (bounded-wait test)
+    int barrier_test = 0;  // persistent or cluster launch one of whose waits cannot complete (bounded-wait test)
 };
 
 // Optional event timing of the first iteration of a chunk.
@@ -1864,7 +1864,7 @@ int solve_fast(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), void* 
         const bool want = p.persistent == 1 || p.persistent == 2;
         if (want && !coop) throw std::invalid_argument("persistent chunks need cooperative launch support");
         cfg.persistent = (want && coop && !h->profiling) ? 1 : 0;
-        cfg.barrier_test = (cfg.persistent && p.persistent == 2) ? 1 : 0;
+        cfg.barrier_test = (cfg.persistent && p.persistent == 2) || (cl && p.persistent == kClWaitTest) ? 1 : 0;
         if (cfg.persistent) {
             NIR_CUDA(cudaMemsetAsync(h->gs_count, 0, sizeof(unsigned), s));
             NIR_CUDA(cudaMemsetAsync(h->gs_gen, 0, sizeof(unsigned), s));

@@ -243,7 +243,7 @@ void launch_batch_chunk(nir_pdhg_batch* B, const SolveCfg& cfg, int phase) {
     if constexpr (sizeof(TX) == 8) {
         if (B->in_cluster)
             cl_launch<TV>(h, *B->cluster, control_args(cfg, phase, nullptr), cfg.K, 1, phase, cfg.p.reflection, B->insts,
-                          B->d_bnorm, B->d_cnorm, B->d_offset);
+                          B->d_bnorm, B->d_cnorm, B->d_offset, cfg.barrier_test != 0);
     }
     if (B->cur)
         with_batch_lays(B, [&](auto lp, auto ld) {
@@ -404,7 +404,7 @@ int batch_solve_impl(nir_pdhg_batch* B, const nir_pdhg_params& p, int (*poll)(vo
         const bool want = p.persistent == 1 || p.persistent == 2;
         if (want && !coop) throw std::invalid_argument("persistent chunks need cooperative launch support");
         cfg.persistent = want ? 1 : 0;
-        cfg.barrier_test = (want && p.persistent == 2) ? 1 : 0;
+        cfg.barrier_test = (want && p.persistent == 2) || (cl && p.persistent == kClWaitTest) ? 1 : 0;
         if (cfg.persistent) {
             NIR_CUDA(cudaMemsetAsync(h->gs_count, 0, sizeof(unsigned), s));
             NIR_CUDA(cudaMemsetAsync(h->gs_gen, 0, sizeof(unsigned), s));

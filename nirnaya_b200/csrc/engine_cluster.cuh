@@ -275,7 +275,7 @@ void cl_prepare_kernel() {
 // instance; the norms and offsets by instance, or null for one LP.
 template <typename TV>
 void cl_launch(nir_pdhg* h, ClusterPlan& P, const nir::CtlArgs& ctl, int K, int halpern, int phase, double rho,
-               nir::DevState* st, const double* bnorm, const double* cnorm, const double* offset) {
+               nir::DevState* st, const double* bnorm, const double* cnorm, const double* offset, bool wait_test) {
     const int q = sizeof(TV) == 8 ? 1 : 0;
     nir::ClArgs a{};
     a.col = cl_side(P.col, P.d_col_off);
@@ -294,6 +294,7 @@ void cl_launch(nir_pdhg* h, ClusterPlan& P, const nir::CtlArgs& ctl, int K, int 
     a.bnorm = bnorm;
     a.cnorm = cnorm;
     a.offset = offset;
+    a.lost = wait_test ? 8 : 0;
     a.ctl = ctl;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(P.members) * unsigned(P.C));
@@ -331,12 +332,15 @@ int cl_resident(int C, size_t smem) {
     return n;
 }
 
+// nir_pdhg_params.persistent: clusters, one of whose waits cannot end.
+constexpr int kClWaitTest = 3;
+
 // The solves a cluster can run: the default iteration in FP64 arithmetic.
 // A caller that fixes a layout, asks for the persistent kernel, for FP32
 // iterates, for single launches or their timing, or for a fresh FP64 phase
 // gets the per-launch kernels.
 bool cl_takes(const nir_pdhg* h, const nir_pdhg_params& p) {
-    return p.spmv_block_nnz == 0 && p.persistent == 0 && p.use_graphs && !h->profiling &&
+    return p.spmv_block_nnz == 0 && (p.persistent == 0 || p.persistent == kClWaitTest) && p.use_graphs && !h->profiling &&
            p.precision != NIR_PREC_FP32 && (p.precision == NIR_PREC_FP64 || p.polish_fresh == 2);
 }
 
@@ -462,9 +466,11 @@ void launch_cluster_chunk(nir_pdhg* h, ClusterPlan& P, const SolveCfg& cfg, int 
     nir::CtlArgs ca = control_args(cfg, phase, h->hist);
     ca.offset = h->offset;
     if (fp64_values)
-        cl_launch<double>(h, P, ca, cfg.K, cfg.halpern, phase, cfg.p.reflection, h->st, nullptr, nullptr, nullptr);
+        cl_launch<double>(h, P, ca, cfg.K, cfg.halpern, phase, cfg.p.reflection, h->st, nullptr, nullptr, nullptr,
+                          cfg.barrier_test != 0);
     else
-        cl_launch<float>(h, P, ca, cfg.K, cfg.halpern, phase, cfg.p.reflection, h->st, nullptr, nullptr, nullptr);
+        cl_launch<float>(h, P, ca, cfg.K, cfg.halpern, phase, cfg.p.reflection, h->st, nullptr, nullptr, nullptr,
+                         cfg.barrier_test != 0);
     nir::k_snap<<<1, 32, 0, h->stream>>>(h->st, h->snap.ring, h->snap.d_seq);
     NIR_LAUNCHED();
     h->launches += 1;

@@ -107,6 +107,7 @@ struct ClArgs {
     double rho;
     DevState* st;       // [instance]
     const double *bnorm, *cnorm, *offset;  // [instance], or null: the state's norms and ctl.offset
+    int lost;           // test of the bounded waits: rank 0 waits for so many bytes that nobody sends
     CtlArgs ctl;
 };
 
@@ -156,8 +157,14 @@ __device__ __forceinline__ void cl_bar_expect(unsigned bar, unsigned bytes) {
 }
 // Waits for a phase's bytes, at most kClWaitCycles; false when they did not
 // come (they always do: the senders run on the same cluster), at once when
-// another wait has failed.
-constexpr long long kClWaitCycles = 2000000000LL;
+// another wait has failed.  A CTA whose wait failed ends the iteration, with
+// what it owes the others in it, and the chunk: it opens no phase and sends
+// nothing any more, so no barrier is re-armed in the middle of a phase and
+// none counts more than three phases' bytes.  The ranks that wait for it give
+// up in turn.  All meet at the check's cluster barrier, after which nobody
+// sends, and a cluster with a failed rank stays kClSettleCycles more, so
+// that copies in flight land in shared memory that is still theirs.
+constexpr long long kClWaitCycles = 2000000000LL, kClSettleCycles = 2000000LL;
 __device__ __forceinline__ bool cl_bar_wait(unsigned bar, unsigned parity, const volatile int* failed) {
     long long t0 = 0;
     for (;;) {
@@ -344,10 +351,11 @@ struct ClShared {
     unsigned long long bar[2];  // arrivals of x-bar and of y
     double tau, sigma, isigma, rho;
     int failed;             // a wait ran out
+    int stop;               // the same at the end of the last dual pass
     double2 w[kClWeights];  // Halpern weights (k + 1) / (k + 2), 1 / (k + 2) of the chunk's first iterations
     double warp[kClWarps][kClSums];
     double rank[kClRanksMax][kClSums];
-    double fail[kClRanksMax];
+    double fail[kClRanksMax];  // 1: a wait of that rank ran out
 };
 
 __device__ __forceinline__ double2 cl_weights(double k) { return make_double2((k + 1.0) / (k + 2.0), 1.0 / (k + 2.0)); }
@@ -436,91 +444,103 @@ __device__ __forceinline__ void cl_dual(ClShared<RES, TV>& S, int xs, unsigned p
                 s[1] += e * e;
             }
         });
+    // What the CTA goes by: thread 0 opens the phases, so its own waits count
+    // here at once; a wait of another thread that ends later, at the latest
+    // with the next iteration.  (A vote of all threads in both barriers took
+    // 1 to 4% of an iteration, this 0.1 to 1.2%.)
+    if (threadIdx.x == 0) S.stop = S.failed;
     cl_flush(R);
 }
 
 // The rest of a check, once per chunk and kept out of the iterations'
 // registers: the KKT sums of (x+, y+) in the original space on the FP64
-// values, the reduction over the cluster and the controller.
+// values, the reduction over the cluster and the controller.  A CTA that a
+// wait of its iterations failed in only reports that.
 template <bool RES, typename TV>
 __device__ __noinline__ void cl_check(const ClArgs& a, ClShared<RES, TV>& S, int xs, int ys, unsigned parity, unsigned rank,
                                       int inst, DevState* st, double sp0, double sp1, double sd0, double sd1) {
     const int C = a.C, tid = threadIdx.x;
-    const double* xp = a.v.xp + S.col.p0;
-    const double* yp = a.v.yp + S.row.p0;
-    __syncthreads();  // every warp is past its last phases; xp and yp as this CTA wrote them
-    // y+ has come from every rank whose rows gather x-bar from here: x+ may take its place there
-    cl_open(S.row);
-    cl_await(S, S.row, parity);
-    __syncthreads();
-    cl_open(S.col);
-    for (int j = tid; j < S.col.n; j += kClThreads) cl_push(S.col, j, S.col.need[j], xp[j], 0, 1, C);
-    cl_flush(S.col);
-    double sum[kClSums] = {sp0, sp1, sd0, sd1};
-    {
-        KktColEpi<double> e;
-        e.dc = a.v.dc + S.col.p0;
-        e.c = a.v.oc + S.col.p0;
-        e.l = a.v.ol + S.col.p0;
-        e.u = a.v.ou + S.col.p0;
-        using Pre = typename KktColEpi<double>::Pre;
-        // x+ was written in this launch: a plain load, not the read-only path
-        cl_pass<Pre, false, double2>(
-            S.col.sl, S.col.ns, S.col.idx_g, S.col.val64, ys, []() {},
-            [&](int j) { return Pre{__ldg(e.dc + j), __ldg(e.c + j), __ldg(e.l + j), __ldg(e.u + j), xp[j]}; },
-            [&](int j, double aty, const Pre& p, int first, int) {
-                if (!first) e.row(j, aty, p);
-            });
+    // every warp is past its last phases; xp and yp as this CTA wrote them
+    if (__syncthreads_and(S.failed == 0)) {
+        const double* xp = a.v.xp + S.col.p0;
+        const double* yp = a.v.yp + S.row.p0;
+        // y+ has come from every rank whose rows gather x-bar from here: x+ may take its place there
+        cl_open(S.row);
+        cl_await(S, S.row, parity);
+        __syncthreads();
+        cl_open(S.col);
+        for (int j = tid; j < S.col.n; j += kClThreads) cl_push(S.col, j, S.col.need[j], xp[j], 0, 1, C);
+        cl_flush(S.col);
+        double sum[kClSums] = {sp0, sp1, sd0, sd1};
+        {
+            KktColEpi<double> e;
+            e.dc = a.v.dc + S.col.p0;
+            e.c = a.v.oc + S.col.p0;
+            e.l = a.v.ol + S.col.p0;
+            e.u = a.v.ou + S.col.p0;
+            using Pre = typename KktColEpi<double>::Pre;
+            // x+ was written in this launch: a plain load, not the read-only path
+            cl_pass<Pre, false, double2>(
+                S.col.sl, S.col.ns, S.col.idx_g, S.col.val64, ys, []() {},
+                [&](int j) { return Pre{__ldg(e.dc + j), __ldg(e.c + j), __ldg(e.l + j), __ldg(e.u + j), xp[j]}; },
+                [&](int j, double aty, const Pre& p, int first, int) {
+                    if (!first) e.row(j, aty, p);
+                });
 #pragma unroll
-        for (int q = 0; q < 4; ++q) sum[8 + q] = e.q[q];
-    }
-    {
-        KktRowEpi<double> e;
-        e.dr = a.v.dr + S.row.p0;
-        e.rl = a.v.orl + S.row.p0;
-        e.ru = a.v.oru + S.row.p0;
-        using Pre = typename KktRowEpi<double>::Pre;
-        cl_pass<Pre, false, double2>(
-            S.row.sl, S.row.ns, S.row.idx_g, S.row.val64, xs, [&]() { cl_await(S, S.col, parity); },
-            [&](int i) { return Pre{__ldg(e.dr + i), __ldg(e.rl + i), __ldg(e.ru + i), yp[i]}; },
-            [&](int i, double ax, const Pre& p, int first, int) {
-                if (!first) e.row(i, ax, p);
-            });
-#pragma unroll
-        for (int q = 0; q < 4; ++q) sum[4 + q] = e.q[q];
-    }
-
-    // sums: lanes, then warps, then ranks, in order (sum[7] is a maximum)
-#pragma unroll
-    for (int q = 0; q < kClSums; ++q) {
-        const double v = q == 7 ? warp_max(sum[q]) : warp_sum(sum[q]);
-        if ((tid & 31) == 0) S.warp[tid >> 5][q] = v;
-    }
-    __syncthreads();
-    if (tid < kClSums) {
-        double v = 0.0;
-        for (int k = 0; k < kClWarps; ++k) v = tid == 7 ? fmax(v, S.warp[k][tid]) : v + S.warp[k][tid];
-        cl_store(unsigned(__cvta_generic_to_shared(&S.rank[rank][tid])), 0, v);
-    }
-    if (tid == kClSums) cl_store(unsigned(__cvta_generic_to_shared(&S.fail[rank])), 0, S.failed ? 1.0 : 0.0);
-    cl_sync();
-    if (rank == 0 && tid == 0) {
-        double t[kClSums];
-        bool failed = false;
-        for (int q = 0; q < kClSums; ++q) {
-            t[q] = 0.0;
-            for (int r = 0; r < C; ++r) t[q] = q == 7 ? fmax(t[q], S.rank[r][q]) : t[q] + S.rank[r][q];
+            for (int q = 0; q < 4; ++q) sum[8 + q] = e.q[q];
         }
-        for (int r = 0; r < C; ++r) failed |= S.fail[r] != 0.0;
-        const CtlSums s{t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10], t[11]};
-        control_update(a.ctl, st, s, a.bnorm ? a.bnorm[inst] : st->bnorm, a.cnorm ? a.cnorm[inst] : st->cnorm,
-                       a.offset ? a.offset[inst] : a.ctl.offset, a.ctl.hist);
+        {
+            KktRowEpi<double> e;
+            e.dr = a.v.dr + S.row.p0;
+            e.rl = a.v.orl + S.row.p0;
+            e.ru = a.v.oru + S.row.p0;
+            using Pre = typename KktRowEpi<double>::Pre;
+            cl_pass<Pre, false, double2>(
+                S.row.sl, S.row.ns, S.row.idx_g, S.row.val64, xs, [&]() { cl_await(S, S.col, parity); },
+                [&](int i) { return Pre{__ldg(e.dr + i), __ldg(e.rl + i), __ldg(e.ru + i), yp[i]}; },
+                [&](int i, double ax, const Pre& p, int first, int) {
+                    if (!first) e.row(i, ax, p);
+                });
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sum[4 + q] = e.q[q];
+        }
+
+        // sums: lanes, then warps, then ranks, in order (sum[7] is a maximum)
+#pragma unroll
+        for (int q = 0; q < kClSums; ++q) {
+            const double v = q == 7 ? warp_max(sum[q]) : warp_sum(sum[q]);
+            if ((tid & 31) == 0) S.warp[tid >> 5][q] = v;
+        }
+        __syncthreads();
+        if (tid < kClSums) {
+            double v = 0.0;
+            for (int k = 0; k < kClWarps; ++k) v = tid == 7 ? fmax(v, S.warp[k][tid]) : v + S.warp[k][tid];
+            cl_store(unsigned(__cvta_generic_to_shared(&S.rank[rank][tid])), 0, v);
+        }
+    }
+    // every rank learns of a failure
+    if (tid < C) cl_store(unsigned(__cvta_generic_to_shared(&S.fail[rank])), unsigned(tid), S.failed ? 1.0 : 0.0);
+    cl_sync();
+    bool failed = false;
+    for (int r = 0; r < C; ++r) failed |= S.fail[r] != 0.0;
+    if (rank == 0 && tid == 0) {
         if (failed) {
             st->done = 1;
             st->status = 14;  // NIR_STATUS_INTERNAL_ERROR
+        } else {
+            double t[kClSums];
+            for (int q = 0; q < kClSums; ++q) {
+                t[q] = 0.0;
+                for (int r = 0; r < C; ++r) t[q] = q == 7 ? fmax(t[q], S.rank[r][q]) : t[q] + S.rank[r][q];
+            }
+            const CtlSums s{t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10], t[11]};
+            control_update(a.ctl, st, s, a.bnorm ? a.bnorm[inst] : st->bnorm, a.cnorm ? a.cnorm[inst] : st->cnorm,
+                           a.offset ? a.offset[inst] : a.ctl.offset, a.ctl.hist);
         }
         __threadfence();
     }
+    if (failed)
+        for (const long long t0 = clock64(); clock64() - t0 < kClSettleCycles;) __nanosleep(1000);
     cl_sync();
 }
 
@@ -574,7 +594,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_chunk(const __grid_co
             R.ns = ns;
             R.sl = int(reinterpret_cast<unsigned char*>(d) - cl_smem);
             R.p0 = size_t(s.off[inst]) + size_t(s.bound[bi]);
-            R.bytes = unsigned(s.bytes[ri]);
+            R.bytes = unsigned(s.bytes[ri]) + (rank == 0 ? unsigned(a.lost) : 0u);
             R.bulk = s.bulk[ri];
             R.seg_bytes = 8u * unsigned((R.n + 1) & ~1);
         }
@@ -672,6 +692,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_chunk(const __grid_co
         else cl_primal<RES, TV, true>(S, ys, par, a.v.xp + S.col.p0, w, halpern, C, sp);
         if (it < K - 1) cl_dual<RES, TV, false>(S, xs, par, nullptr, w, halpern, C, sd);
         else cl_dual<RES, TV, true>(S, xs, par, a.v.yp + S.row.p0, w, halpern, C, sd);
+        if (S.stop) break;
     }
     cl_check<RES, TV>(a, S, xs, ys, unsigned(K) & 1u, rank, inst, st, sp[0], sp[1], sd[0], sd[1]);
 
