@@ -38,6 +38,7 @@
 #include "k_batch.cuh"
 #include "k_cluster.cuh"
 #include "cluster_plan.hpp"
+#include "grown.hpp"
 #include "nir_pdhg.h"
 
 namespace {
@@ -342,10 +343,8 @@ struct nir_pdhg {
     // objective's offset), and their partial sums and results (dd_sums)
     int *one_row = nullptr, *one_col = nullptr;
     double* one_offset = nullptr;
-    nir::vfy::DD* dd_part = nullptr;
-    size_t dd_len = 0;
-    double* dd_out = nullptr;
-    size_t dd_out_len = 0;
+    nir::Grown<nir::vfy::DD> dd_part;
+    nir::Grown<double> dd_out;
     int cluster_size = -1;                 // its cluster size: 0 = not in clusters, -1 = not decided yet
     const double* last_x = nullptr;  // the point the last solve returned, still on the device (null before one)
     // the engine's row order: internal row k is the caller's row
@@ -1518,23 +1517,14 @@ template <class F>
 void dd_sums(nir_pdhg* h, int count, int Q, const double* base, double* out, F&& launch) {
     // enough CTAs for the device, at most 128 per instance
     const int G = std::max(1, std::min(128, 4 * h->sms / count));
-    const size_t need = size_t(count) * G * Q;
-    if (need > h->dd_len) {
-        h->release(h->dd_part);
-        h->dd_part = h->alloc<nir::vfy::DD>(need);
-        h->dd_len = need;
-    }
     const size_t res = size_t(count) * Q;
-    if (res > h->dd_out_len) {
-        h->release(h->dd_out);
-        h->dd_out = h->alloc<double>(res);
-        h->dd_out_len = res;
-    }
-    launch(G, h->dd_part);
-    nir::k_dd_finish<<<grid_for((long long)res), nir::kBlock, 0, h->stream>>>(count, G, Q, h->dd_part, base, h->dd_out);
+    h->dd_part.ensure(*h, res * G);
+    h->dd_out.ensure(*h, res);
+    launch(G, h->dd_part.p);
+    nir::k_dd_finish<<<grid_for((long long)res), nir::kBlock, 0, h->stream>>>(count, G, Q, h->dd_part.p, base, h->dd_out.p);
     NIR_LAUNCHED();
     h->launches += 2;
-    d2h(h, out, h->dd_out, res * sizeof(double));
+    d2h(h, out, h->dd_out.p, res * sizeof(double));
 }
 
 // The norms of each instance: ||c||, ||c scaled||, ||b||, ||b scaled||

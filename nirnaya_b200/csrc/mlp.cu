@@ -33,6 +33,7 @@
 #include <string>
 #include <vector>
 
+#include "grown.hpp"
 #include "nir_mlp.h"
 
 namespace {
@@ -693,34 +694,28 @@ struct nir_mlp {
     std::vector<Layer> layers;
     float* outw = nullptr;  // per-output loss weights
     float outw_sum = 0.f;
-    // activations for up to cap_rows samples
-    int cap_rows = 0;
-    bf16* x = nullptr;
-    std::vector<bf16*> act;  // hidden outputs
-    float* pred = nullptr;
-    float* tgt = nullptr;
-    bf16* dy = nullptr;
-    std::vector<bf16*> grad;            // masked gradients at the hidden outputs
-    bf16* ep_x = nullptr;               // the epoch's samples in its order
-    float* ep_y = nullptr;
-    int ep_len = 0;
-    float2* bc = nullptr;               // Adam's bias corrections of the epoch's steps
-    int bc_len = 0;
-    int cap_back = 0;
-    float* colsum_ws = nullptr;  // every layer's chunks, one after another
-    float* part = nullptr;       // loss partials, loss_blocks() per step
-    size_t part_len = 0;
-    float* losses = nullptr;  // device loss per step
-    int losses_len = 0;
+    // activations of a forward pass
+    nir::Grown<bf16> x;
+    std::vector<nir::Grown<bf16>> act;  // hidden outputs
+    nir::Grown<float> pred;
+    // buffers of a backward pass
+    nir::Grown<float> tgt;
+    nir::Grown<bf16> dy;
+    std::vector<nir::Grown<bf16>> grad;  // masked gradients at the hidden outputs
+    nir::Grown<float> colsum_ws;         // every layer's chunks, one after another
+    nir::Grown<float> part;              // loss partials, loss_blocks() per step
+    nir::Grown<float> losses;            // loss per step
+    nir::Grown<bf16> ep_x;               // the epoch's samples in its order
+    nir::Grown<float> ep_y;
+    nir::Grown<float2> bc;               // Adam's bias corrections of the epoch's steps
     // training set
     int n_data = 0;
-    bf16* data_x = nullptr;
-    float* data_y = nullptr;
-    int* perm = nullptr;
+    nir::Grown<bf16> data_x;
+    nir::Grown<float> data_y;
+    nir::Grown<int> perm;
     int64_t adam_t = 0;
     double us_per_step = 0.0, flops_per_step = 0.0;
-    float* stage = nullptr;  // FP32 staging of uploaded rows, grown on demand
-    size_t stage_len = 0;
+    nir::Grown<float> stage;  // FP32 staging of uploaded rows
     // output map of nir_mlp_predict_device_affine
     bool gemm_ready[8] = {};  // GEMM kernels prepared for launches
     int* fault = nullptr;     // mapped host memory, set if a wait inside a GEMM gives up
@@ -952,36 +947,22 @@ void finish(nir_mlp* h) {
 }
 
 void ensure_rows(nir_mlp* h, int rows) {
-    if (rows <= h->cap_rows) return;
-    for (bf16* p : h->act) h->release(p);
-    for (void* p : {(void*)h->x, (void*)h->pred})
-        if (p) h->release(p);
-    const int din = h->cfg.d_in, dout = h->cfg.d_out;
-    h->x = h->alloc<bf16>((size_t)rows * din);
-    h->act.assign(h->cfg.depth, nullptr);
-    for (auto& a : h->act) a = h->alloc<bf16>((size_t)rows * h->cfg.width);
-    h->pred = h->alloc<float>((size_t)rows * dout);
-    h->cap_rows = rows;
+    h->x.ensure(*h, (size_t)rows * h->cfg.d_in);
+    h->act.resize(size_t(h->cfg.depth));
+    for (auto& a : h->act) a.ensure(*h, (size_t)rows * h->cfg.width);
+    h->pred.ensure(*h, (size_t)rows * h->cfg.d_out);
 }
 
 // The buffers of a backward pass over `rows` samples (a forward pass alone
 // needs none of them).
 void ensure_backward(nir_mlp* h, int rows) {
-    if (rows <= h->cap_back) return;
-    for (bf16* p : h->grad) h->release(p);
-    for (void* p : {(void*)h->tgt, (void*)h->dy, (void*)h->colsum_ws, (void*)h->part})
-        if (p) h->release(p);
-    const int dout = h->cfg.d_out;
-    h->tgt = h->alloc<float>((size_t)rows * dout);
-    h->dy = h->alloc<bf16>((size_t)rows * dout);
-    h->grad.assign(h->cfg.depth, nullptr);
-    for (auto& g : h->grad) g = h->alloc<bf16>((size_t)rows * h->cfg.width);
+    h->tgt.ensure(*h, (size_t)rows * h->cfg.d_out);
+    h->dy.ensure(*h, (size_t)rows * h->cfg.d_out);
+    h->grad.resize(size_t(h->cfg.depth));
+    for (auto& g : h->grad) g.ensure(*h, (size_t)rows * h->cfg.width);
     size_t cols = 0;
     for (auto& ly : h->layers) cols += (size_t)ly.out;
-    h->colsum_ws = h->alloc<float>((size_t)((rows + kColChunkRows - 1) / kColChunkRows) * cols);
-    h->part = nullptr;
-    h->part_len = 0;
-    h->cap_back = rows;
+    h->colsum_ws.ensure(*h, (size_t)((rows + kColChunkRows - 1) / kColChunkRows) * cols);
 }
 
 void forward(nir_mlp* h, int rows, const bf16* in) {
@@ -989,11 +970,11 @@ void forward(nir_mlp* h, int rows, const bf16* in) {
     for (int l = 0; l < L; ++l) {
         auto& ly = h->layers[l];
         if (l + 1 < L) {
-            gemm(h, true, true, in, ly.in, ly.Wb, ly.in, rows, ly.out, ly.in, EPI_BIAS_RELU_BF16, ly.b, h->act[l],
+            gemm(h, true, true, in, ly.in, ly.Wb, ly.in, rows, ly.out, ly.in, EPI_BIAS_RELU_BF16, ly.b, h->act[l].p,
                  nullptr, ly.out, nullptr, 0);
-            in = h->act[l];
+            in = h->act[l].p;
         } else {
-            gemm(h, true, true, in, ly.in, ly.Wb, ly.in, rows, ly.out, ly.in, EPI_BIAS_F32, ly.b, nullptr, h->pred,
+            gemm(h, true, true, in, ly.in, ly.Wb, ly.in, rows, ly.out, ly.in, EPI_BIAS_F32, ly.b, nullptr, h->pred.p,
                  ly.out, nullptr, 0);
         }
     }
@@ -1001,17 +982,10 @@ void forward(nir_mlp* h, int rows, const bf16* in) {
 
 unsigned loss_blocks(const nir_mlp* h, int rows) { return grid1d((size_t)rows * h->cfg.d_out, 1024); }
 
-void ensure_parts(nir_mlp* h, size_t len) {
-    if (len <= h->part_len) return;
-    if (h->part) h->release(h->part);
-    h->part = h->alloc<float>(len);
-    h->part_len = len;
-}
-
 // The losses of `steps` steps of `rows` samples from their partials.
 void finish_losses(nir_mlp* h, int rows, int steps) {
     const float denom = float(rows) * std::max(h->outw_sum, 1.f);
-    k_sum_partials<<<unsigned(steps), 256, 0, h->stream>>>(int(loss_blocks(h, rows)), h->part, 1.f / denom, h->losses);
+    k_sum_partials<<<unsigned(steps), 256, 0, h->stream>>>(int(loss_blocks(h, rows)), h->part.p, 1.f / denom, h->losses.p);
     MLP_LAUNCHED();
 }
 
@@ -1020,7 +994,7 @@ int colsum_chunks(int rows) { return (rows + kColChunkRows - 1) / kColChunkRows;
 float* colsum_of(nir_mlp* h, int rows, int l) {
     size_t o = 0;
     for (int k = 0; k < l; ++k) o += (size_t)h->layers[k].out;
-    return h->colsum_ws + o * (size_t)colsum_chunks(rows);
+    return h->colsum_ws.p + o * (size_t)colsum_chunks(rows);
 }
 
 // Loss partials (of step `slot`) and dY, the gradients down the layers, then
@@ -1032,21 +1006,21 @@ void backward(nir_mlp* h, int rows, const bf16* x, const float* tgt, int slot) {
     const int dout = h->cfg.d_out;
     const float denom = float(rows) * std::max(h->outw_sum, 1.f);
     const unsigned gb = loss_blocks(h, rows);
-    launch_early(h, k_loss, dim3(gb), 256, 0, 1, rows, dout, (const float*)h->pred, tgt, (const float*)h->outw,
-                 2.f / denom, h->dy, h->part + (size_t)slot * gb);
+    launch_early(h, k_loss, dim3(gb), 256, 0, 1, rows, dout, (const float*)h->pred.p, tgt, (const float*)h->outw,
+                 2.f / denom, h->dy.p, h->part.p + (size_t)slot * gb);
     const int L = int(h->layers.size());
-    auto grad_of = [&](int l) { return l == L - 1 ? h->dy : h->grad[l]; };
+    auto grad_of = [&](int l) { return l == L - 1 ? h->dy.p : h->grad[l].p; };
     for (int l = L - 1; l > 0; --l) {
         auto& ly = h->layers[l];
         // d(in) = g W, masked by the ReLU of the layer below
-        gemm(h, true, false, grad_of(l), ly.out, ly.Wb, ly.in, rows, ly.in, ly.out, EPI_MASK_BF16, nullptr, h->grad[l - 1],
-             nullptr, ly.in, h->act[l - 1], ly.in);
+        gemm(h, true, false, grad_of(l), ly.out, ly.Wb, ly.in, rows, ly.in, ly.out, EPI_MASK_BF16, nullptr, h->grad[l - 1].p,
+             nullptr, ly.in, h->act[l - 1].p, ly.in);
     }
     GemmArgs gs[GROUP_MAX];
     ColsumTable ct{};
     for (int l = 0; l < L; ++l) {
         auto& ly = h->layers[l];
-        const bf16* in = (l == 0) ? x : h->act[l - 1];
+        const bf16* in = (l == 0) ? x : h->act[l - 1].p;
         // dW = g^T in   (out x in), contraction over the rows
         gs[l] = gemm_args(h, false, false, grad_of(l), ly.out, in, ly.in, ly.out, ly.in, rows, EPI_F32, nullptr, nullptr,
                           ly.gW, ly.in, nullptr, 0);
@@ -1073,7 +1047,7 @@ void adam(nir_mlp* h, int rows, int slot) {
     }
     t.count = L;
     t.chunks = colsum_chunks(rows);
-    t.bc = h->bc + slot;
+    t.bc = h->bc.p + slot;
     t.lr = h->cfg.lr;
     t.b1 = h->cfg.beta1;
     t.b2 = h->cfg.beta2;
@@ -1082,24 +1056,13 @@ void adam(nir_mlp* h, int rows, int slot) {
     MLP_LAUNCHED();
 }
 
-void ensure_losses(nir_mlp* h, int n) {
-    if (n <= h->losses_len) return;
-    h->release(h->losses);
-    h->losses = h->alloc<float>(n);
-    h->losses_len = n;
-}
-
 // Host FP32 rows -> device BF16, through a staging buffer that grows on
 // demand and is kept (no allocation per call once it is large enough).
 void upload_rows(nir_mlp* h, const float* x, int rows, bf16* dst, int cols) {
     const size_t len = (size_t)rows * cols;
-    if (len > h->stage_len) {
-        if (h->stage) h->release(h->stage);
-        h->stage = h->alloc<float>(len);
-        h->stage_len = len;
-    }
-    MLP_CUDA(cudaMemcpyAsync(h->stage, x, len * sizeof(float), cudaMemcpyHostToDevice, h->stream));
-    k_to_bf16<<<grid1d(len), 256, 0, h->stream>>>(len, h->stage, dst);
+    float* const stage = h->stage.ensure(*h, len);
+    MLP_CUDA(cudaMemcpyAsync(stage, x, len * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    k_to_bf16<<<grid1d(len), 256, 0, h->stream>>>(len, stage, dst);
     MLP_LAUNCHED();
     finish(h);
 }
@@ -1161,7 +1124,7 @@ int nir_mlp_create(const nir_mlp_config* cfg, int device, nir_mlp** out) {
         std::vector<float> ones(cfg->d_out, 1.f);
         MLP_CUDA(cudaMemcpyAsync(h->outw, ones.data(), ones.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
         h->outw_sum = float(cfg->d_out);
-        ensure_losses(h.get(), 1024);
+        h->losses.ensure(*h, 1024);
         finish(h.get());
     } catch (const std::invalid_argument& e) {
         return fail(e, true);
@@ -1253,20 +1216,18 @@ int nir_mlp_set_data(nir_mlp* h, const float* x, const float* targets, int32_t n
     }
     try {
         MLP_CUDA(cudaSetDevice(h->device));
-        h->release(h->data_x);
-        h->release(h->data_y);
-        h->release(h->perm);
         const int din = h->cfg.d_in, dout = h->cfg.d_out;
-        h->data_x = h->alloc<bf16>((size_t)n * din);
-        h->data_y = h->alloc<float>((size_t)n * dout);
-        h->perm = h->alloc<int>(n);
+        h->n_data = 0;  // none until the new one is complete
+        h->data_x.renew(*h, (size_t)n * din);
+        h->data_y.renew(*h, (size_t)n * dout);
+        h->perm.renew(*h, size_t(n));
         // in slices so that the FP32 staging buffer stays small
         const int slice = std::max(1, int((size_t(256) << 20) / (sizeof(float) * din)));
         for (int r = 0; r < n; r += slice) {
             const int k = std::min(slice, n - r);
-            upload_rows(h, x + (size_t)r * din, k, h->data_x + (size_t)r * din, din);
+            upload_rows(h, x + (size_t)r * din, k, h->data_x.p + (size_t)r * din, din);
         }
-        MLP_CUDA(cudaMemcpyAsync(h->data_y, targets, (size_t)n * dout * sizeof(float), cudaMemcpyHostToDevice,
+        MLP_CUDA(cudaMemcpyAsync(h->data_y.p, targets, (size_t)n * dout * sizeof(float), cudaMemcpyHostToDevice,
                                  h->stream));
         finish(h);
         h->n_data = n;
@@ -1290,24 +1251,15 @@ int nir_mlp_train(nir_mlp* h, int32_t epochs, int32_t batch, float* epoch_loss) 
         ensure_rows(h, batch);
         ensure_backward(h, batch);
         const int steps = h->n_data / batch, used = steps * batch;
-        ensure_losses(h, steps);
-        ensure_parts(h, (size_t)steps * loss_blocks(h, batch));
-        if (used > h->ep_len) {
-            h->release(h->ep_x);
-            h->release(h->ep_y);
-            h->ep_x = h->alloc<bf16>((size_t)used * h->cfg.d_in);
-            h->ep_y = h->alloc<float>((size_t)used * h->cfg.d_out);
-            h->ep_len = used;
-        }
+        h->losses.ensure(*h, size_t(steps));
+        h->part.ensure(*h, (size_t)steps * loss_blocks(h, batch));
+        h->ep_x.ensure(*h, (size_t)used * h->cfg.d_in);
+        h->ep_y.ensure(*h, (size_t)used * h->cfg.d_out);
         std::mt19937_64 rng(h->cfg.seed ^ 0x5bd1e995ULL ^ (uint64_t)h->adam_t);
         std::vector<int> perm(h->n_data);
         std::vector<float> lossv(steps);
         std::vector<float2> bcv(steps);
-        if (steps > h->bc_len) {
-            if (h->bc) h->release(h->bc);
-            h->bc = h->alloc<float2>(steps);
-            h->bc_len = steps;
-        }
+        h->bc.ensure(*h, size_t(steps));
         cudaEvent_t e0, e1;
         MLP_CUDA(cudaEventCreate(&e0));
         MLP_CUDA(cudaEventCreate(&e1));
@@ -1316,30 +1268,30 @@ int nir_mlp_train(nir_mlp* h, int32_t epochs, int32_t batch, float* epoch_loss) 
         for (int ep = 0; ep < epochs; ++ep) {
             for (int i = 0; i < h->n_data; ++i) perm[i] = i;
             std::shuffle(perm.begin(), perm.end(), rng);
-            MLP_CUDA(cudaMemcpyAsync(h->perm, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice,
+            MLP_CUDA(cudaMemcpyAsync(h->perm.p, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice,
                                      h->stream));
             MLP_CUDA(cudaEventRecord(e0, h->stream));
             // the epoch's samples in its order, at once
-            k_gather_rows<bf16><<<grid1d((size_t)used * h->cfg.d_in), 256, 0, h->stream>>>(h->perm, used, h->cfg.d_in,
-                                                                                           h->data_x, h->ep_x);
-            k_gather_rows<float><<<grid1d((size_t)used * h->cfg.d_out), 256, 0, h->stream>>>(h->perm, used, h->cfg.d_out,
-                                                                                             h->data_y, h->ep_y);
+            k_gather_rows<bf16><<<grid1d((size_t)used * h->cfg.d_in), 256, 0, h->stream>>>(h->perm.p, used, h->cfg.d_in,
+                                                                                           h->data_x.p, h->ep_x.p);
+            k_gather_rows<float><<<grid1d((size_t)used * h->cfg.d_out), 256, 0, h->stream>>>(h->perm.p, used, h->cfg.d_out,
+                                                                                             h->data_y.p, h->ep_y.p);
             MLP_LAUNCHED();
             for (int s = 0; s < steps; ++s) {
                 h->adam_t += 1;
                 bcv[size_t(s)] = make_float2(1.f - std::pow(h->cfg.beta1, float(h->adam_t)),
                                              1.f - std::pow(h->cfg.beta2, float(h->adam_t)));
             }
-            MLP_CUDA(cudaMemcpyAsync(h->bc, bcv.data(), bcv.size() * sizeof(float2), cudaMemcpyHostToDevice, h->stream));
+            MLP_CUDA(cudaMemcpyAsync(h->bc.p, bcv.data(), bcv.size() * sizeof(float2), cudaMemcpyHostToDevice, h->stream));
             for (int s = 0; s < steps; ++s) {
-                const bf16* x = h->ep_x + (size_t)s * batch * h->cfg.d_in;
+                const bf16* x = h->ep_x.p + (size_t)s * batch * h->cfg.d_in;
                 forward(h, batch, x);
-                backward(h, batch, x, h->ep_y + (size_t)s * batch * h->cfg.d_out, s);
+                backward(h, batch, x, h->ep_y.p + (size_t)s * batch * h->cfg.d_out, s);
                 adam(h, batch, s);
             }
             finish_losses(h, batch, steps);
             MLP_CUDA(cudaEventRecord(e1, h->stream));
-            MLP_CUDA(cudaMemcpyAsync(lossv.data(), h->losses, steps * sizeof(float), cudaMemcpyDeviceToHost,
+            MLP_CUDA(cudaMemcpyAsync(lossv.data(), h->losses.p, steps * sizeof(float), cudaMemcpyDeviceToHost,
                                      h->stream));
             finish(h);
             float ms = 0.f;
@@ -1378,9 +1330,9 @@ int nir_mlp_predict(nir_mlp* h, const float* x, int32_t n, float* y) {
         ensure_rows(h, chunk);
         for (int r = 0; r < n; r += chunk) {
             const int k = std::min(chunk, n - r);  // a multiple of 8
-            upload_rows(h, x + (size_t)r * h->cfg.d_in, k, h->x, h->cfg.d_in);
-            forward(h, k, h->x);
-            MLP_CUDA(cudaMemcpyAsync(y + (size_t)r * h->cfg.d_out, h->pred, (size_t)k * h->cfg.d_out * sizeof(float),
+            upload_rows(h, x + (size_t)r * h->cfg.d_in, k, h->x.p, h->cfg.d_in);
+            forward(h, k, h->x.p);
+            MLP_CUDA(cudaMemcpyAsync(y + (size_t)r * h->cfg.d_out, h->pred.p, (size_t)k * h->cfg.d_out * sizeof(float),
                                      cudaMemcpyDeviceToHost, h->stream));
             finish(h);
         }
@@ -1402,10 +1354,10 @@ int nir_mlp_predict_device(nir_mlp* h, const float* x_dev, int32_t n, float* y) 
         for (int r = 0; r < n; r += chunk) {
             const int k = std::min(chunk, n - r);
             const size_t len = (size_t)k * h->cfg.d_in;
-            k_to_bf16<<<grid1d(len), 256, 0, h->stream>>>(len, x_dev + (size_t)r * h->cfg.d_in, h->x);
+            k_to_bf16<<<grid1d(len), 256, 0, h->stream>>>(len, x_dev + (size_t)r * h->cfg.d_in, h->x.p);
             MLP_LAUNCHED();
-            forward(h, k, h->x);
-            MLP_CUDA(cudaMemcpyAsync(y + (size_t)r * h->cfg.d_out, h->pred, (size_t)k * h->cfg.d_out * sizeof(float),
+            forward(h, k, h->x.p);
+            MLP_CUDA(cudaMemcpyAsync(y + (size_t)r * h->cfg.d_out, h->pred.p, (size_t)k * h->cfg.d_out * sizeof(float),
                                      cudaMemcpyDeviceToHost, h->stream));
             finish(h);
         }
@@ -1462,10 +1414,10 @@ int nir_mlp_predict_device_affine(nir_mlp* h, const float* x_dev, int32_t n, con
         for (int r = 0; r < n; r += chunk) {
             const int k = std::min(chunk, n - r);
             const size_t len = (size_t)k * h->cfg.d_in;
-            k_to_bf16<<<grid1d(len), 256, 0, h->stream>>>(len, x_dev + (size_t)r * h->cfg.d_in, h->x);
+            k_to_bf16<<<grid1d(len), 256, 0, h->stream>>>(len, x_dev + (size_t)r * h->cfg.d_in, h->x.p);
             MLP_LAUNCHED();
-            forward(h, k, h->x);
-            k_affine_out<<<unsigned((k + 255) / 256), 256, 0, h->stream>>>(k, r, h->pred, h->cfg.d_out, h->aff_col,
+            forward(h, k, h->x.p);
+            k_affine_out<<<unsigned((k + 255) / 256), 256, 0, h->stream>>>(k, r, h->pred.p, h->cfg.d_out, h->aff_col,
                                                                           h->aff_lo, h->aff_hi, h->aff_scale,
                                                                           h->aff_shift, h->aff_out);
             MLP_LAUNCHED();
@@ -1487,19 +1439,20 @@ int nir_mlp_gradients(nir_mlp* h, const float* x, const float* targets, int32_t 
         MLP_CUDA(cudaSetDevice(h->device));
         ensure_rows(h, n);
         ensure_backward(h, n);
-        ensure_parts(h, loss_blocks(h, n));
-        upload_rows(h, x, n, h->x, h->cfg.d_in);
-        MLP_CUDA(cudaMemcpyAsync(h->tgt, targets, (size_t)n * h->cfg.d_out * sizeof(float), cudaMemcpyHostToDevice,
+        h->losses.ensure(*h, 1);
+        h->part.ensure(*h, loss_blocks(h, n));
+        upload_rows(h, x, n, h->x.p, h->cfg.d_in);
+        MLP_CUDA(cudaMemcpyAsync(h->tgt.p, targets, (size_t)n * h->cfg.d_out * sizeof(float), cudaMemcpyHostToDevice,
                                  h->stream));
-        forward(h, n, h->x);
-        backward(h, n, h->x, h->tgt, 0);
+        forward(h, n, h->x.p);
+        backward(h, n, h->x.p, h->tgt.p, 0);
         finish_losses(h, n, 1);
         for (size_t l = 0; l < h->layers.size(); ++l)
             k_colsum_final<<<(h->layers[l].out + 255) / 256, 256, 0, h->stream>>>(
                 colsum_chunks(n), h->layers[l].out, colsum_of(h, n, int(l)), h->layers[l].gb);
         MLP_LAUNCHED();
         float lv = 0.f;
-        MLP_CUDA(cudaMemcpyAsync(&lv, h->losses, sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+        MLP_CUDA(cudaMemcpyAsync(&lv, h->losses.p, sizeof(float), cudaMemcpyDeviceToHost, h->stream));
         if (grads) {
             size_t o = 0;
             for (auto& ly : h->layers) {
