@@ -38,6 +38,7 @@
 #include "k_batch.cuh"
 #include "k_cluster.cuh"
 #include "cluster_plan.hpp"
+#include "dev_arena.hpp"
 #include "grown.hpp"
 #include "nir_pdhg.h"
 
@@ -45,17 +46,8 @@ namespace {
 
 thread_local std::string g_err;
 
-struct CudaError : std::runtime_error {
-    using std::runtime_error::runtime_error;
-};
-
-#define NIR_CUDA(call)                                                                                  \
-    do {                                                                                                \
-        cudaError_t e_ = (call);                                                                        \
-        if (e_ != cudaSuccess)                                                                          \
-            throw CudaError(std::string(#call) + ": " + cudaGetErrorString(e_) + " (" __FILE__ ":" +    \
-                            std::to_string(__LINE__) + ")");                                            \
-    } while (0)
+using nir::CudaError;
+using nir::DevArena;
 
 #define NIR_LAUNCHED() NIR_CUDA(cudaGetLastError())
 
@@ -100,70 +92,6 @@ inline DD dd_add_prod(DD a, double x, double y) {
     p.lo = std::fma(x, y, -p.hi);
     return dd_add(a, p);
 }
-
-// Device memory in chunks that allocations are carved from: large ones
-// reserved beforehand for what is known to come, small ones on demand, and
-// a block of its own for what is large and fits none.  A cudaMalloc takes
-// 20 us below 64 KB, 70 at 300 KB and 330 from 2 MB on, its cudaFree as
-// long, and a handle holds about 60 arrays.
-struct DevArena {
-    static constexpr size_t kAlign = 256, kOwn = size_t(1) << 20, kSmallChunk = size_t(128) << 10;
-    static size_t aligned(size_t bytes) { return (std::max<size_t>(1, bytes) + kAlign - 1) / kAlign * kAlign; }
-    struct Block {
-        char* p;
-        size_t size, used;
-        bool carved;  // a chunk; false: one allocation
-    };
-    std::vector<Block> blocks;
-    int cur = -1;  // the chunk being carved
-    long long bytes = 0;
-
-    char* block(size_t size, bool carved) {
-        blocks.reserve(blocks.size() + 1);
-        void* p = nullptr;
-        NIR_CUDA(cudaMalloc(&p, size));
-        blocks.push_back({static_cast<char*>(p), size, 0, carved});
-        bytes += (long long)size;
-        return static_cast<char*>(p);
-    }
-    void reserve(size_t size) {
-        block(size, true);
-        cur = int(blocks.size()) - 1;
-    }
-    void* alloc(size_t size) {
-        size = aligned(size);
-        if (cur < 0 || blocks[size_t(cur)].size - blocks[size_t(cur)].used < size) {
-            if (size >= kOwn) return block(size, false);
-            reserve(std::max(size, kSmallChunk));
-        }
-        Block& c = blocks[size_t(cur)];
-        char* p = c.p + c.used;
-        c.used += size;
-        return p;
-    }
-    // Frees a block of its own; a carved allocation stays with its chunk.
-    void release(void* p) {
-        for (size_t i = 0; i < blocks.size(); ++i)
-            if (blocks[i].p == p && !blocks[i].carved) {
-                cudaFree(p);
-                bytes -= (long long)blocks[i].size;
-                blocks.erase(blocks.begin() + long(i));
-                if (cur > int(i)) --cur;
-                return;
-            }
-    }
-    // Scratch carved last is given back by rewinding to the mark before it.
-    size_t mark() const { return cur < 0 ? 0 : blocks[size_t(cur)].used; }
-    void rewind(size_t m) {
-        if (cur >= 0) blocks[size_t(cur)].used = m;
-    }
-    void clear() {
-        for (auto& b : blocks) cudaFree(b.p);
-        blocks.clear();
-        cur = -1;
-        bytes = 0;
-    }
-};
 
 // The per-orientation layout choice of a solve.
 struct LayChoice {
@@ -701,7 +629,7 @@ void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
     R.v_orig = h->allocz<double>(nnz);
     R.v64 = h->allocz<double>(nnz);
     R.v32 = h->allocz<float>(nnz);
-    const size_t scratch_mark = h->mem.mark();
+    const DevArena::Mark scratch_mark = h->mem.mark();
     long long* d_start = h->alloc<long long>(n + 1);
     NIR_CUDA(cudaMemcpyAsync(d_start, lp->col_start, (n + 1) * sizeof(long long), cudaMemcpyHostToDevice, s));
     NIR_CUDA(cudaMemcpyAsync(T.ci, lp->row_index, nnz * sizeof(int), cudaMemcpyHostToDevice, s));
