@@ -9,7 +9,6 @@
 #include <atomic>
 #include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -37,7 +36,7 @@ void cl_for_each(int n, int threads, F&& f) {
     for (int t = 1; t < threads; ++t) {
         try {
             pool.emplace_back(work);
-        } catch (const std::system_error&) {
+        } catch (const std::exception&) {  // no thread, or no memory for one
             break;
         }
     }
