@@ -60,7 +60,8 @@ def build_engine(force: bool = False, verbose: bool = False) -> str:
 
 def build_mlp(force: bool = False, verbose: bool = False) -> str:
     target = os.path.join(HERE, "libnir_mlp.so")
-    srcs = [os.path.join(CSRC, "mlp.cu"), os.path.join(CSRC, "grown.hpp"), os.path.join(INC, "nir_mlp.h")]
+    srcs = [os.path.join(CSRC, "mlp.cu"), os.path.join(CSRC, "grown.hpp"), os.path.join(CSRC, "mapped_host.hpp"),
+            os.path.join(INC, "nir_mlp.h")]
     if force or _stale(target, srcs):
         cmd = [_nvcc(), *NVCC_FLAGS, srcs[0], "-o", target]
         if verbose:

@@ -40,6 +40,7 @@
 #include "cluster_plan.hpp"
 #include "dev_arena.hpp"
 #include "grown.hpp"
+#include "mapped_host.hpp"
 #include "nir_pdhg.h"
 
 namespace {
@@ -168,41 +169,10 @@ struct ClusterPlan;  // engine_cluster.cuh
 
 namespace {
 
-// Status rings in host-mapped memory, kept for the next handle: taking one
-// from the driver costs 1 to 3 ms, giving it back 0.4.  At most kSnapKeep
-// of 8 KB are kept, for the life of the process; any thread may take and
-// give (a ring belongs to one handle in between, whose stream has ended
-// when it is given back).
-constexpr size_t kSnapKeep = 16;
-std::mutex g_snap_mu;
-std::vector<nir::HostSnap*> g_snap_free;
-
-nir::HostSnap* snap_ring_take() {
-    {
-        std::lock_guard<std::mutex> g(g_snap_mu);
-        if (!g_snap_free.empty()) {
-            nir::HostSnap* r = g_snap_free.back();
-            g_snap_free.pop_back();
-            return r;
-        }
-    }
-    void* p = nullptr;
-    NIR_CUDA(cudaHostAlloc(&p, sizeof(nir::HostSnap) * nir::kSnapRing, cudaHostAllocMapped | cudaHostAllocPortable));
-    return static_cast<nir::HostSnap*>(p);
-}
-
-void snap_ring_put(nir::HostSnap* r) {
-    {
-        std::lock_guard<std::mutex> g(g_snap_mu);
-        if (g_snap_free.size() < kSnapKeep) {
-            try {
-                g_snap_free.push_back(r);
-                return;
-            } catch (const std::bad_alloc&) {
-            }
-        }
-    }
-    cudaFreeHost(r);
+// Status rings, in host memory that kernels write to.
+nir::MappedBlocks& snap_rings() {
+    static auto* const rings = new nir::MappedBlocks(sizeof(nir::HostSnap) * nir::kSnapRing);  // outlives every handle
+    return *rings;
 }
 
 }  // namespace
@@ -321,7 +291,7 @@ struct nir_pdhg {
             if (g.g) cudaGraphDestroy(g.g);
         }
         mem.clear();
-        if (snap.ring) snap_ring_put(snap.ring);
+        if (snap.ring) snap_rings().give(device, snap.ring);
         if (stream) cudaStreamDestroy(stream);
         inner.reset();
     }
@@ -708,7 +678,9 @@ void create_impl(nir_pdhg* h, const nir_lp_view* lp, int device) {
     h->gs_gen = h->allocz<unsigned>(1);
     h->gs_err = h->allocz<int>(1);
     NIR_CUDA(cudaMemsetAsync(h->snap.d_seq, 0, sizeof(long long), s));
-    h->snap.ring = snap_ring_take();
+    void* ring = nullptr;
+    NIR_CUDA(snap_rings().take(h->device, &ring));
+    h->snap.ring = static_cast<nir::HostSnap*>(ring);
     std::memset(h->snap.ring, 0, sizeof(nir::HostSnap) * nir::kSnapRing);
     NIR_CUDA(cudaStreamSynchronize(s));
 }

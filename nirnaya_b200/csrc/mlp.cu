@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "grown.hpp"
+#include "mapped_host.hpp"
 #include "nir_mlp.h"
 
 namespace {
@@ -639,42 +640,10 @@ unsigned grid1d(size_t n, int cap = 148 * 16) {
 // ------------------------------------------------------------ the handle
 
 namespace {
-// Flags in mapped host memory that a kernel sets when one of its waits gives
-// up: the host reads them after a synchronisation at no cost.  A page of them
-// serves the handles of the process, taken on the first use and kept (a
-// pinned allocation for each handle took 2.5 ms of the 4.4 its creation did);
-// handles beyond the page's flags have their own.
-struct FaultFlags {
-    static constexpr int kFlags = 1024;
-    std::mutex mu;
-    int* page = nullptr;
-    std::vector<int*> spare;
-
-    static int* allocate(int n) {
-        int* p = nullptr;
-        MLP_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), n * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-        return p;
-    }
-    int* take() {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!page) {
-            spare.reserve(kFlags);
-            page = allocate(kFlags);
-            for (int i = 0; i < kFlags; ++i) spare.push_back(page + i);
-        }
-        int* f = spare.empty() ? allocate(1) : spare.back();
-        if (!spare.empty()) spare.pop_back();
-        *f = 0;
-        return f;
-    }
-    void give(int* f) {
-        std::lock_guard<std::mutex> lock(mu);
-        if (f >= page && f < page + kFlags) spare.push_back(f);
-        else cudaFreeHost(f);
-    }
-};
-FaultFlags& fault_flags() {
-    static FaultFlags* flags = new FaultFlags;  // outlives every handle
+// A flag for each handle in host memory, which a kernel sets when one of its
+// waits gives up: the host reads it after a synchronisation at no cost.
+nir::MappedBlocks& fault_flags() {
+    static auto* const flags = new nir::MappedBlocks(sizeof(int));  // outlives every handle
     return *flags;
 }
 }  // namespace
@@ -742,7 +711,7 @@ struct nir_mlp {
     ~nir_mlp() {
         cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
-        if (fault) fault_flags().give(fault);
+        if (fault) fault_flags().give(device, fault);
         for (void* p : allocs)
             if (p) cudaFree(p);
         if (stream) cudaStreamDestroy(stream);
@@ -1119,7 +1088,10 @@ int nir_mlp_create(const nir_mlp_config* cfg, int device, nir_mlp** out) {
             MLP_LAUNCHED();
             h->layers.push_back(ly);
         }
-        h->fault = fault_flags().take();
+        void* flag = nullptr;
+        MLP_CUDA(fault_flags().take(device, &flag));
+        h->fault = static_cast<int*>(flag);
+        *h->fault = 0;
         h->outw = h->alloc<float>(cfg->d_out);
         std::vector<float> ones(cfg->d_out, 1.f);
         MLP_CUDA(cudaMemcpyAsync(h->outw, ones.data(), ones.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
