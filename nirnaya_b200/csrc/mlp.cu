@@ -490,7 +490,8 @@ __device__ __forceinline__ float block_sum_f(float v, float* sh) {
 }
 
 // dY = scale * w * (pred - target) (BF16) and per-block sums of w*(pred-target)^2.
-__global__ void k_loss(int rows, int cols, const float* __restrict__ pred, const float* __restrict__ tgt,
+// (pred is still being written when an early launch starts: not restrict.)
+__global__ void k_loss(int rows, int cols, const float* pred, const float* __restrict__ tgt,
                        const float* __restrict__ w, float scale, bf16* __restrict__ dy, float* __restrict__ part) {
     __shared__ float sh[32];
     const size_t total = (size_t)rows * cols;
@@ -559,7 +560,8 @@ __global__ void __launch_bounds__(256) k_colsum_part(const __grid_constant__ Col
     t.part[l][(size_t)z * cols + c0 + c] = s;
 }
 
-__device__ __forceinline__ float colsum_total(int chunks, int cols, int c, const float* __restrict__ part) {
+// (part: not restrict, k_adam starts while it is written)
+__device__ __forceinline__ float colsum_total(int chunks, int cols, int c, const float* part) {
     float s = 0.f;
     for (int z = 0; z < chunks; ++z) s += part[(size_t)z * cols + c];
     return s;
