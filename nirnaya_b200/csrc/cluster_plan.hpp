@@ -9,6 +9,7 @@
 #include <atomic>
 #include <exception>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -170,6 +171,25 @@ inline void cl_build_side(const std::vector<int>& off, const std::vector<int>& r
     for (int i = 0; i < count; ++i) {
         s.slices.insert(s.slices.end(), sl[size_t(i)].begin(), sl[size_t(i)].end());
         s.owner.insert(s.owner.end(), own[size_t(i)].begin(), own[size_t(i)].end());
+    }
+}
+
+// C, or the largest smaller cluster that the device can hold; 0 when it can
+// hold none.  clusters(C) says how many of size C it holds at once.
+template <class F>
+int cl_size_held(int C, F&& clusters) {
+    while (C > 0 && clusters(C) <= 0) C /= 2;
+    return C;
+}
+
+// build's plan, or null when there is no memory for it: the per-launch
+// kernels need none.
+template <class Build>
+auto cl_if_memory(Build&& build) -> decltype(build()) {
+    try {
+        return build();
+    } catch (const std::bad_alloc&) {
+        return nullptr;
     }
 }
 

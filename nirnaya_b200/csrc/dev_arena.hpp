@@ -4,8 +4,10 @@
 #include <cuda_runtime_api.h>
 
 #include <algorithm>
+#include <new>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace nir {
@@ -13,13 +15,25 @@ namespace nir {
 struct CudaError : std::runtime_error {
     using std::runtime_error::runtime_error;
 };
+// The device is out of memory: a caller that can do without may go on.
+struct CudaNoMemory : std::bad_alloc {
+    std::string text;
+    explicit CudaNoMemory(std::string t) : text(std::move(t)) {}
+    const char* what() const noexcept override { return text.c_str(); }
+};
 
-#define NIR_CUDA(call)                                                                                  \
-    do {                                                                                                \
-        cudaError_t e_ = (call);                                                                        \
-        if (e_ != cudaSuccess)                                                                          \
-            throw CudaError(std::string(#call) + ": " + cudaGetErrorString(e_) + " (" __FILE__ ":" +    \
-                            std::to_string(__LINE__) + ")");                                            \
+[[noreturn]] inline void cuda_failed(cudaError_t e, const char* call, const char* file, int line) {
+    (void)cudaGetLastError();  // reported here and not by the next launch's check too
+    const std::string t =
+        std::string(call) + ": " + cudaGetErrorString(e) + " (" + file + ":" + std::to_string(line) + ")";
+    if (e == cudaErrorMemoryAllocation) throw CudaNoMemory(t);
+    throw CudaError(t);
+}
+
+#define NIR_CUDA(call)                                                            \
+    do {                                                                          \
+        cudaError_t e_ = (call);                                                  \
+        if (e_ != cudaSuccess) nir::cuda_failed(e_, #call, __FILE__, __LINE__);   \
     } while (0)
 
 // Device memory in chunks that allocations are carved from: large ones

@@ -312,12 +312,14 @@ void cl_launch(nir_pdhg* h, ClusterPlan& P, const nir::CtlArgs& ctl, int K, int 
     h->launches += 1;
 }
 
-// Clusters of C CTAs with `smem` dynamic bytes the device holds at once.
-int cl_resident(int C, size_t smem) {
+// Clusters of C CTAs the device holds at once with all the dynamic shared
+// memory a plan may use (after cl_prepare_kernels; the kernels' registers and
+// static memory are alike): 0 where a GPC has fewer than C SMs for the process.
+int cl_resident(int C) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(C) * 148u);
     cfg.blockDim = dim3(nir::kClThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = kClSmemMax;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = unsigned(C);
@@ -387,13 +389,14 @@ double cl_arrivals(const ClusterPlan& P, int i) {
 
 // The plan a single LP's solve runs on, or null for the per-launch kernels.
 // The cluster is as large as shortens an iteration: 16 CTAs, fewer on an LP
-// whose rows do not fill them.  Built where clusters are faster even with
-// nothing to exchange (below about 85,000 nonzeros), kept where they still
-// are with what the plan exchanges: 2.7 against 5.4 us an iteration on a
-// 60 x 150 LP, 4.8 against 5.9 on a random 2,000 x 5,000 one of 40,000
-// nonzeros, 3.5 against 5.2 on a multiperiod one of 15,000, but 6.3 against
-// 6.3 on one of 126,000 and 10 against 6.9 on a blending LP of 100,000 whose
-// ranks need nearly all entries.
+// whose rows do not fill them or where the device holds none of 16.  Built
+// where clusters are faster even with nothing to exchange (below about
+// 85,000 nonzeros), kept where they still are with what the plan exchanges:
+// 2.7 against 5.4 us an iteration on a 60 x 150 LP, 4.8 against 5.9 on a
+// random 2,000 x 5,000 one of 40,000 nonzeros, 3.5 against 5.2 on a
+// multiperiod one of 15,000, but 6.3 against 6.3 on one of 126,000 and 10
+// against 6.9 on a blending LP of 100,000 whose ranks need nearly all
+// entries.
 ClusterPlan* cl_single(nir_pdhg* h, const nir_pdhg_params& p) {
     if (!cl_takes(h, p) || h->m < 1 || h->n < 1) return nullptr;
     if (h->cluster_size < 0) {
@@ -404,10 +407,15 @@ ClusterPlan* cl_single(nir_pdhg* h, const nir_pdhg_params& p) {
         if (f < 0 && cl_time(nnz, 0.0, C) >= kClMargin * cl_launch_time(nnz)) C = 0;
         if (C > 0) {
             cl_prepare_kernels();
-            int* off = h->alloc<int>(4);
-            const int o[4] = {0, h->m, 0, h->n};
-            h2d(h, off, o, sizeof(o));
-            std::unique_ptr<ClusterPlan> P = cl_build(h, C, {0, h->m}, {0, h->n}, off, off + 2, nullptr, nullptr);
+            const int held = nir::cl_size_held(C, cl_resident);
+            // a size that the caller fixed is not replaced
+            const bool ok = held == C || (f < 0 && held > 0 && cl_time(nnz, 0.0, held) < kClMargin * cl_launch_time(nnz));
+            C = ok ? held : 0;
+        }
+        if (C > 0) {
+            one_instance(h);
+            std::unique_ptr<ClusterPlan> P = nir::cl_if_memory(
+                [&] { return cl_build(h, C, {0, h->m}, {0, h->n}, h->one_row, h->one_col, nullptr, nullptr); });
             if (P && (f >= 0 || cl_time(nnz, cl_arrivals(*P, 0), C) < kClMargin * cl_launch_time(nnz))) {
                 h->cluster = std::move(P);
                 h->cluster_size = C;
@@ -420,8 +428,9 @@ ClusterPlan* cl_single(nir_pdhg* h, const nir_pdhg_params& p) {
 // The plan a batch runs on, or null: the cluster size with the shortest
 // iteration of the whole batch by the times above, the instances dealt to
 // as many clusters as the device holds; the next larger one while an
-// instance does not fit.  A plan may leave out instances that fit no
-// cluster; the per-launch kernels then run those.
+// instance does not fit, or there is no memory for the plan.  A plan may
+// leave out instances that fit no cluster; the per-launch kernels then run
+// those.
 std::unique_ptr<ClusterPlan> cl_batch(nir_pdhg* h, const std::vector<int>& row_off, const std::vector<int>& col_off,
                                       const int* d_row_off, const int* d_col_off, const int* d_row_inst,
                                       const int* d_col_inst) {
@@ -435,7 +444,8 @@ std::unique_ptr<ClusterPlan> cl_batch(nir_pdhg* h, const std::vector<int>& row_o
     } else {
         double best = 1e300;
         for (int k = 0; k < 5; ++k) {
-            const int slots = std::max(1, cl_resident(sizes[k], kClSmemMax));
+            const int slots = cl_resident(sizes[k]);
+            if (slots < 1) continue;
             double sum = 0.0, mx = 0.0;
             for (int i = 0; i < count; ++i) {
                 const double nnz = double(h->A.h_rp[size_t(row_off[size_t(i) + 1])] - h->A.h_rp[size_t(row_off[size_t(i)])]);
@@ -454,8 +464,11 @@ std::unique_ptr<ClusterPlan> cl_batch(nir_pdhg* h, const std::vector<int>& row_o
     }
     std::unique_ptr<ClusterPlan> best;
     for (int k = first; k < 5; ++k) {
-        std::unique_ptr<ClusterPlan> P =
-            cl_build(h, sizes[k], row_off, col_off, d_row_off, d_col_off, d_row_inst, d_col_inst);
+        std::unique_ptr<ClusterPlan> P;
+        if (cl_resident(sizes[k]) > 0)
+            P = nir::cl_if_memory([&] {
+                return cl_build(h, sizes[k], row_off, col_off, d_row_off, d_col_off, d_row_inst, d_col_inst);
+            });
         if (P && (!best || P->members > best->members)) best = std::move(P);
         if (f > 0 || (best && best->members == count)) break;
     }
