@@ -676,7 +676,7 @@ struct nir_mlp {
     nir::Grown<float> colsum_ws;         // every layer's chunks, one after another
     nir::Grown<float> part;              // loss partials, loss_blocks() per step
     nir::Grown<float> losses;            // loss per step
-    nir::Grown<bf16> ep_x;               // the epoch's samples in its order
+    nir::Grown<bf16> ep_x;               // a piece of the epoch's samples in its order
     nir::Grown<float> ep_y;
     nir::Grown<float2> bc;               // Adam's bias corrections of the epoch's steps
     // training set
@@ -1038,6 +1038,11 @@ void upload_rows(nir_mlp* h, const float* x, int rows, bf16* dst, int cols) {
     finish(h);
 }
 
+// An epoch's samples are gathered into its order in pieces of at most this
+// size (one step at least): a copy of the whole set would take its memory a
+// second time, and a piece that stays in L2 costs two launches in 100 steps.
+constexpr size_t kPieceBytes = size_t(32) << 20;
+
 int fail(const std::exception& e, bool input) {
     g_err = e.what();
     return input ? 2 : 3;
@@ -1224,11 +1229,13 @@ int nir_mlp_train(nir_mlp* h, int32_t epochs, int32_t batch, float* epoch_loss) 
         MLP_CUDA(cudaSetDevice(h->device));
         ensure_rows(h, batch);
         ensure_backward(h, batch);
-        const int steps = h->n_data / batch, used = steps * batch;
+        const int steps = h->n_data / batch;
         h->losses.ensure(*h, size_t(steps));
         h->part.ensure(*h, (size_t)steps * loss_blocks(h, batch));
-        h->ep_x.ensure(*h, (size_t)used * h->cfg.d_in);
-        h->ep_y.ensure(*h, (size_t)used * h->cfg.d_out);
+        const size_t per_step = (size_t)batch * (h->cfg.d_in * sizeof(bf16) + h->cfg.d_out * sizeof(float));
+        const int piece = int(std::min<size_t>(size_t(steps), std::max<size_t>(1, kPieceBytes / per_step)));  // steps
+        h->ep_x.ensure(*h, (size_t)piece * batch * h->cfg.d_in);
+        h->ep_y.ensure(*h, (size_t)piece * batch * h->cfg.d_out);
         std::mt19937_64 rng(h->cfg.seed ^ 0x5bd1e995ULL ^ (uint64_t)h->adam_t);
         std::vector<int> perm(h->n_data);
         std::vector<float> lossv(steps);
@@ -1245,23 +1252,27 @@ int nir_mlp_train(nir_mlp* h, int32_t epochs, int32_t batch, float* epoch_loss) 
             MLP_CUDA(cudaMemcpyAsync(h->perm.p, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice,
                                      h->stream));
             MLP_CUDA(cudaEventRecord(e0, h->stream));
-            // the epoch's samples in its order, at once
-            k_gather_rows<bf16><<<grid1d((size_t)used * h->cfg.d_in), 256, 0, h->stream>>>(h->perm.p, used, h->cfg.d_in,
-                                                                                           h->data_x.p, h->ep_x.p);
-            k_gather_rows<float><<<grid1d((size_t)used * h->cfg.d_out), 256, 0, h->stream>>>(h->perm.p, used, h->cfg.d_out,
-                                                                                             h->data_y.p, h->ep_y.p);
-            MLP_LAUNCHED();
             for (int s = 0; s < steps; ++s) {
                 h->adam_t += 1;
                 bcv[size_t(s)] = make_float2(1.f - std::pow(h->cfg.beta1, float(h->adam_t)),
                                              1.f - std::pow(h->cfg.beta2, float(h->adam_t)));
             }
             MLP_CUDA(cudaMemcpyAsync(h->bc.p, bcv.data(), bcv.size() * sizeof(float2), cudaMemcpyHostToDevice, h->stream));
-            for (int s = 0; s < steps; ++s) {
-                const bf16* x = h->ep_x.p + (size_t)s * batch * h->cfg.d_in;
-                forward(h, batch, x);
-                backward(h, batch, x, h->ep_y.p + (size_t)s * batch * h->cfg.d_out, s);
-                adam(h, batch, s);
+            for (int s0 = 0; s0 < steps; s0 += piece) {
+                // the piece's samples in the epoch's order, at once
+                const int k = std::min(piece, steps - s0), rows = k * batch;
+                const int* idx = h->perm.p + (size_t)s0 * batch;
+                k_gather_rows<bf16><<<grid1d((size_t)rows * h->cfg.d_in), 256, 0, h->stream>>>(
+                    idx, rows, h->cfg.d_in, h->data_x.p, h->ep_x.p);
+                k_gather_rows<float><<<grid1d((size_t)rows * h->cfg.d_out), 256, 0, h->stream>>>(
+                    idx, rows, h->cfg.d_out, h->data_y.p, h->ep_y.p);
+                MLP_LAUNCHED();
+                for (int s = 0; s < k; ++s) {
+                    const bf16* x = h->ep_x.p + (size_t)s * batch * h->cfg.d_in;
+                    forward(h, batch, x);
+                    backward(h, batch, x, h->ep_y.p + (size_t)s * batch * h->cfg.d_out, s0 + s);
+                    adam(h, batch, s0 + s);
+                }
             }
             finish_losses(h, batch, steps);
             MLP_CUDA(cudaEventRecord(e1, h->stream));
