@@ -13,9 +13,10 @@
 // tcgen05.mma on them, the FP32 accumulators lie in tensor memory, and 8
 // warps finish the tile (bias, ReLU, mask) and store it.
 // A product with few output tiles and a long K is a sum of splits of K, added
-// in order: a CTA keeps an accumulator for each, or the CTAs of a thread-block
-// cluster compute them side by side and add them through each other's shared
-// memory (deterministic).
+// in order (deterministic): a CTA keeps an accumulator for each, or the CTAs
+// of a thread-block cluster compute them side by side and add them through
+// each other's shared memory, or as many CTAs as there are splits leave them
+// in a workspace, where another kernel adds them.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -142,7 +143,9 @@ __device__ __forceinline__ void epilogue8(const GemmArgs& g, int row, int col, c
 // cluster share the tile: in each round a rank computes one split and leaves
 // it in shared memory, where the stages were, and every rank adds its share
 // of the tile's rows over the splits in order, reading the other ranks'
-// shared memory.  Neither the tile nor the ranks decide the order of any sum.
+// shared memory; or (G.parts) each split of a tile has a CTA of its own, which
+// leaves it in the workspace as rows of a taller product, for k_add_splits.
+// Neither the tile nor the ranks decide the order of any sum.
 // One launch takes a group of independent products (the weight gradients of
 // all layers).
 // Small products are bound by their latency (load, multiply, read back,
@@ -178,7 +181,8 @@ struct GemmGroupOf {
     GemmOne g[MAX];
     int first[MAX + 1];  // first tile of each product
     int count;
-    int rank_bits;       // 2^rank_bits CTAs per tile
+    int rank_bits;       // 2^rank_bits CTAs per tile, a cluster
+    int parts;           // splits per tile that CTAs leave in the workspace, or 0 (then rank_bits = 0, accs = 1)
     int accs;            // splits that a CTA computes one after another, each in its own accumulator (one CTA per tile)
     int stages;          // at most STAGES_MAX
     uint32_t tmem;       // columns of tensor memory for them, a power of two
@@ -285,7 +289,12 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + i * 8) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const int tile = blockIdx.x >> G.rank_bits, ranks = 1 << G.rank_bits, rank = blockIdx.x & (ranks - 1);
+    int ranks = 1 << G.rank_bits, tile = int(blockIdx.x) >> G.rank_bits, rank = int(blockIdx.x) & (ranks - 1);
+    if (G.parts) {
+        ranks = G.parts;
+        tile = int(blockIdx.x) / ranks;
+        rank = int(blockIdx.x) % ranks;
+    }
     int p = 0;
     while (p + 1 < G.count && tile >= G.first[p + 1]) ++p;
     const GemmOne& o = G.g[p];
@@ -394,7 +403,8 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         if (!split) {
             __syncthreads();
-            for (int e = tid; e < (rank == 0 ? 128 * GROUPS : 0); e += 256) {
+            const int part = G.parts ? rank * g.M : 0;  // first row of this split in the workspace
+            for (int e = tid; e < ((G.parts ? z1 > z0 : rank == 0) ? 128 * GROUPS : 0); e += 256) {
                 const int r = e / GROUPS, c = 8 * (e % GROUPS);
                 if (m0 + r >= g.M || n0 + c >= g.N) continue;
                 float v[8];
@@ -407,7 +417,7 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
                              : "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
                              : "r"(at + 16)
                              : "memory");
-                epilogue8(g, m0 + r, n0 + c, v);
+                epilogue8(g, part + m0 + r, n0 + c, v);
             }
         } else {
             cluster_arrive();
@@ -440,6 +450,28 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
     if (!ok) *G.fault = 1;
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(G.tmem));
+}
+
+// C of each product from its splits in the workspace, one element per thread.
+struct AddTable {
+    GemmArgs g[GROUP_MAX];
+    const float* ws[GROUP_MAX];  // splits x M x N
+    int first[GROUP_MAX + 1];    // first CTA of each product
+    int count;
+};
+__global__ void __launch_bounds__(256) k_add_splits(const __grid_constant__ AddTable t) {
+    pdl_release();
+    int p = 0;
+    while (p + 1 < t.count && int(blockIdx.x) >= t.first[p + 1]) ++p;
+    const GemmArgs& g = t.g[p];
+    const size_t n = (size_t)g.M * g.N, i = (size_t)(int(blockIdx.x) - t.first[p]) * 256 + threadIdx.x;
+    pdl_wait();
+    if (i >= n) return;
+    const float* ws = t.ws[p] + i;
+    float v = 0.f;
+#pragma unroll 16
+    for (int z = 0; z < g.splits; ++z) v += ws[(size_t)z * n];
+    epilogue1(g, int(i / g.N), int(i % g.N), v);
 }
 
 // ------------------------------------------------------------ elementwise
@@ -666,6 +698,7 @@ struct nir_mlp {
     float* outw = nullptr;  // per-output loss weights
     float outw_sum = 0.f;
     // activations of a forward pass
+    nir::Grown<float> ws;  // splits of products (k_add_splits)
     nir::Grown<bf16> x;
     std::vector<nir::Grown<bf16>> act;  // hidden outputs
     nir::Grown<float> pred;
@@ -801,10 +834,10 @@ CUtensorMap operand_map(const bf16* P, int ld, int rows, int K, bool kmaj, int t
     return m;
 }
 
-// How a launch is cut: 128 x tn tiles, 2^bits CTAs each.
+// How a launch is cut: 128 x tn tiles, of 2^bits or of `parts` CTAs each.
 struct GemmPlan {
     double time = 1e300;
-    int tn = 64, bits = 0, stages = 0;
+    int tn = 64, bits = 0, parts = 0, stages = 0;
     uint32_t tmem = 0;
 };
 // Estimated time (us) of a group, from runs over M 128..65536, N 16..8192 and
@@ -818,15 +851,23 @@ struct GemmPlan {
 // after it loads anew.  Two CTAs fit on an SM unless their tensor memory or
 // their stages do not; clusters of 16 fill about half of the SMs, and those
 // of 8 and more find an SM for each CTA only while half of the SMs do.
-GemmPlan gemm_plan(const nir_mlp* h, const GemmArgs* gs, int count, int splits, int tn, int bits) {
-    const int ranks = 1 << bits;
+// With few tiles and a long K clusters leave SMs idle and take many rounds;
+// a CTA for each split does not, for a second kernel of 2 us and the splits'
+// way through L2 (1.4 us per million of them, and 0.04 for each one a sum is
+// deep): 256 x 512 x 52000 in 37 splits takes 31 us, 77 at best by clusters,
+// 128 x 128 x 65536 in 256 splits 25 against 128, 512 x 512 x 4096 in 16 15
+// against 24; but 512 x 512 x 1024 in four 9.2 against 7.6, 2048 x 1024 x
+// 16384 in three 109 against 97 by one CTA a tile.
+GemmPlan gemm_plan(const nir_mlp* h, const GemmArgs* gs, int count, int splits, int tn, int bits, bool parts) {
+    const int ranks = parts ? splits : 1 << bits;
     long long ctas = 0;
     for (int i = 0; i < count; ++i) ctas += (long long)((gs[i].M + 127) / 128) * ((gs[i].N + tn - 1) / tn) * ranks;
     GemmPlan p;
     p.tn = tn;
     p.bits = bits;
+    p.parts = parts ? splits : 0;
     p.tmem = tn;
-    while (bits == 0 && p.tmem < uint32_t(tn * splits)) p.tmem *= 2;
+    while (bits == 0 && !parts && p.tmem < uint32_t(tn * splits)) p.tmem *= 2;
     const int slots = bits == RANK_BITS_MAX || 2 * p.tmem > TMEM_COLUMNS ? h->sms : 2 * h->sms;
     // one CTA to an SM, with all of its memory
     const bool alone = ctas <= (bits >= 3 ? h->sms / 2 : h->sms) || 2 * p.tmem > TMEM_COLUMNS;
@@ -836,13 +877,19 @@ GemmPlan gemm_plan(const nir_mlp* h, const GemmArgs* gs, int count, int splits, 
     const double swap = alone ? (tn == 64 ? 0.8 + 0.3 * bits + 0.004 * there : 1.5 + 0.6 * bits + 0.005 * there)
                               : (tn == 64 ? 2.3 + 0.5 * bits + 0.012 * there : 3.0 + 1.5 * bits + 0.03 * there);
     const double again = !alone ? 0.0 : tn == 64 ? 1.0 : 1.8;
-    double longest = 0.0;
+    double longest = 0.0, add = 0.0;
     for (int i = 0; i < count; ++i) {
         const double split = (std::min(gs[i].kps, gs[i].K) + SK - 1) / SK * stage;
         const int rounds = (gs[i].splits + ranks - 1) / ranks;
+        if (parts) {
+            longest = std::max(longest, split);
+            add += 1.4e-6 * double(gs[i].splits) * gs[i].M * gs[i].N;
+            continue;
+        }
         longest = std::max(longest, bits ? rounds * (split + swap) + (rounds - 1) * again : gs[i].splits * split);
     }
     p.time = double((ctas + slots - 1) / slots) * ((tn == 64 ? 4.0 : 5.0) + longest);
+    if (parts) p.time += 2.0 + 0.04 * splits + add;
     return p;
 }
 
@@ -856,6 +903,9 @@ void prepare_gemm(nir_mlp* h) {
     MLP_CUDA(cudaFuncSetAttribute(k_gemm<TN, AK, BKM>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     ready = true;
 }
+
+// Floats of a product's splits in the workspace, whole 256-byte lines.
+size_t parts_len(const GemmArgs& g) { return ((size_t)g.splits * g.M * g.N + 63) / 64 * 64; }
 
 template <int TN, bool AK, bool BKM>
 void launch_tiles(nir_mlp* h, const GemmArgs* gs, int count, int splits, const GemmPlan& plan) {
@@ -873,11 +923,36 @@ void launch_tiles(nir_mlp* h, const GemmArgs* gs, int count, int splits, const G
     G.count = count;
     G.fault = h->fault;
     G.rank_bits = plan.bits;
-    G.accs = plan.bits ? 1 : splits;
+    G.parts = plan.parts;
+    G.accs = plan.bits || plan.parts ? 1 : splits;
     G.tmem = plan.tmem;
     G.stages = plan.stages;
-    launch_early(h, k_gemm<TN, AK, BKM>, dim3(unsigned(tiles) << G.rank_bits), GTile<TN>::threads,
-                 GTile<TN>::smem(G.stages), 1 << G.rank_bits, G);
+    if (plan.parts) {
+        size_t floats = 0;
+        for (int i = 0; i < count; ++i) floats += parts_len(gs[i]);
+        float* ws = h->ws.ensure(*h, floats);
+        AddTable t;
+        t.count = count;
+        t.first[0] = 0;
+        for (int i = 0; i < count; ++i) {
+            const GemmArgs& g = gs[i];
+            t.g[i] = g;
+            t.ws[i] = ws;
+            t.first[i + 1] = t.first[i] + int(((size_t)g.M * g.N + 255) / 256);
+            GemmArgs& q = G.g[i].g;
+            q.epi = EPI_F32;
+            q.out_f = ws;
+            q.ldc = g.N;
+            q.wide = g.N % 8 == 0;
+            ws += parts_len(g);
+        }
+        launch_early(h, k_gemm<TN, AK, BKM>, dim3(unsigned(tiles * plan.parts)), GTile<TN>::threads,
+                     GTile<TN>::smem(G.stages), 1, G);
+        launch_early(h, k_add_splits, dim3(unsigned(t.first[count])), 256, 0, 1, t);
+    } else {
+        launch_early(h, k_gemm<TN, AK, BKM>, dim3(unsigned(tiles) << G.rank_bits), GTile<TN>::threads,
+                     GTile<TN>::smem(G.stages), 1 << G.rank_bits, G);
+    }
     MLP_LAUNCHED();
 }
 
@@ -890,7 +965,12 @@ void launch_gemm(nir_mlp* h, const GemmArgs* gs, int count) {
     for (int tn : {64, 128})
         for (int bits = splits * tn > TMEM_COLUMNS; bits == 0 || (bits <= RANK_BITS_MAX && (1 << bits) < 2 * splits);
              ++bits) {
-            const GemmPlan p = gemm_plan(h, gs, count, splits, tn, bits);
+            const GemmPlan p = gemm_plan(h, gs, count, splits, tn, bits, false);
+            if (p.time < best.time) best = p;
+        }
+    if (splits > 1)
+        for (int tn : {64, 128}) {
+            const GemmPlan p = gemm_plan(h, gs, count, splits, tn, 0, true);
             if (p.time < best.time) best = p;
         }
     if (best.tn == 64) launch_tiles<64, AK, BKM>(h, gs, count, splits, best);
