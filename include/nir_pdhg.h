@@ -244,7 +244,8 @@ int nir_pdhg_kernel_times(nir_pdhg* h, nir_pdhg_kernel_time* out);
 /* Steady-state CUDA-event timing of the two fused iteration kernels (A' y
  * + primal step, A x-bar + dual step) after a PDHG/PDLP solve on this handle:
  * `reps` back-to-back launches of each kernel alone and of the pair, on the
- * last solve's layout and state.  precision: NIR_PREC_FP64 (FP64 values and
+ * last solve's layout and state (after solves in thread-block clusters only,
+ * on the default layout, which the first such call builds).  precision: NIR_PREC_FP64 (FP64 values and
  * iterates), NIR_PREC_MIXED (FP32 values, FP64 iterates) or NIR_PREC_FP32.
  * The kernels overwrite the handle's iterates (not x_out / y_out of the
  * solve, nor the point nir_pdhg_verify checks); the next solve starts anew.
@@ -258,11 +259,14 @@ int nir_pdhg_time_iteration(nir_pdhg* h, int precision, int reps, double* primal
  * of entries written (at most max_entries and the last 4096 checks). */
 int nir_pdhg_history(nir_pdhg* h, double* out, int max_entries);
 
-/* Matrix and layout facts: nnz, rows, row blocks of each orientation. */
+/* Matrix and layout facts: nnz, rows, row blocks of each orientation, as the
+ * last PDHG/PDLP solve with the per-launch kernels used them.  On a handle
+ * whose solves all ran in thread-block clusters, which use no such blocks:
+ * those that the per-launch kernels would have by default. */
 typedef struct nir_pdhg_layout {
     int32_t nrow, ncol;
     int64_t nnz;
-    int32_t blocks_a, blocks_at;        /* SpMV blocks of A and A' of the last solve */
+    int32_t blocks_a, blocks_at;        /* SpMV blocks of A and A'                   */
     int32_t block_nnz;                  /* nonzeros per block of A: 32..256 for warp row
                                            blocks, 1024 for CTA blocks               */
     int64_t device_bytes;               /* device memory held by the handle    */

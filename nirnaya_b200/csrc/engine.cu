@@ -184,6 +184,8 @@ struct nir_pdhg {
     long long nnz = 0;
     double offset = 0.0;
     Orient A, At;
+    // the row blocks of the reference loop (its own: a reference solve leaves the layouts in use alone)
+    Orient::Layout ref_a{}, ref_at{};
     // original vectors on the device (bounds sanitised to +-inf)
     double *c = nullptr, *l = nullptr, *u = nullptr, *rl = nullptr, *ru = nullptr;
     std::vector<double> h_c, h_l, h_u, h_rl, h_ru;
@@ -316,24 +318,26 @@ void d2h(nir_pdhg* h, void* dst, const void* src, size_t bytes) {
 using nir::build_row_blocks;
 using nir::check_row_blocks;
 
-void set_blocks(nir_pdhg* h, Orient& o, int cap) {
-    if (o.cap == cap && o.blk) return;
-    // a capacity used before keeps its device copy: switching back and forth
-    // (the autotuner, or solves with different spmv_block_nnz) allocates once
+// The row blocks of one capacity.  Each keeps its device copy: switching
+// back and forth (the autotuner, or solves with different spmv_block_nnz)
+// allocates once.
+Orient::Layout row_layout(nir_pdhg* h, Orient& o, int cap) {
     for (const auto& l : o.layouts)
-        if (l.cap == cap) {
-            o.blk = l.blk;
-            o.nblk = l.nblk;
-            o.cap = cap;
-            return;
-        }
+        if (l.cap == cap) return l;
     std::vector<int2> b = build_row_blocks(o.h_rp, cap);
     check_row_blocks(b, o.h_rp, cap);
-    o.nblk = int(b.size()) - 1;
-    o.blk = h->alloc<int2>(b.size());
-    h2d(h, o.blk, b.data(), b.size() * sizeof(int2));
-    o.cap = cap;
-    o.layouts.push_back({cap, o.nblk, o.blk});
+    const Orient::Layout l{cap, int(b.size()) - 1, h->alloc<int2>(b.size())};
+    h2d(h, l.blk, b.data(), b.size() * sizeof(int2));
+    o.layouts.push_back(l);
+    return l;
+}
+
+void set_blocks(nir_pdhg* h, Orient& o, int cap) {
+    if (o.cap == cap && o.blk) return;
+    const Orient::Layout l = row_layout(h, o, cap);
+    o.blk = l.blk;
+    o.nblk = l.nblk;
+    o.cap = l.cap;
 }
 
 // The CTA-block layout of an orientation for capacity `cap` (256 E), built
@@ -1117,15 +1121,16 @@ struct RefProbe {
 void launch_ref_chunk(nir_pdhg* h, int K, const RefProbe* probe) {
     cudaStream_t s = h->stream;
     const PartLayout L = part_layout(h);
-    auto ctas = [](const Orient& o) { return std::max(1, (o.nblk + nir::kWarps - 1) / nir::kWarps); };
-    const int gn = ctas(h->At), gm = ctas(h->A);
+    const Orient::Layout &bc = h->ref_at, &br = h->ref_a;
+    auto ctas = [](const Orient::Layout& b) { return std::max(1, (b.nblk + nir::kWarps - 1) / nir::kWarps); };
+    const int gn = ctas(bc), gm = ctas(br);
     for (int i = 0; i < K; ++i) {
         // the first step of the chunk and the one after the stop test read
         // the state a kernel before them wrote; the others start early
-        launch_kernel(h, i > 1, nir::k_refb_primal, gn, 0, (const int2*)h->At.blk, h->At.nblk, h->At.cap, h->At.rp,
+        launch_kernel(h, i > 1, nir::k_refb_primal, gn, 0, (const int2*)bc.blk, bc.nblk, bc.cap, h->At.rp,
                       h->At.ci, h->At.v_orig, h->y64, h->c, h->l, h->u, h->x64, h->xb64, h->st, i);
-        launch_kernel(h, true, i == 0 ? nir::k_refb_dual<true> : nir::k_refb_dual<false>, gm, 0, (const int2*)h->A.blk,
-                      h->A.nblk, h->A.cap, h->A.rp, h->A.ci, h->A.v_orig, h->xb64, h->rl, h->ru, h->y64, h->tmp_m, h->st, i);
+        launch_kernel(h, true, i == 0 ? nir::k_refb_dual<true> : nir::k_refb_dual<false>, gm, 0, (const int2*)br.blk,
+                      br.nblk, br.cap, h->A.rp, h->A.ci, h->A.v_orig, h->xb64, h->rl, h->ru, h->y64, h->tmp_m, h->st, i);
         h->launches += 2;
         if (i == 0) {
             // one maximum per CTA, at most one CTA per row
@@ -1284,7 +1289,8 @@ int solve_reference(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), v
     const double t0 = now_sec();
     ensure_partials(h);
     // row blocks of both orientations (the order of a row's sum does not depend on them)
-    for (Orient* o : {&h->A, &h->At}) set_blocks(h, *o, auto_cap(h->nnz, o->rows));
+    h->ref_a = row_layout(h, h->A, auto_cap(h->nnz, h->m));
+    h->ref_at = row_layout(h, h->At, auto_cap(h->nnz, h->n));
     const int n = h->n, m = h->m;
     nir::DevState st0{};
     st0.max_iters = p.max_iters;
@@ -1329,7 +1335,7 @@ int solve_reference(nir_pdhg* h, const nir_pdhg_params& p, int (*poll)(void*), v
             KeyHash key;
             key.add(1000).add(probing).add(probe.bnorm).add(probe.cnorm).add(probe.tol).add(h->offset);
             if (probing) key.add(lay_of(h->A).blk).add(lay_of(h->At).blk).add(h->A.lay).add(h->At.lay);
-            key.add(h->part).add(h->A.blk).add(h->A.cap).add(h->At.blk).add(h->At.cap);
+            key.add(h->part).add(h->ref_a.blk).add(h->ref_a.cap).add(h->ref_at.blk).add(h->ref_at.cap);
             cudaGraphExec_t ge = chunk_graph(h, 0, key.h, launch);
             const int per = launches_per_chunk(K, true) + (probing ? 3 : 0);
             R = run_chunks(h, p, poll, ctx, t0, 0, per, [&]() { NIR_CUDA(cudaGraphLaunch(ge, s)); }, nullptr);
@@ -2631,18 +2637,25 @@ int nir_pdhg_get_layout(nir_pdhg* h, nir_pdhg_layout* out) {
     out->nrow = h->m;
     out->ncol = h->n;
     out->nnz = h->nnz;
-    nir_pdhg* src = h->inner ? h->inner.get() : h;  // PDHG / PDLP solves ran on the equivalent LP
-    try {
-        NIR_CUDA(cudaSetDevice(src->device));
-        ensure_kernel_layouts(src);
-    } catch (const std::exception& e) {
-        g_err = e.what();
-        return NIR_STATUS_INTERNAL_ERROR;
+    const nir_pdhg* src = h->inner ? h->inner.get() : h;  // PDHG / PDLP solves ran on the equivalent LP
+    if (src->cluster && (src->A.lay < 0 || src->At.lay < 0)) {
+        // only solves in clusters so far: the layout the per-launch kernels would have by default
+        const LayChoice c = default_layouts(src);
+        try {
+            out->blocks_a = int(build_row_blocks(src->A.h_rp, c.cap_a).size()) - 1;
+            out->blocks_at = int(build_row_blocks(src->At.h_rp, c.cap_at).size()) - 1;
+        } catch (const std::exception& e) {
+            g_err = e.what();
+            return NIR_STATUS_INTERNAL_ERROR;
+        }
+        out->block_nnz = c.cap_a;
+        out->block_nnz_at = c.cap_at;
+    } else {
+        out->blocks_a = src->A.lay >= 0 ? lay_nblk(src->A) : 0;
+        out->blocks_at = src->At.lay >= 0 ? lay_nblk(src->At) : 0;
+        out->block_nnz = src->A.lay == nir::kLayCta ? kCtaCap : src->A.cap;
+        out->block_nnz_at = src->At.lay == nir::kLayCta ? kCtaCap : src->At.cap;
     }
-    out->blocks_a = src->A.lay >= 0 ? lay_nblk(src->A) : 0;
-    out->blocks_at = src->At.lay >= 0 ? lay_nblk(src->At) : 0;
-    out->block_nnz = src->A.lay == nir::kLayCta ? kCtaCap : src->A.cap;
-    out->block_nnz_at = src->At.lay == nir::kLayCta ? kCtaCap : src->At.cap;
     out->device_bytes = h->mem.bytes + (h->cluster ? h->cluster->mem.bytes : 0);
     return 0;
 }
