@@ -107,6 +107,12 @@ int nir_mlp_gradients(nir_mlp* h, const float* x, const float* targets, int32_t 
 int nir_mlp_gemm_check(nir_mlp* h, int a_kmaj, int b_kmaj, int32_t M, int32_t N, int32_t K, const float* A,
                        int32_t lda, const float* B, int32_t ldb, float* C);
 
+/* Test of the GEMM's bounded waits, on an M x N x K product (multiples of 8):
+ * its loads are waited for with bytes that nobody sends, so it must return 3
+ * within seconds ("a wait inside a GEMM kernel gave up"), and the handle
+ * works on. */
+int nir_mlp_wait_test(nir_mlp* h, int32_t M, int32_t N, int32_t K);
+
 /* Mean device time (microseconds, CUDA events, after one warm-up) of the
  * forward-layer GEMM (bias + ReLU epilogue) on M x K and N x K BF16
  * operands, for throughput measurements: 2*M*N*K FLOP per call. */

@@ -159,7 +159,9 @@ constexpr int RANK_BITS_MAX = 4;
 constexpr int STAGES_MAX = 6;
 constexpr int SK = 64;         // K of a stage
 constexpr int TMEM_COLUMNS = 512;  // of an SM
-constexpr int GEMM_WAIT_MAX = 1 << 20;
+// A wait ends after so many tries (about 30 ms), one for loads after another
+// wait has failed sooner.
+constexpr int WAIT_TRIES = 1 << 20, DRAIN_TRIES = 1 << 12;
 
 template <int TN>
 struct GTile {
@@ -186,6 +188,7 @@ struct GemmGroupOf {
     int accs;            // splits that a CTA computes one after another, each in its own accumulator (one CTA per tile)
     int stages;          // at most STAGES_MAX
     uint32_t tmem;       // columns of tensor memory for them, a power of two
+    uint32_t lost;       // test of the bounded waits: bytes of every stage that nobody loads
     int* fault;          // set if a wait of the kernel gives up
 };
 // Weight gradients come in groups, the other products one by one (the
@@ -216,8 +219,8 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
            (uint64_t(2) << 61);
 }
 
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < GEMM_WAIT_MAX; ++i) {
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, int tries = WAIT_TRIES) {
+    for (int i = 0; i < tries; ++i) {
         uint32_t done;
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
@@ -272,6 +275,7 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
     constexpr int SUMS = 128 * GROUPS / 2 / 256;   // groups that a thread adds, for two ranks
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint32_t tmem_at;
+    __shared__ int gave_up;  // a wait of the multiplying thread ran out
     __shared__ __align__(8) unsigned long long bars[2 * STAGES_MAX + 1];  // stage full, stage free, round multiplied
     pdl_release();
     const uint32_t sb = (static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + 1023u) & ~1023u;
@@ -285,6 +289,7 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     } else if (tid == 32) {
+        gave_up = 0;
         for (int i = 0; i <= 2 * STAGES_MAX; ++i)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + i * 8) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -311,7 +316,9 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
                                (uint32_t(TN / 8) << 17) | (8u << 24);
     constexpr uint32_t step_a = AK ? 32 : 2048, step_b = BKM ? 32 : 2048;  // 16 of K
     bool ok = true;
+    int bad = 0;           // gave_up
     int rounds = 0;        // multiplied so far
+    const uint32_t expect = uint32_t(L::stage) + G.lost;  // bytes of a stage
     int s = 0, phase = 0;  // of the loading and of the multiplying thread: the next stage, and how often all were passed
     float sum[SUMS][8];
 #pragma unroll
@@ -330,16 +337,12 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
                     if (!ok) break;
                     const uint32_t at = sb + s * L::stage;
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + s * 8),
-                                 "r"(uint32_t(L::stage))
+                                 "r"(expect)
                                  : "memory");
                     load_operand<128, AK>(at, &o.a, m0, k, full + s * 8);
                     load_operand<TN, BKM>(at + L::bytes_a, &o.b, n0, k, full + s * 8);
                     if (++s == S) s = 0, ++phase;
                 }
-            // given up: what was started still arrives before this CTA ends
-            if (!ok)
-                for (int j = 0; j < S; ++j)
-                    if (j < s || phase > 0) bar_wait(full + j * 8, (j < s ? phase : phase - 1) & 1);
         } else if (tid == 0 && z1 > z0) {
             for (int z = z0; z < z1; ++z) {
                 const int kbeg = z * g.kps, kend = min(g.K, kbeg + g.kps);
@@ -373,7 +376,9 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
             ++rounds;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (tid == 0 && !ok) gave_up = 1;
         __syncthreads();  // the finished tile lies where the stages were
+        bad |= gave_up;
         if (z1 > z0) {
             // warp w holds rows 32 (w % 4).. and half of the columns
             const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * (TN / 2);
@@ -447,6 +452,10 @@ __global__ void __launch_bounds__(256, 2) k_gemm(const __grid_constant__ GemmGro
             cluster_wait();
         }
     }
+    // given up: the loads that were started land while this CTA is there
+    if (tid == 32 && bad)
+        for (int j = 0; j < S; ++j)
+            if (j < s || phase > 0) bar_wait(full + j * 8, (j < s ? phase : phase - 1) & 1, DRAIN_TRIES);
     if (!ok) *G.fault = 1;
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(G.tmem));
@@ -723,6 +732,7 @@ struct nir_mlp {
     // output map of nir_mlp_predict_device_affine
     bool gemm_ready[8] = {};  // GEMM kernels prepared for launches
     int* fault = nullptr;     // mapped host memory, set if a wait inside a GEMM gives up
+    bool wait_test = false;   // the next products' waits cannot end (nir_mlp_wait_test)
     int aff_n = 0, aff_col = 0;
     double aff_lo = 0.0, aff_hi = 0.0;
     double *aff_scale = nullptr, *aff_shift = nullptr, *aff_out = nullptr;
@@ -922,6 +932,7 @@ void launch_tiles(nir_mlp* h, const GemmArgs* gs, int count, int splits, const G
     G.first[count] = tiles;
     G.count = count;
     G.fault = h->fault;
+    G.lost = h->wait_test ? 16 : 0;
     G.rank_bits = plan.bits;
     G.parts = plan.parts;
     G.accs = plan.bits || plan.parts ? 1 : splits;
@@ -1565,6 +1576,25 @@ int nir_mlp_gemm_check(nir_mlp* h, int a_kmaj, int b_kmaj, int32_t M, int32_t N,
         return fail(e, false);
     }
     return 0;
+}
+
+int nir_mlp_wait_test(nir_mlp* h, int32_t M, int32_t N, int32_t K) {
+    if (!h || M < 8 || N < 8 || K < 8 || M % 8 || N % 8 || K % 8) {
+        g_err = "invalid arguments";
+        return 2;
+    }
+    std::vector<float> a, b, c;
+    try {
+        a.resize((size_t)M * K);
+        b.resize((size_t)N * K);
+        c.resize((size_t)M * N);
+    } catch (const std::exception& e) {
+        return fail(e, false);
+    }
+    h->wait_test = true;
+    const int rc = nir_mlp_gemm_check(h, 1, 1, M, N, K, a.data(), K, b.data(), K, c.data());
+    h->wait_test = false;
+    return rc;
 }
 
 int nir_mlp_gemm_time(nir_mlp* h, int32_t M, int32_t N, int32_t K, int32_t reps, double* us) {

@@ -13,7 +13,7 @@ LIB_PATH = os.path.join(_HERE, "libnir_mlp.so")
 EXPORTED = [
     "nir_mlp_create", "nir_mlp_free", "nir_mlp_last_error", "nir_mlp_param_count", "nir_mlp_get_params",
     "nir_mlp_set_params", "nir_mlp_set_output_weights", "nir_mlp_set_data", "nir_mlp_train", "nir_mlp_predict",
-    "nir_mlp_gradients", "nir_mlp_gemm_check", "nir_mlp_gemm_time", "nir_mlp_step_stats", "nir_mlp_predict_device",
+    "nir_mlp_gradients", "nir_mlp_gemm_check", "nir_mlp_gemm_time", "nir_mlp_wait_test", "nir_mlp_step_stats", "nir_mlp_predict_device",
     "nir_mlp_set_affine", "nir_mlp_predict_device_affine",
 ]
 BLEND_EXPORTED = ["nir_blend_features_create", "nir_blend_features_build", "nir_blend_features_free"]
@@ -64,6 +64,7 @@ def lib():
         L.nir_mlp_gemm_check.argtypes = [VP, C.c_int, C.c_int, C.c_int32, C.c_int32, C.c_int32, F, C.c_int32, F,
                                          C.c_int32, F]
         L.nir_mlp_step_stats.argtypes = [VP, C.POINTER(C.c_double), C.POINTER(C.c_double)]
+        L.nir_mlp_wait_test.argtypes = [VP, C.c_int32, C.c_int32, C.c_int32]
         L.nir_mlp_gemm_time.argtypes = [VP, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.POINTER(C.c_double)]
         L.nir_mlp_predict_device.argtypes = [VP, VP, C.c_int32, F]
         D = C.POINTER(C.c_double)
