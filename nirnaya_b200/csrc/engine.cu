@@ -902,6 +902,15 @@ void launch_kernel(nir_pdhg* h, bool early, void (*k)(P...), int grid, size_t sm
     NIR_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...));
 }
 
+// Whether k_dual may start before the k_primal ahead of it has ended.  Not on
+// a large LP whose rows are held longest first: its first CTAs take the long
+// rows and would all go to the SMs that come free first.  Us per iteration of
+// power-law LPs, early and not: 14.5 and 17.7 at 1M nonzeros, 27.7 and 28.3 at
+// 2M, but 30.4 to 31.9 and 29.8 at 2.25M, 40.5 and 38.9 at 3M, 57.6 and 57.2
+// at 5M, 105.5 and 103.0 at 10M.
+constexpr long long kEarlyDualMax = 2100000;
+bool early_dual(const nir_pdhg* h) { return h->row_orig.empty() || h->nnz <= kEarlyDualMax; }
+
 // The two FP64 KKT passes of a check over the layouts in use, at (xp, yp)
 // of type TX; returns their grids (the number of partials each wrote).
 template <typename TX>
@@ -1026,7 +1035,7 @@ void launch_fast_chunk_l(nir_pdhg* h, const SolveCfg& cfg, int phase, ChunkTimer
                       Vec<TX>::xb(h), Vec<TX>::xp(h), Vec<TX>::c(h), Vec<TX>::l(h), Vec<TX>::u(h), Vec<TX>::x0(h));
         if (timed) NIR_CUDA(cudaEventRecord(tm->e[1], s));
         const auto kd = check ? nir::k_dual<LD, TV, TX, true> : nir::k_dual<LD, TV, TX, false>;
-        launch_kernel(h, early, kd, check ? gd1 : gd0, sd, ad, valA, Vec<TX>::xb(h), Vec<TX>::y(h), Vec<TX>::yp(h),
+        launch_kernel(h, early && early_dual(h), kd, check ? gd1 : gd0, sd, ad, valA, Vec<TX>::xb(h), Vec<TX>::y(h), Vec<TX>::yp(h),
                       Vec<TX>::rl(h), Vec<TX>::ru(h), Vec<TX>::y0(h));
         if (timed) NIR_CUDA(cudaEventRecord(tm->e[2], s));
         h->launches += 2;
@@ -2539,7 +2548,7 @@ void time_iteration_l(nir_pdhg* h, int reps, double* primal_us, double* dual_us,
         NIR_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         for (int r = 0; r < reps; ++r) {
             if (which != 1) primal(r > 0);
-            if (which != 0) dual(r > 0 || which == 2);
+            if (which != 0) dual((r > 0 || which == 2) && early_dual(h));
         }
         const cudaError_t launched = cudaGetLastError();
         const cudaError_t ended = cudaStreamEndCapture(s, &g);
