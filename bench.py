@@ -700,7 +700,8 @@ def run_blocks(args, local):
                     "loop_algorithmic_GBs": alg / tts / 1e9,
                     "persistent_time_to_tol_s": float(np.mean(ptimes)),
                     "persistent_same_iterations": [r[2].iterations for r in pres] == its,
-                    "launch_mode": "graph-launched kernels per half-iteration (the default); "
+                    "launch_mode": "chunks of iterations in thread-block clusters for the instances that fit, "
+                                   "graph-launched kernels per half-iteration for the others (the default); "
                                    "persistent_time_to_tol_s: the cooperative persistent chunk kernel",
                     "note": "algorithmic bytes of the iterations each instance ran, counted at FP32 values with "
                             "FP64 vectors, over the device time of the whole solve"}

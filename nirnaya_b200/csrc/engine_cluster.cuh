@@ -392,10 +392,10 @@ double cl_arrivals(const ClusterPlan& P, int i) {
 // whose rows do not fill them or where the device holds none of 16.  Built
 // where clusters are faster even with nothing to exchange (below about
 // 85,000 nonzeros), kept where they still are with what the plan exchanges:
-// 2.7 against 5.4 us an iteration on a 60 x 150 LP, 4.8 against 5.9 on a
-// random 2,000 x 5,000 one of 40,000 nonzeros, 3.5 against 5.2 on a
-// multiperiod one of 15,000, but 6.3 against 6.3 on one of 126,000 and 10
-// against 6.9 on a blending LP of 100,000 whose ranks need nearly all
+// 2.5 against 4.3 us an iteration on a 60 x 150 LP, 4.6 against 5.9 on a
+// random 2,000 x 5,000 one of 40,000 nonzeros, 3.4 against 4.4 on a
+// multiperiod one of 15,000, but 6.0 against 5.6 on one of 126,000 and 9.5
+// against 5.6 on a blending LP of 100,000 whose ranks need nearly all
 // entries.
 ClusterPlan* cl_single(nir_pdhg* h, const nir_pdhg_params& p) {
     if (!cl_takes(h, p) || h->m < 1 || h->n < 1) return nullptr;

@@ -1,7 +1,7 @@
 // Chunks of iterations inside one thread-block cluster per LP.
 //
 // A small or medium LP spends its iteration on latency, not on bandwidth:
-// two kernels of a CUDA graph take about 5.9 us on a 2,000 x 5,000 LP of
+// two overlapping kernels take about 5.9 us on a 2,000 x 5,000 LP of
 // 40,000 nonzeros whose arithmetic takes a tenth of that, and a batch of
 // such LPs gathers from a vector that would fit in shared memory.  Here a
 // cluster of C CTAs (C = 1, 2, 4, 8 or 16) takes one LP through a whole
@@ -18,22 +18,22 @@
 //     and a gather costs bank conflicts instead of L2 latency.  Whoever
 //     computes an entry sends it to the ranks that gather it, all of a
 //     rank's entries by one bulk copy where the receiver takes an eighth of
-//     them or more, one by one (st.async) where it takes few; the bytes count on
-//     the receiver's mbarrier;
-//     a half-iteration starts when its entries have come, with no barrier
-//     over the cluster (its release fence alone took 490 cycles).  On a block-structured matrix a rank
-//     holds little more than its own part.
+//     them or more, one by one (st.async) where it takes few; the bytes
+//     count on the receiver's mbarrier; a half-iteration starts when its
+//     entries have come, with no barrier over the cluster (its release fence
+//     alone took 490 cycles).  On a block-structured matrix a rank holds
+//     little more than its own part.
 //   * What else fits is kept in shared memory too: the own vector entries,
 //     the slots to store to, and the matrix itself.
 //
 // Measured on B200 (us per iteration, checks included, against the
-// per-launch kernels): 2.7 against 5.4 on a 60 x 150 LP, 4.8 against 5.9 on
-// the 2,000 x 5,000 one (16 CTAs); 85 against 180 for a batch of 128
-// multiperiod LPs of 500 to 20,000 rows (16M nonzeros, clusters of 4), 5.5
-// against 12.6 for 96 LPs of 50 to 400 rows (clusters of 1).  Small LPs are
+// per-launch kernels): 2.5 against 4.3 on a 60 x 150 LP, 4.6 against 5.9 on
+// the 2,000 x 5,000 one (16 CTAs); 85 against 186 for a batch of 128
+// multiperiod LPs of 500 to 20,000 rows (16M nonzeros, clusters of 4), 5.9
+// against 9.1 for 96 LPs of 50 to 400 rows (clusters of 1).  Small LPs are
 // bound by the latency of a pass, about 1,300 cycles from the last arrival
 // to the last departure; large ones by the shared-memory pipe, where 32
-// random 8-byte gathers take 6 wavefronts (4.7-way conflicts measured).
+// random 8-byte gathers take 6 wavefronts.
 //
 // Sums are FP64, in an order fixed by the plan (never by timing); there are
 // no atomics.  The
